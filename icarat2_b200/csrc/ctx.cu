@@ -575,6 +575,17 @@ int icarat_ctx_create_sel_impl(const icarat_grid *grid, const icarat_material *m
     hexa8_stress_operator(c->hx, c->hy, c->hz, mat->poisson, c->sb0.s);
     for(int q = 0; q < 576; q++)
       c->ke0f.k[q] = (float)c->ke0.k[q];
+    {
+      constexpr int nk = sizeof(KhParam<double>) / sizeof(double);
+      static_assert(nk == 33 && sizeof(KhParam<float>) == nk * sizeof(float), "KhParam layout");
+      double k33[nk];
+      float k33f[nk];
+      hexa8_parity_blocks(c->ke0.k, k33);
+      for(int q = 0; q < nk; q++)
+        k33f[q] = (float)k33[q];
+      std::memcpy(&c->kh, k33, sizeof k33);
+      std::memcpy(&c->khf, k33f, sizeof k33f);
+    }
     c->ke_diag_max = 0.0;
     for(int a = 0; a < 24; a++)
       c->ke_diag_max = std::fmax(c->ke_diag_max, c->ke0.k[25 * a]);

@@ -122,6 +122,14 @@ struct KeParamF
 {
   float k[576];
 };
+// Ke0 (E = 1) in the corner sums and differences of the box element: the
+// symmetric 3 x 3 blocks c0, c7 (xx xy xz yy yz zz) and 2 x 2 blocks c1 .. c6
+// (first, coupling, second) of the parity classes (bit 0 x, 1 y, 2 z), with
+// the decoupled third entries s3, s5, s6; see modal.cuh
+template <typename T> struct KhParam
+{
+  T c0[6], c7[6], c1[3], c2[3], c3[3], c4[3], c5[3], c6[3], s3, s5, s6;
+};
 // Gauss-averaged stress operator at E = 1 (6 x 24, Voigt rows)
 struct StressParam
 {
@@ -339,6 +347,8 @@ struct icarat_ctx
   icarat_material mat;
   icarat_b200::KeParam ke0;
   icarat_b200::KeParamF ke0f; // ke0 rounded to FP32
+  icarat_b200::KhParam<double> kh; // ke0 by parity class (modal.cuh)
+  icarat_b200::KhParam<float> khf; // kh rounded to FP32
   icarat_b200::StressParam sb0; // stress operator at E = 1
   double vol0;
   double ke_diag_max; // max_a Ke0[a][a]
@@ -443,6 +453,7 @@ void hexa8_stress_operator(double hx, double hy, double hz, double nu, double *s
 void hexa8_stiffness(double hx, double hy, double hz, double nu, double *ke,
                      double *volume);
 double jacobi_bound(const double *ke);
+void hexa8_parity_blocks(const double *ke, double *k33);
 
 // noalloc.cu: resolves c->noalloc_scratch (context creation)
 void noalloc_resolve(icarat_ctx *c);
@@ -469,9 +480,6 @@ void launch_apply_K_f32(icarat_ctx *c, const GridDev &g, const float *E,
                         const uint8_t *fix, const float *u, float *y);
 void launch_diag(icarat_ctx *c, const GridDev &g, const double *E,
                  const uint8_t *fix, double *invd, cudaStream_t st = nullptr);
-void launch_residual(icarat_ctx *c, const GridDev &g, const double *E,
-                     const uint8_t *fix, const double *b, const double *x,
-                     double *r);
 void launch_fint(icarat_ctx *c, double *d_out_full);
 
 // reduce helpers (stiffness.cu)

@@ -11,6 +11,7 @@
 // Ke = sum B^T D B det(J) w.  Element DOF index = 3 * local node + component.
 #include <cmath>
 #include <cstring>
+#include <initializer_list>
 
 namespace icarat_b200
 {
@@ -206,6 +207,50 @@ double jacobi_bound(const double *ke)
   for(int i = 0; i < 24; i++)
     lmax = A[i][i] > lmax ? A[i][i] : lmax;
   return lmax;
+}
+
+// Ke in the corner sums and differences of the box, T Ke T^T / 64 with T the
+// 2 x 2 x 2 Hadamard transform per component: reflections leave one symmetric
+// 3 x 3 block per parity class p, of component c in the mode whose parity is
+// p with bit c flipped, and the translations (mode 0) carry nothing.  k33
+// takes the entries in the order of KhParam (internal.cuh).  Formed in long
+// double, so the transform adds one rounding to Ke's own.
+void hexa8_parity_blocks(const double *ke, double *k33)
+{
+  auto corner = [](int a) { // bits x, y, z -> reference local node
+    return 4 * (a >> 2) + ((a & 2) ? ((a & 1) ? 2 : 3) : (a & 1));
+  };
+  auto sign = [](int mode, int a) { // the corner's sign in the mode
+    const int minus = mode & ~a;
+    return ((minus ^ (minus >> 1) ^ (minus >> 2)) & 1) ? -1.0L : 1.0L;
+  };
+  auto entry = [&](int p, int c, int d) {
+    const int mc = p ^ (1 << c), md = p ^ (1 << d);
+    long double s = 0.0L;
+    for(int a = 0; a < 8; a++)
+      for(int b = 0; b < 8; b++)
+        s += sign(mc, a) * sign(md, b) *
+             (0.5L * ((long double)ke[24 * (3 * corner(a) + c) + 3 * corner(b) + d] +
+                      (long double)ke[24 * (3 * corner(b) + d) + 3 * corner(a) + c]));
+    return (double)(s / 64.0L);
+  };
+  double *o = k33;
+  for(int p : {0, 7})
+    for(int c = 0; c < 3; c++)
+      for(int d = c; d < 3; d++)
+        *o++ = entry(p, c, d);
+  // the coupled components of classes 1 .. 6
+  const int pair[7][2] = {{0, 0}, {1, 2}, {0, 2}, {0, 1}, {0, 1}, {0, 2}, {1, 2}};
+  for(int p = 1; p <= 6; p++)
+  {
+    const int c = pair[p][0], d = pair[p][1];
+    *o++ = entry(p, c, c);
+    *o++ = entry(p, c, d);
+    *o++ = entry(p, d, d);
+  }
+  *o++ = entry(3, 2, 2);
+  *o++ = entry(5, 1, 1);
+  *o++ = entry(6, 0, 0);
 }
 
 } // namespace icarat_b200

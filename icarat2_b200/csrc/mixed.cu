@@ -28,39 +28,39 @@
 // chunk.
 #include <cmath>
 
-#include "stencil.cuh"
+#include "modal.cuh"
 
 namespace icarat_b200
 {
 
 // Warm start: x kept, x32 = 0, r32 = b - K x in FP64; ||b|| and ||r||.
-__global__ void __launch_bounds__(128)
-    k_mx_init_warm(GridDev g, KeParam ke, const double *__restrict__ E,
+__global__ void __launch_bounds__(ModalCfg<double>::threads, ModalCfg<double>::blocks)
+    k_mx_init_warm(GridDev g, ModalPlan m, KhParam<double> kh, const double *__restrict__ E,
                    const uint8_t *__restrict__ fix, const double *__restrict__ b,
                    const double *__restrict__ x, float *__restrict__ x32,
                    float *__restrict__ r32, double *__restrict__ partials, MxScalars *s,
                    double tol, double delta, int maxit)
 {
+  ModalShared<double> &ms = modal_shared<double>();
   __shared__ double sh[64];
   double bb = 0.0, rr = 0.0;
-  for(int n = blockIdx.x * blockDim.x + threadIdx.x; n < g.numnp;
-      n += gridDim.x * blockDim.x)
-  {
-    double acc[3], uc[3];
-    node_Ku(g, ke, E, x, n, acc, uc);
-    const unsigned f = fix[n];
+  modal_march(g, m, kh, E, x, ms,
+              [&](int n) { return modal_rhs(g, fix, b, n); },
+              [&](int n, const double(&acc)[3], const double(&)[3], const ModalRhs<double> &pre)
+              {
+                const unsigned f = pre.fix;
 #pragma unroll
-    for(int q = 0; q < 3; q++)
-    {
-      const long id = (long)q * g.numnp + n;
-      const double bi = b[id];
-      const double r = ((f >> q) & 1u) ? 0.0 : bi - acc[q];
-      x32[id] = 0.0f;
-      r32[id] = (float)r;
-      bb += bi * bi;
-      rr += r * r;
-    }
-  }
+                for(int q = 0; q < 3; q++)
+                {
+                  const long id = (long)q * g.numnp + n;
+                  const double bi = pre.b[q];
+                  const double r = ((f >> q) & 1u) ? 0.0 : bi - acc[q];
+                  x32[id] = 0.0f;
+                  r32[id] = (float)r;
+                  bb += bi * bi;
+                  rr += r * r;
+                }
+              });
   double v[2] = {bb, rr};
   block_sum<2>(v, sh);
   if(threadIdx.x == 0)
@@ -147,27 +147,21 @@ __global__ void k_mx_init(int n, const double *__restrict__ b, double *__restric
 }
 
 // Ap = K32 p (constrained rows 0); alpha = zr / (p . Ap).
-__global__ void __launch_bounds__(128)
-    k_mx_spmv(GridDev g, MarchPlan m, KeParamF ke, const float *__restrict__ E,
+__global__ void __launch_bounds__(ModalCfg<float>::threads, ModalCfg<float>::blocks)
+    k_mx_spmv(GridDev g, ModalPlan m, KhParam<float> kh, const float *__restrict__ E,
               const uint8_t *__restrict__ fix, const float *__restrict__ p,
               float *__restrict__ Ap, double *__restrict__ partials, MxScalars *s)
 {
   chain_wait();
+  ModalShared<float> &ms = modal_shared<float>();
   __shared__ double sh[32];
   if(s->done)
     return;
   double dot = 0.0;
-  for(long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < m.items;
-      t += (long)gridDim.x * blockDim.x)
-  {
-    int i, j, k0, k1;
-    if(!march_item(g, m, t, i, j, k0, k1))
-      continue;
-    column_Ku(g, ke, E, p, i, j, k0, k1,
-              [&](int k, const float(&acc)[3], const float(&uc)[3])
+  modal_march(g, m, kh, E, p, ms,
+              [&](int n) { return (unsigned)fix[n]; },
+              [&](int n, const float(&acc)[3], const float(&uc)[3], unsigned f)
               {
-                const int n = i + j * g.NX + k * g.NX * g.NY;
-                const unsigned f = fix[n];
 #pragma unroll
                 for(int q = 0; q < 3; q++)
                 {
@@ -176,7 +170,6 @@ __global__ void __launch_bounds__(128)
                   dot += (double)uc[q] * (double)y;
                 }
               });
-  }
   double v[1] = {dot};
   block_sum<1>(v, sh);
   if(threadIdx.x == 0)
@@ -258,38 +251,32 @@ __global__ void k_mx_flush(int n, double *__restrict__ x, float *__restrict__ x3
 }
 
 // Refresh, part 2: r = b - K x in FP64, r32 = (float) r, stop test on ||r||.
-__global__ void __launch_bounds__(128)
-    k_mx_residual(GridDev g, MarchPlan m, KeParam ke, const double *__restrict__ E,
+__global__ void __launch_bounds__(ModalCfg<double>::threads, ModalCfg<double>::blocks)
+    k_mx_residual(GridDev g, ModalPlan m, KhParam<double> kh, const double *__restrict__ E,
                   const uint8_t *__restrict__ fix, const double *__restrict__ b,
                   const double *__restrict__ x, float *__restrict__ r32,
                   double *__restrict__ partials, MxScalars *s)
 {
   chain_wait();
+  ModalShared<double> &ms = modal_shared<double>();
   __shared__ double sh[32];
   if(s->done || !s->refresh)
     return;
   double rr = 0.0;
-  for(long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < m.items;
-      t += (long)gridDim.x * blockDim.x)
-  {
-    int i, j, k0, k1;
-    if(!march_item(g, m, t, i, j, k0, k1))
-      continue;
-    column_Ku(g, ke, E, x, i, j, k0, k1,
-              [&](int k, const double(&acc)[3], const double(&)[3])
+  modal_march(g, m, kh, E, x, ms,
+              [&](int n) { return modal_rhs(g, fix, b, n); },
+              [&](int n, const double(&acc)[3], const double(&)[3], const ModalRhs<double> &pre)
               {
-                const int n = i + j * g.NX + k * g.NX * g.NY;
-                const unsigned f = fix[n];
+                const unsigned f = pre.fix;
 #pragma unroll
                 for(int q = 0; q < 3; q++)
                 {
                   const long id = (long)q * g.numnp + n;
-                  const double r = ((f >> q) & 1u) ? 0.0 : b[id] - acc[q];
+                  const double r = ((f >> q) & 1u) ? 0.0 : pre.b[q] - acc[q];
                   r32[id] = (float)r;
                   rr += r * r;
                 }
               });
-  }
   double v[1] = {rr};
   block_sum<1>(v, sh);
   if(threadIdx.x == 0)
@@ -478,12 +465,6 @@ void apply_K_lowp(icarat_ctx *c, int op, const float *u, float *y)
 constexpr int kDefaultFineOp = ICARAT_OP_TC_BF16;
 constexpr int kDefaultKrylovOp = ICARAT_OP_FP32;
 
-static int spmv_blocks(const icarat_ctx *c)
-{
-  int b = (c->numnp + 127) / 128;
-  return b > kMaxRedBlocks ? kMaxRedBlocks : (b < 1 ? 1 : b);
-}
-
 // z = M r32, zr, beta, p update
 // z = M r (the FP32 V-cycle), z . r, beta and p = z + beta p
 static void enqueue_precondition(icarat_ctx *c, int smooth, int first)
@@ -517,11 +498,12 @@ static void enqueue_krylov_step(icarat_ctx *c, int krylov_op, const double *b, d
   if(krylov_op == ICARAT_OP_FP32)
   {
     int blocks;
-    const MarchPlan m = march_launch(L.g, (const void *)k_mx_spmv, 128, c->sm_count, blocks);
+    size_t smem;
+    const ModalPlan m =
+        modal_launch<float>(L.g, (const void *)k_mx_spmv, c->sm_count, kMaxRedBlocks, blocks, smem);
     note_launch();
-    launch_chained(k_mx_spmv, blocks < kMaxRedBlocks ? blocks : kMaxRedBlocks, 128, 0,
-                   c->stream, L.g, m, c->ke0f, L.E32, L.fix, c->f_p, c->f_Ap, c->d_partials,
-                   c->d_mx);
+    launch_chained(k_mx_spmv, blocks, ModalCfg<float>::threads, smem, c->stream, L.g, m, c->khf,
+                   L.E32, L.fix, c->f_p, c->f_Ap, c->d_partials, c->d_mx);
   }
   else
   {
@@ -540,11 +522,12 @@ static void enqueue_krylov_step(icarat_ctx *c, int krylov_op, const double *b, d
                  c->f_p, c->f_Ap, c->d_partials, c->d_mx);
   launch_chained(k_mx_flush, c->red_blocks, kRedThreads, 0, c->stream, n, x, c->f_x, c->d_mx);
   int rblocks;
-  const MarchPlan rm =
-      march_launch(L.g, (const void *)k_mx_residual, 128, c->sm_count, rblocks);
-  launch_chained(k_mx_residual, rblocks < kMaxRedBlocks ? rblocks : kMaxRedBlocks, 128, 0,
-                 c->stream, L.g, rm, c->ke0, c->d_E, L.fix, b, (const double *)x, c->f_r,
-                 c->d_partials, c->d_mx);
+  size_t smem;
+  const ModalPlan rm =
+      modal_launch<double>(L.g, (const void *)k_mx_residual,
+                           c->sm_count, kMaxRedBlocks, rblocks, smem);
+  launch_chained(k_mx_residual, rblocks, ModalCfg<double>::threads, smem, c->stream, L.g, rm,
+                 c->kh, c->d_E, L.fix, b, (const double *)x, c->f_r, c->d_partials, c->d_mx);
 }
 
 static const MxScalars &read_scalars(icarat_ctx *c)
@@ -609,9 +592,14 @@ void mixed_begin(icarat_ctx *c, const icarat_solve_opts *o, const double *d_b, d
   if(o->warm_start || learned)
   {
     const MgLevel &L0 = c->mg[0];
-    k_mx_init_warm<<<spmv_blocks(c), 128, 0, c->stream>>>(L0.g, c->ke0, c->d_E, L0.fix, d_b,
-                                                          d_x, c->f_x, c->f_r, c->d_partials,
-                                                          c->d_mx, o->rtol, delta, o->maxit);
+    int blocks;
+    size_t smem;
+    const ModalPlan m =
+        modal_launch<double>(L0.g, (const void *)k_mx_init_warm,
+                             c->sm_count, kMaxRedBlocks, blocks, smem);
+    k_mx_init_warm<<<blocks, ModalCfg<double>::threads, smem, c->stream>>>(
+        L0.g, m, c->kh, c->d_E, L0.fix, d_b, d_x, c->f_x, c->f_r, c->d_partials, c->d_mx, o->rtol,
+        delta, o->maxit);
   }
   else
     k_mx_init<<<c->red_blocks, kRedThreads, 0, c->stream>>>(

@@ -26,6 +26,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "modal.cuh"
 #include "stencil.cuh"
 
 namespace icarat_b200
@@ -174,68 +175,73 @@ __global__ void k_cheb_first(int n, const T *__restrict__ b, const T *__restrict
 
 // One Chebyshev step: r = b - K x, d = c1 d + c2 invd r, xo = x + d.
 // x and xo are distinct buffers (neighbours of x are read by other threads).
-template <typename T, typename KP>
-__global__ void __launch_bounds__(128)
-    k_cheb_step(GridDev g, MarchPlan m, KP ke, const T *__restrict__ E,
+template <typename T>
+__global__ void __launch_bounds__(ModalCfg<T>::threads, ModalCfg<T>::blocks)
+    k_cheb_step(GridDev g, ModalPlan m, KhParam<T> kh, const T *__restrict__ E,
                 const uint8_t *__restrict__ fix, const T *__restrict__ invd,
                 const T *__restrict__ b, const T *__restrict__ x, T *__restrict__ d,
                 T *__restrict__ xo, T c1, T c2, const int *__restrict__ halt)
 {
   chain_wait();
+  ModalShared<T> &ms = modal_shared<T>();
   if(halted(halt))
     return;
-  for(long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < m.items;
-      t += (long)gridDim.x * blockDim.x)
+  struct Pre
   {
-    int i, j, k0, k1;
-    if(!march_item(g, m, t, i, j, k0, k1))
-      continue;
-    column_Ku(g, ke, E, x, i, j, k0, k1,
-              [&](int k, const T(&acc)[3], const T(&uc)[3])
+    ModalRhs<T> r;
+    T invd[3], d[3];
+  };
+  modal_march(g, m, kh, E, x, ms,
+              [&](int n) {
+                Pre pre;
+                pre.r = modal_rhs(g, fix, b, n);
+#pragma unroll
+                for(int q = 0; q < 3; q++)
+                {
+                  const long id = (long)q * g.numnp + n;
+                  pre.invd[q] = invd[id];
+                  pre.d[q] = c1 != T(0) ? d[id] : T(0);
+                }
+                return pre;
+              },
+              [&](int n, const T(&acc)[3], const T(&uc)[3], const Pre &pre)
               {
-                const int n = i + j * g.NX + k * g.NX * g.NY;
-                const unsigned f = fix[n];
+                const unsigned f = pre.r.fix;
 #pragma unroll
                 for(int q = 0; q < 3; q++)
                 {
                   const long id = (long)q * g.numnp + n;
                   T dn = 0;
                   if(!((f >> q) & 1u))
-                    dn = (c1 != T(0) ? c1 * d[id] : T(0)) + c2 * invd[id] * (b[id] - acc[q]);
+                    dn = (c1 != T(0) ? c1 * pre.d[q] : T(0)) +
+                         c2 * pre.invd[q] * (pre.r.b[q] - acc[q]);
                   d[id] = dn;
                   xo[id] = uc[q] + dn;
                 }
               });
-  }
 }
 
 // r = b - K x (constrained rows 0)
-template <typename T, typename KP>
-__global__ void __launch_bounds__(128)
-    k_mg_residual(GridDev g, MarchPlan m, KP ke, const T *__restrict__ E,
+template <typename T>
+__global__ void __launch_bounds__(ModalCfg<T>::threads, ModalCfg<T>::blocks)
+    k_mg_residual(GridDev g, ModalPlan m, KhParam<T> kh, const T *__restrict__ E,
                   const uint8_t *__restrict__ fix, const T *__restrict__ b,
                   const T *__restrict__ x, T *__restrict__ r, const int *__restrict__ halt)
 {
   chain_wait();
+  ModalShared<T> &ms = modal_shared<T>();
   if(halted(halt))
     return;
-  for(long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < m.items;
-      t += (long)gridDim.x * blockDim.x)
-  {
-    int i, j, k0, k1;
-    if(!march_item(g, m, t, i, j, k0, k1))
-      continue;
-    column_Ku(g, ke, E, x, i, j, k0, k1,
-              [&](int k, const T(&acc)[3], const T(&)[3])
+  modal_march(g, m, kh, E, x, ms,
+              [&](int n) { return modal_rhs(g, fix, b, n); },
+              [&](int n, const T(&acc)[3], const T(&)[3], const ModalRhs<T> &pre)
               {
-                const int n = i + j * g.NX + k * g.NX * g.NY;
-                const unsigned f = fix[n];
+                const unsigned f = pre.fix;
 #pragma unroll
                 for(int c = 0; c < 3; c++)
                   r[(long)c * g.numnp + n] =
-                      ((f >> c) & 1u) ? T(0) : b[(long)c * g.numnp + n] - acc[c];
+                      ((f >> c) & 1u) ? T(0) : pre.b[c] - acc[c];
               });
-  }
 }
 
 // ---------------------------------------------------------------- coarse
@@ -317,7 +323,7 @@ template <> struct LevelBuf<double>
   static double *r(MgLevel &L) { return L.r; }
   static double *t(MgLevel &L) { return L.t; }
   static double *S(MgLevel &L) { return L.S; }
-  static const KeParam &ke(icarat_ctx *c) { return c->ke0; }
+  static const KhParam<double> &kh(icarat_ctx *c) { return c->kh; }
 };
 template <> struct LevelBuf<float>
 {
@@ -328,7 +334,7 @@ template <> struct LevelBuf<float>
   static float *r(MgLevel &L) { return L.r32; }
   static float *t(MgLevel &L) { return L.t32; }
   static float *S(MgLevel &L) { return L.S32; }
-  static const KeParamF &ke(icarat_ctx *c) { return c->ke0f; }
+  static const KhParam<float> &kh(icarat_ctx *c) { return c->khf; }
 };
 
 void mg_free(icarat_ctx *c)
@@ -895,12 +901,12 @@ static void cheb_step(icarat_ctx *c, MgLevel &L, int lvl, const T *b, const T *x
       return;
     }
   int blocks;
-  const MarchPlan m =
-      march_launch(L.g, (const void *)k_cheb_step<T, typename KeOf<T>::type>, 128,
-                   c->sm_count, blocks);
+  size_t smem;
+  const ModalPlan m =
+      modal_launch<T>(L.g, (const void *)k_cheb_step<T>, c->sm_count, 1 << 30, blocks, smem);
   note_launch();
-  launch_chained(k_cheb_step<T, typename KeOf<T>::type>, blocks, 128, 0, c->stream, L.g, m,
-                 B::ke(c), B::E(L), L.fix, B::invd(L), b, x, d, xo, T(c1), T(c2), c->mg_halt);
+  launch_chained(k_cheb_step<T>, blocks, ModalCfg<T>::threads, smem, c->stream, L.g, m, B::kh(c),
+                 B::E(L), L.fix, B::invd(L), b, x, d, xo, T(c1), T(c2), c->mg_halt);
 }
 
 // r = b - K x on level lvl
@@ -941,12 +947,12 @@ static void mg_residual(icarat_ctx *c, MgLevel &L, int lvl, const T *b, const T 
       return;
     }
   int blocks;
-  const MarchPlan m =
-      march_launch(L.g, (const void *)k_mg_residual<T, typename KeOf<T>::type>, 128,
-                   c->sm_count, blocks);
+  size_t smem;
+  const ModalPlan m =
+      modal_launch<T>(L.g, (const void *)k_mg_residual<T>, c->sm_count, 1 << 30, blocks, smem);
   note_launch();
-  launch_chained(k_mg_residual<T, typename KeOf<T>::type>, blocks, 128, 0, c->stream, L.g, m,
-                 B::ke(c), B::E(L), L.fix, b, x, r, c->mg_halt);
+  launch_chained(k_mg_residual<T>, blocks, ModalCfg<T>::threads, smem, c->stream, L.g, m, B::kh(c),
+                 B::E(L), L.fix, b, x, r, c->mg_halt);
 }
 
 // Chebyshev smoothing of K x = b on level lvl, deg steps.  from_zero: x = 0

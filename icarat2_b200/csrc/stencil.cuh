@@ -6,25 +6,10 @@
 // write the same output and no atomics or colouring are needed.  Ke0 is a
 // by-value kernel parameter (constant bank).
 #pragma once
-#include <map>
-#include <mutex>
-#include <utility>
-
 #include "internal.cuh"
 
 namespace icarat_b200
 {
-
-// element matrix of the value type T (the FP32 copy is rounded from FP64)
-template <typename T> struct KeOf;
-template <> struct KeOf<double>
-{
-  using type = KeParam;
-};
-template <> struct KeOf<float>
-{
-  using type = KeParamF;
-};
 
 // local node number of the corner (lx, ly, lz) of a hexa8
 // (mesh_icarat.hpp:489-509 order)
@@ -272,79 +257,6 @@ __device__ __forceinline__ void column_Ku(const GridDev &g, const KP &ke,
       for(int d = 0; d < 3; d++)
         ul[0][s][d] = ul[1][s][d];
   }
-}
-
-// Work items of a column march: ncol columns (NX NY rounded up to whole
-// warps, so a warp never straddles two z chunks) times ceil(NZ / kc) chunks.
-struct MarchPlan
-{
-  int kc, ncol;
-  long items;
-};
-
-// node layers per chunk: the largest count that still gives every resident
-// thread slot (slots) about two items, down to one layer per item on the
-// small multigrid levels, which are latency-bound (their operands sit in L2,
-// so the layers a short chunk re-reads cost little; results do not depend on
-// the chunking)
-inline MarchPlan march_plan(const GridDev &g, long slots)
-{
-  MarchPlan m;
-  m.ncol = ((g.NX * g.NY + 31) / 32) * 32;
-  int kc = g.NZ;
-  while(kc > 1 && (long)m.ncol * ((g.NZ + kc - 1) / kc) < 2 * slots)
-    kc = (kc + 1) / 2;
-  m.kc = kc < 1 ? 1 : kc;
-  m.items = (long)m.ncol * ((g.NZ + m.kc - 1) / m.kc);
-  return m;
-}
-
-// resident threads of `kernel` at `threads` per block on the whole GPU
-// (occupancy cached per kernel)
-inline long resident_threads(const void *kernel, int threads, int sms)
-{
-  static std::mutex mu;
-  static std::map<std::pair<const void *, int>, int> cache;
-  std::lock_guard<std::mutex> lock(mu);
-  auto key = std::make_pair(kernel, threads);
-  auto it = cache.find(key);
-  int occ;
-  if(it == cache.end())
-  {
-    occ = 0;
-    if(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, 0) != cudaSuccess ||
-       occ < 1)
-      occ = 1;
-    cache[key] = occ;
-  }
-  else
-    occ = it->second;
-  return (long)occ * threads * sms;
-}
-
-// plan and block count of a column-march launch of `kernel`
-inline MarchPlan march_launch(const GridDev &g, const void *kernel, int threads, int sms,
-                              int &blocks)
-{
-  const MarchPlan m = march_plan(g, resident_threads(kernel, threads, sms));
-  const long b = (m.items + threads - 1) / threads;
-  blocks = (int)(b < 1 ? 1 : b);
-  return m;
-}
-
-// the column and z range of item t; false for the padding columns
-__device__ __forceinline__ bool march_item(const GridDev &g, const MarchPlan &m, long t,
-                                           int &i, int &j, int &k0, int &k1)
-{
-  const int col = (int)(t % m.ncol);
-  const int chunk = (int)(t / m.ncol);
-  if(col >= g.NX * g.NY)
-    return false;
-  i = col % g.NX;
-  j = col / g.NX;
-  k0 = chunk * m.kc;
-  k1 = k0 + m.kc < g.NZ ? k0 + m.kc : g.NZ;
-  return true;
 }
 
 } // namespace icarat_b200

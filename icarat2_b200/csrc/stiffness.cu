@@ -4,39 +4,33 @@
 // (src/analysis/linear.hpp:117-166, src/analysis/solver/CG.cpp:76-99).
 // Work per node: 8 elements x 3 rows x 24 = 576 DFMA (1152 flop); compulsory
 // bytes per node: 24 read + 24 written (+ 8 per element modulus).
+#include "modal.cuh"
 #include "stencil.cuh"
 
 namespace icarat_b200
 {
 
 // y = K u (constrained rows zeroed); optional per-block partial of u . y.
-__global__ void __launch_bounds__(128)
-    k_apply_K_f64(GridDev g, MarchPlan m, KeParam ke, const double *__restrict__ E,
+__global__ void __launch_bounds__(ModalCfg<double>::threads, ModalCfg<double>::blocks)
+    k_apply_K_f64(GridDev g, ModalPlan m, KhParam<double> kh, const double *__restrict__ E,
                   const uint8_t *__restrict__ fix, const double *__restrict__ u,
                   double *__restrict__ y, double *__restrict__ partials)
 {
+  ModalShared<double> &ms = modal_shared<double>();
   __shared__ double sh[32];
   double dot = 0.0;
-  for(long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < m.items;
-      t += (long)gridDim.x * blockDim.x)
-  {
-    int i, j, k0, k1;
-    if(!march_item(g, m, t, i, j, k0, k1))
-      continue;
-    column_Ku(g, ke, E, u, i, j, k0, k1,
-              [&](int k, const double(&acc)[3], const double(&uc)[3])
+  modal_march(g, m, kh, E, u, ms,
+              [&](int n) { return (unsigned)fix[n]; },
+              [&](int n, const double(&acc)[3], const double(&uc)[3], unsigned f)
               {
-                const int n = i + j * g.NX + k * g.NX * g.NY;
-                const unsigned f = fix[n];
-                const double y0 = (f & 1u) ? 0.0 : acc[0];
-                const double y1 = (f & 2u) ? 0.0 : acc[1];
-                const double y2 = (f & 4u) ? 0.0 : acc[2];
-                y[n] = y0;
-                y[(long)g.numnp + n] = y1;
-                y[2L * g.numnp + n] = y2;
-                dot += uc[0] * y0 + uc[1] * y1 + uc[2] * y2;
+#pragma unroll
+                for(int q = 0; q < 3; q++)
+                {
+                  const double yq = ((f >> q) & 1u) ? 0.0 : acc[q];
+                  y[(long)q * g.numnp + n] = yq;
+                  dot += uc[q] * yq;
+                }
               });
-  }
   if(partials)
   {
     double v[1] = {dot};
@@ -77,24 +71,6 @@ __global__ void k_inv_diag(GridDev g, KeParam ke, const double *__restrict__ E,
       // a zero diagonal is treated as 1, as Eigen's DiagonalPreconditioner
       // does for the "Eigen_CG" solver (solvers.cpp:63-91)
       invd[(long)c * g.numnp + n] = ((f >> c) & 1u) ? 0.0 : (d[c] != 0.0 ? 1.0 / d[c] : 1.0);
-  }
-}
-
-// r = b - K x (constrained rows 0).  Used by multigrid.
-__global__ void __launch_bounds__(128)
-    k_residual_f64(GridDev g, KeParam ke, const double *__restrict__ E,
-                   const uint8_t *__restrict__ fix, const double *__restrict__ b,
-                   const double *__restrict__ x, double *__restrict__ r)
-{
-  for(int n = blockIdx.x * blockDim.x + threadIdx.x; n < g.numnp;
-      n += gridDim.x * blockDim.x)
-  {
-    double acc[3], uc[3];
-    node_Ku(g, ke, E, x, n, acc, uc);
-    const unsigned f = fix[n];
-#pragma unroll
-    for(int c = 0; c < 3; c++)
-      r[(long)c * g.numnp + n] = ((f >> c) & 1u) ? 0.0 : b[(long)c * g.numnp + n] - acc[c];
   }
 }
 
@@ -179,45 +155,42 @@ void launch_apply_K(icarat_ctx *c, const GridDev &g, const double *E,
     return;
   }
   int blocks;
-  const MarchPlan m = march_launch(g, (const void *)k_apply_K_f64, 128, c->sm_count, blocks);
-  if(dot_partials && blocks > kMaxRedBlocks)
-    blocks = kMaxRedBlocks;
+  size_t smem;
+  const ModalPlan m =
+      modal_launch<double>(g, (const void *)k_apply_K_f64,
+                           c->sm_count, kMaxRedBlocks, blocks, smem);
   note_launch();
-  k_apply_K_f64<<<blocks, 128, 0, c->stream>>>(g, m, c->ke0, E, fix, u, y, dot_partials);
+  k_apply_K_f64<<<blocks, ModalCfg<double>::threads, smem, c->stream>>>(g, m, c->kh, E, fix, u, y,
+                                                         dot_partials);
   ICK(cudaGetLastError());
 }
 
 // y = K u in FP32 (the FP32 copies of Ke0 and of the moduli)
-__global__ void __launch_bounds__(128)
-    k_apply_K_f32(GridDev g, MarchPlan m, KeParamF ke, const float *__restrict__ E,
+__global__ void __launch_bounds__(ModalCfg<float>::threads, ModalCfg<float>::blocks)
+    k_apply_K_f32(GridDev g, ModalPlan m, KhParam<float> kh, const float *__restrict__ E,
                   const uint8_t *__restrict__ fix, const float *__restrict__ u,
                   float *__restrict__ y)
 {
-  for(long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < m.items;
-      t += (long)gridDim.x * blockDim.x)
-  {
-    int i, j, k0, k1;
-    if(!march_item(g, m, t, i, j, k0, k1))
-      continue;
-    column_Ku(g, ke, E, u, i, j, k0, k1,
-              [&](int k, const float(&acc)[3], const float(&)[3])
+  ModalShared<float> &ms = modal_shared<float>();
+  modal_march(g, m, kh, E, u, ms,
+              [&](int n) { return (unsigned)fix[n]; },
+              [&](int n, const float(&acc)[3], const float(&)[3], unsigned f)
               {
-                const int n = i + j * g.NX + k * g.NX * g.NY;
-                const unsigned f = fix[n];
 #pragma unroll
                 for(int c = 0; c < 3; c++)
                   y[(long)c * g.numnp + n] = ((f >> c) & 1u) ? 0.0f : acc[c];
               });
-  }
 }
 
 void launch_apply_K_f32(icarat_ctx *c, const GridDev &g, const float *E,
                         const uint8_t *fix, const float *u, float *y)
 {
   int blocks;
-  const MarchPlan m = march_launch(g, (const void *)k_apply_K_f32, 128, c->sm_count, blocks);
+  size_t smem;
+  const ModalPlan m =
+      modal_launch<float>(g, (const void *)k_apply_K_f32, c->sm_count, 1 << 30, blocks, smem);
   note_launch();
-  k_apply_K_f32<<<blocks, 128, 0, c->stream>>>(g, m, c->ke0f, E, fix, u, y);
+  k_apply_K_f32<<<blocks, ModalCfg<float>::threads, smem, c->stream>>>(g, m, c->khf, E, fix, u, y);
   ICK(cudaGetLastError());
 }
 
@@ -226,16 +199,6 @@ void launch_diag(icarat_ctx *c, const GridDev &g, const double *E,
 {
   note_launch();
   k_inv_diag<<<node_blocks(g, 256), 256, 0, st ? st : c->stream>>>(g, c->ke0, E, fix, invd);
-  ICK(cudaGetLastError());
-}
-
-void launch_residual(icarat_ctx *c, const GridDev &g, const double *E,
-                     const uint8_t *fix, const double *b, const double *x,
-                     double *r)
-{
-  note_launch();
-  k_residual_f64<<<node_blocks(g, 128), 128, 0, c->stream>>>(g, c->ke0, E, fix,
-                                                             b, x, r);
   ICK(cudaGetLastError());
 }
 
