@@ -7,8 +7,11 @@
 // id (dk, dj, di lexicographic), weight w = R - d.  The kernels accumulate in
 // that order with separate multiply and add (no contraction), so forward and
 // transposed results match the reference loop operation for operation.
+#include <algorithm>
+#include <atomic>
 #include <cmath>
 
+#include "filter_tile.cuh"
 #include "internal.cuh"
 
 namespace icarat_b200
@@ -172,6 +175,99 @@ __global__ void k_filter_trans2(ElemGrid g, int nofs, const int *__restrict__ of
   }
 }
 
+// forward on a compiled ball: one staged array, a_i from the set-up (the same
+// sum in the same order)
+template <int D2>
+__global__ void __launch_bounds__(kBallX *kBallY)
+    k_ball_fwd(BallGrid g, const __grid_constant__ BallWeights<D2> W, const double *__restrict__ aa,
+               const double *__restrict__ in, double *__restrict__ out)
+{
+  extern __shared__ double s_ball[];
+  int x0, y0, z0;
+  ball_origin(g, blockIdx.x, x0, y0, z0);
+  ball_stage<D2>(g, x0, y0, z0, [&](int q, int e) { ball_copy(s_ball + q, in, e); });
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
+  __syncthreads();
+  double acc[kBallZ];
+#pragma unroll
+  for(int o = 0; o < kBallZ; o++)
+    acc[o] = 0.0;
+  ball_sum<D2>([&](int at) { return s_ball[at]; },
+               [&](int o, int t, double v) { acc[o] = __dadd_rn(acc[o], __dmul_rn(W.w[t], v)); });
+  const int x = x0 + threadIdx.x % kBallX, y = y0 + threadIdx.x / kBallX;
+  if(x >= g.nx || y >= g.ny)
+    return;
+#pragma unroll
+  for(int o = 0; o < kBallZ; o++)
+    if(z0 + o < g.nz)
+    {
+      const int e = x + y * g.nx + (z0 + o) * g.nx * g.ny;
+      out[e] = (g.mask && !g.mask[e]) ? 0.0 : __ddiv_rn(acc[o], aa[e]);
+    }
+}
+
+// transposed on a compiled ball, NIN inputs at once; a_j and its reciprocal
+// are staged beside the inputs
+template <int D2, int NIN>
+__global__ void __launch_bounds__(kBallX *kBallY)
+    k_ball_trans(BallGrid g, const __grid_constant__ BallWeights<D2> W, const double *__restrict__ aa,
+                 const double *__restrict__ ra, const double *__restrict__ in1,
+                 const double *__restrict__ in2, double *__restrict__ out1,
+                 double *__restrict__ out2)
+{
+  constexpr int tile = Ball<D2>::tile;
+  extern __shared__ double s_ball[];
+  double *s_a = s_ball, *s_r = s_ball + tile, *s_1 = s_ball + 2 * tile, *s_2 = s_ball + 3 * tile;
+  int x0, y0, z0;
+  ball_origin(g, blockIdx.x, x0, y0, z0);
+  ball_stage<D2>(g, x0, y0, z0, [&](int q, int e) {
+    ball_copy(s_a + q, aa, e);
+    ball_copy(s_r + q, ra, e);
+    ball_copy(s_1 + q, in1, e);
+    if(NIN == 2)
+      ball_copy(s_2 + q, in2, e);
+  });
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
+  __syncthreads();
+  double acc[NIN][kBallZ];
+#pragma unroll
+  for(int o = 0; o < kBallZ; o++)
+    for(int q = 0; q < NIN; q++)
+      acc[q][o] = 0.0;
+  struct Value
+  {
+    double a, r, v[NIN];
+  };
+  ball_sum<D2>(
+      [&](int at) {
+        Value v;
+        v.a = s_a[at];
+        v.r = s_r[at];
+        v.v[0] = s_1[at];
+        if(NIN == 2)
+          v.v[NIN - 1] = s_2[at];
+        return v;
+      },
+      [&](int o, int t, const Value &v) {
+#pragma unroll
+        for(int q = 0; q < NIN; q++)
+          acc[q][o] = __dadd_rn(acc[q][o], div_by_recip(__dmul_rn(W.w[t], v.v[q]), v.a, v.r));
+      });
+  const int x = x0 + threadIdx.x % kBallX, y = y0 + threadIdx.x / kBallX;
+  if(x >= g.nx || y >= g.ny)
+    return;
+#pragma unroll
+  for(int o = 0; o < kBallZ; o++)
+    if(z0 + o < g.nz)
+    {
+      const int e = x + y * g.nx + (z0 + o) * g.nx * g.ny;
+      const bool keep = !(g.mask && !g.mask[e]);
+      out1[e] = keep ? acc[0][o] : 0.0;
+      if(NIN == 2)
+        out2[e] = keep ? acc[NIN - 1][o] : 0.0;
+    }
+}
+
 // sensitivityFilter (filter.hpp:77-104)
 __global__ void k_sens_filter(ElemGrid g, int nofs, const int *__restrict__ ofs,
                               const double *__restrict__ w, double vol,
@@ -225,6 +321,29 @@ static ElemGrid egrid(const icarat_ctx *c)
   return ElemGrid{c->nx, c->ny, c->nz, c->nelx, c->d_emask};
 }
 
+static BallGrid bgrid(const icarat_ctx *c)
+{
+  return BallGrid{c->nx, c->ny, c->nz, c->nelx, c->d_emask};
+}
+
+// dynamic shared memory of Arrays staged arrays of ball D2, the kernel's limit
+// raised (once per device) where that passes 48 KB
+template <int D2, int Arrays> static size_t ball_smem(const void *kernel)
+{
+  static std::atomic<bool> ready[kMaxDevices];
+  const size_t n = sizeof(double) * (size_t)Arrays * Ball<D2>::tile;
+  if(n > 48 * 1024)
+  {
+    const int d = device_slot();
+    if(!ready[d].load())
+    {
+      ICK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)n));
+      ready[d].store(true);
+    }
+  }
+  return n;
+}
+
 static int eblocks(const icarat_ctx *c)
 {
   int b = (c->nelx + 255) / 256;
@@ -238,6 +357,41 @@ void filter_free(icarat_ctx *c)
   dfree(c->filt.d_aa);
   dfree(c->filt.d_ra);
   c->filt = FilterState{};
+}
+
+// The compiled ball whose taps are exactly the list's, with its octant of
+// weights in cube, or 0 (larger radii, stretched voxels).
+static int find_ball(const FilterState &F, std::vector<double> &cube)
+{
+  int found = 0;
+  for(int d2 : {1, 2, 3, 4, 5, 6, 8, 9})
+    ball_dispatch(d2, [&](auto D) {
+      using B = Ball<decltype(D)::value>;
+      int n = 0;
+      bool same = true;
+      std::vector<double> w(B::weights, -1.0);
+      for(int dk = -B::r; dk <= B::r; dk++)
+        for(int dj = -B::r; dj <= B::r; dj++)
+          for(int di = -B::r; di <= B::r; di++)
+            if(B::in(dk, dj, di))
+            {
+              same = same && n < F.nofs && F.ofs[3 * n] == di && F.ofs[3 * n + 1] == dj &&
+                     F.ofs[3 * n + 2] == dk;
+              if(same)
+              {
+                double &v = w[B::index(dk, dj, di)];
+                same = v == -1.0 || v == F.w[n]; // weights are >= 0
+                v = F.w[n];
+              }
+              n++;
+            }
+      if(same && n == F.nofs)
+      {
+        found = D();
+        cube = w;
+      }
+    });
+  return found;
 }
 
 void filter_setup(icarat_ctx *c, double R)
@@ -264,6 +418,7 @@ void filter_setup(icarat_ctx *c, double R)
         }
       }
   F.nofs = (int)F.w.size();
+  F.ball = find_ball(F, F.cube);
   ICK(cudaMalloc(&F.d_ofs, sizeof(int) * F.ofs.size()));
   ICK(cudaMemcpy(F.d_ofs, F.ofs.data(), sizeof(int) * F.ofs.size(),
                  cudaMemcpyHostToDevice));
@@ -281,6 +436,36 @@ void filter_setup(icarat_ctx *c, double R)
   F.have_forward = false;
 }
 
+template <int D2> static BallWeights<D2> ball_weights(const FilterState &F)
+{
+  BallWeights<D2> W;
+  std::copy(F.cube.begin(), F.cube.end(), W.w);
+  return W;
+}
+
+// The compiled ball is the faster form from about 1e5 taps in all: below, the
+// launch is all the time there is and the tile's halo only adds to it (7 taps
+// on 7 k elements: 5.8 us by the list, 6.6 staged; 19 taps: 8.3 and 6.0).
+static bool use_ball(const icarat_ctx *c)
+{
+  return c->filt.ball > 0 && (double)c->filt.nofs * c->nelx >= 1.0e5 &&
+         ball_blocks(c->nx, c->ny, c->nz) < (1L << 31);
+}
+
+template <int NIN>
+static void launch_ball_trans(icarat_ctx *c, const double *in1, const double *in2, double *out1,
+                              double *out2)
+{
+  const FilterState &F = c->filt;
+  ball_dispatch(F.ball, [&](auto D) {
+    constexpr int d2 = decltype(D)::value;
+    const auto kernel = k_ball_trans<d2, NIN>;
+    kernel<<<(unsigned)ball_blocks(c->nx, c->ny, c->nz), kBallX * kBallY,
+             ball_smem<d2, 2 + NIN>((const void *)kernel), c->stream>>>(
+        bgrid(c), ball_weights<d2>(F), F.d_aa, F.d_ra, in1, in2, out1, out2);
+  });
+}
+
 // The forward pass fails like the reference when a weight sum is below 1e-10
 // (filter.hpp:130-134); that can only happen for R < 1e-10.
 void filter_apply(icarat_ctx *c, const double *in, double *out, bool is_sens)
@@ -292,8 +477,15 @@ void filter_apply(icarat_ctx *c, const double *in, double *out, bool is_sens)
     IREQUIRE(F.radius >= 1.0e-10, ICARAT_ERR_FILTER,
              "coefficient aa is too small in the density filter");
     note_launch();
-    k_filter_fwd<<<eblocks(c), 256, 0, c->stream>>>(egrid(c), F.nofs, F.d_ofs, F.d_w,
-                                                    in, out);
+    if(use_ball(c))
+      ball_dispatch(F.ball, [&](auto D) {
+        constexpr int d2 = decltype(D)::value;
+        k_ball_fwd<d2><<<(unsigned)ball_blocks(c->nx, c->ny, c->nz), kBallX * kBallY,
+                         ball_smem<d2, 1>((const void *)k_ball_fwd<d2>), c->stream>>>(
+            bgrid(c), ball_weights<d2>(F), F.d_aa, in, out);
+      });
+    else
+      k_filter_fwd<<<eblocks(c), 256, 0, c->stream>>>(egrid(c), F.nofs, F.d_ofs, F.d_w, in, out);
     F.have_forward = true;
   }
   else
@@ -301,8 +493,11 @@ void filter_apply(icarat_ctx *c, const double *in, double *out, bool is_sens)
     IREQUIRE(F.have_forward, ICARAT_ERR_STATE,
              "transposed filter needs a forward call first (filter.hpp:140-153)");
     note_launch();
-    k_filter_trans<<<eblocks(c), 256, 0, c->stream>>>(egrid(c), F.nofs, F.d_ofs,
-                                                      F.d_w, F.d_aa, F.d_ra, in, out);
+    if(use_ball(c))
+      launch_ball_trans<1>(c, in, nullptr, out, nullptr);
+    else
+      k_filter_trans<<<eblocks(c), 256, 0, c->stream>>>(egrid(c), F.nofs, F.d_ofs, F.d_w, F.d_aa,
+                                                        F.d_ra, in, out);
   }
   ICK(cudaGetLastError());
 }
@@ -316,8 +511,11 @@ void filter_trans2(icarat_ctx *c, const double *in1, const double *in2, double *
   IREQUIRE(F.have_forward, ICARAT_ERR_STATE,
            "transposed filter needs a forward call first (filter.hpp:140-153)");
   note_launch();
-  k_filter_trans2<<<eblocks(c), 256, 0, c->stream>>>(egrid(c), F.nofs, F.d_ofs, F.d_w, F.d_aa,
-                                                     F.d_ra, in1, in2, out1, out2);
+  if(use_ball(c))
+    launch_ball_trans<2>(c, in1, in2, out1, out2);
+  else
+    k_filter_trans2<<<eblocks(c), 256, 0, c->stream>>>(egrid(c), F.nofs, F.d_ofs, F.d_w, F.d_aa,
+                                                       F.d_ra, in1, in2, out1, out2);
   ICK(cudaGetLastError());
 }
 

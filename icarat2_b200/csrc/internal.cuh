@@ -286,6 +286,8 @@ struct FilterState
   int rx = 0, ry = 0, rz = 0;   // index reach per axis
   std::vector<int> ofs;         // 3 * nofs (di, dj, dk), ascending element id
   std::vector<double> w;        // nofs weights R - d
+  int ball = 0;                 // compiled ball of these taps (filter_tile.cuh), 0: none
+  std::vector<double> cube;     // its weights, one octant
   int *d_ofs = nullptr;
   double *d_w = nullptr;
   double *d_aa = nullptr;       // nelx sums of weights (dfilters_ds)

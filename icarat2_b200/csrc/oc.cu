@@ -10,8 +10,10 @@
 // same lambda decision without another barrier or a host round trip.
 #include <cooperative_groups.h>
 
+#include <algorithm>
 #include <cmath>
 
+#include "filter_tile.cuh"
 #include "internal.cuh"
 
 namespace cg = cooperative_groups;
@@ -117,6 +119,88 @@ __global__ void __launch_bounds__(256) k_oc_bisect(OcArgs a)
   }
 }
 
+// The same bisection with the filter of a compiled ball (filter_tile.cuh): the
+// blocks walk the tiles, a_i comes from the filter's set-up.  The trial
+// densities are read through L2 (other blocks wrote them in this launch).
+template <int D2>
+__global__ void __launch_bounds__(kBallX *kBallY)
+    k_oc_bisect_ball(OcArgs a, const __grid_constant__ BallWeights<D2> W,
+                     const double *__restrict__ aa, int tiles)
+{
+  cg::grid_group grid = cg::this_grid();
+  extern __shared__ double s_ball[];
+  __shared__ double sh[32];
+  __shared__ double s_total;
+  const BallGrid g{a.nx, a.ny, a.nz, a.nelx, a.emask};
+  double l0 = a.lmin, l1 = a.lmax;
+  int counter = 0;
+  const double tb = a.use_thr ? tanh(a.T * a.beta) : 1.0;
+  const int tid = blockIdx.x * blockDim.x + threadIdx.x;
+  const int stride = gridDim.x * blockDim.x;
+  double lambda = 0.0;
+  while((l1 - l0) / (l1 + l0) > a.leps && a.maxiter > counter)
+  {
+    lambda = 0.5 * (l1 + l0);
+    for(int e = tid; e < a.nelx; e += stride)
+      a.xk[e] = (a.emask && !a.emask[e]) ? 0.0 : oc_trial(a, e, lambda);
+    grid.sync();
+    double part = 0.0;
+    for(int tile = blockIdx.x; tile < tiles; tile += gridDim.x)
+    {
+      int x0, y0, z0;
+      ball_origin(g, tile, x0, y0, z0);
+      __syncthreads(); // the previous tile has been read
+      ball_stage<D2>(g, x0, y0, z0,
+                     [&](int q, int e) { s_ball[q] = e >= 0 ? __ldcg(a.xk + e) : 0.0; });
+      __syncthreads();
+      double acc[kBallZ];
+#pragma unroll
+      for(int o = 0; o < kBallZ; o++)
+        acc[o] = 0.0;
+      ball_sum<D2>([&](int at) { return s_ball[at]; },
+                   [&](int o, int t, double v) {
+                     acc[o] = __dadd_rn(acc[o], __dmul_rn(W.w[t], v));
+                   });
+      const int x = x0 + threadIdx.x % kBallX, y = y0 + threadIdx.x / kBallX;
+      if(x < g.nx && y < g.ny)
+      {
+#pragma unroll
+        for(int o = 0; o < kBallZ; o++)
+        {
+          const int e = x + y * g.nx + (z0 + o) * g.nx * g.ny;
+          if(z0 + o < g.nz && !(g.mask && !g.mask[e]))
+          {
+            double rho = __ddiv_rn(acc[o], aa[e]);
+            if(a.use_thr)
+              rho = 0.5 * (tb + tanh(a.beta * (rho - a.T))) / tb;
+            part += rho * a.vol;
+          }
+        }
+      }
+    }
+    double v[1] = {part};
+    block_sum<1>(v, sh);
+    if(threadIdx.x == 0)
+      a.partials[blockIdx.x] = v[0];
+    grid.sync();
+    double t[1];
+    sum_partials<1>(a.partials, gridDim.x, t, sh);
+    if(threadIdx.x == 0)
+      s_total = t[0];
+    __syncthreads();
+    if(s_total - a.g > 0.0)
+      l0 = lambda;
+    else
+      l1 = lambda;
+    counter++;
+  }
+  if(blockIdx.x == 0 && threadIdx.x == 0)
+  {
+    a.result[0] = counter;
+    a.result[1] = lambda;
+  }
+}
+
 // one trial design of the bisection (the Helmholtz volume functor's input)
 __global__ void k_oc_trial(OcArgs a, double lambda)
 {
@@ -194,20 +278,41 @@ int oc_update_dev(icarat_ctx *c, double *x, const double *dfdx, double g,
   a.maxiter = o->maxiter;
   a.use_thr = o->use_threshold ? 1 : 0;
   a.emask = c->d_emask;
-  int per_sm = 0, sms = 0;
-  ICK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_oc_bisect, 256, 0));
+  int sms = 0;
   ICK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
-  int blocks = sms * (per_sm > 2 ? 2 : per_sm);
-  const int need = (c->nelx + 255) / 256;
-  if(blocks > need)
-    blocks = need;
-  if(blocks > kMaxRedBlocks)
-    blocks = kMaxRedBlocks;
-  IREQUIRE(blocks >= 1, ICARAT_ERR_CUDA, "no co-resident blocks for the OC kernel");
-  void *args[] = {&a};
+  // co-resident blocks for `need` blocks' work, at most `most` per SM
+  auto resident = [&](const void *kernel, int threads, size_t smem, int most, long need) {
+    int per_sm = 0;
+    ICK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
+    long blocks = (long)sms * (per_sm > most ? most : per_sm);
+    blocks = blocks > need ? need : blocks;
+    blocks = blocks > kMaxRedBlocks ? kMaxRedBlocks : blocks;
+    IREQUIRE(blocks >= 1, ICARAT_ERR_CUDA, "no co-resident blocks for the OC kernel");
+    return (int)blocks;
+  };
   note_launch();
-  ICK(cudaLaunchCooperativeKernel((void *)k_oc_bisect, dim3(blocks), dim3(256), args,
-                                  0, c->stream));
+  const long tiles = ball_blocks(c->nx, c->ny, c->nz);
+  if(c->filt.ball > 0 && tiles < (1L << 31))
+    ball_dispatch(c->filt.ball, [&](auto D) {
+      constexpr int d2 = decltype(D)::value;
+      const void *kernel = (const void *)k_oc_bisect_ball<d2>;
+      const size_t smem = sizeof(double) * Ball<d2>::tile;
+      static_assert(sizeof(double) * Ball<d2>::tile <= 48 * 1024, "tile above 48 KB");
+      BallWeights<d2> W;
+      std::copy(c->filt.cube.begin(), c->filt.cube.end(), W.w);
+      int nt = (int)tiles;
+      void *args[] = {&a, &W, &c->filt.d_aa, &nt};
+      const int threads = kBallX * kBallY;
+      ICK(cudaLaunchCooperativeKernel(kernel, dim3(resident(kernel, threads, smem, 4, tiles)),
+                                      dim3(threads), args, smem, c->stream));
+    });
+  else
+  {
+    void *args[] = {&a};
+    const int blocks = resident((const void *)k_oc_bisect, 256, 0, 2, (c->nelx + 255) / 256);
+    ICK(cudaLaunchCooperativeKernel((void *)k_oc_bisect, dim3(blocks), dim3(256), args, 0,
+                                    c->stream));
+  }
   ICK(cudaMemcpyAsync(c->h_scalar, c->d_scalar, 2 * sizeof(double),
                       cudaMemcpyDeviceToHost, c->stream));
   ICK(cudaStreamSynchronize(c->stream));
