@@ -1,6 +1,7 @@
 // Context setup: structured hexa8 box, Dirichlet boxes, DOF numbering, point
 // loads, device arrays, and the numeq <-> node-vector conversions.
 #include <climits>
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cstdio>
@@ -635,8 +636,11 @@ int icarat_ctx_create_sel_impl(const icarat_grid *grid, const icarat_material *m
       ICK(cudaMemset(c->d_tc_err, 0, sizeof(int)));
     }
     // streaming CG kernels at full occupancy (8 blocks of 256 threads per
-    // SM): with 4 per SM they reached 3-4 TB/s on the B200
+    // SM): with 4 per SM they reached 3-4 TB/s on the B200.  Small grids take
+    // a block per 512 values: every block's partial sums are read again by
+    // the last one (1184 of them cost 10.4 us a reduction on 28 k values)
     c->red_blocks = sms * 8 > kMaxRedBlocks ? kMaxRedBlocks : sms * 8;
+    c->red_blocks = std::max(1, std::min(c->red_blocks, (c->neq + 511) / 512));
     // icarat_solve_noalloc's buffer: its address is taken here, where the
     // context allocates anyway, so that the solve itself never loads a module
     noalloc_resolve(c);

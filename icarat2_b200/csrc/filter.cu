@@ -210,8 +210,8 @@ __global__ void __launch_bounds__(kBallX *kBallY)
 // are staged beside the inputs
 template <int D2, int NIN>
 __global__ void __launch_bounds__(kBallX *kBallY)
-    k_ball_trans(BallGrid g, const __grid_constant__ BallWeights<D2> W, const double *__restrict__ aa,
-                 const double *__restrict__ ra, const double *__restrict__ in1,
+    k_ball_trans(BallGrid g, const __grid_constant__ BallWeights<D2> W,
+                 const double *__restrict__ aa, const double *__restrict__ ra, const double *__restrict__ in1,
                  const double *__restrict__ in2, double *__restrict__ out1,
                  double *__restrict__ out2)
 {

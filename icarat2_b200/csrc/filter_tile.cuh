@@ -101,8 +101,8 @@ __device__ __forceinline__ void ball_copy(double *dst, const double *src, int e)
 {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
   const int n = e >= 0 ? 8 : 0;
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src + (e >= 0 ? e : 0)),
-               "r"(n)
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d),
+               "l"(src + (e >= 0 ? e : 0)), "r"(n)
                : "memory");
 }
 

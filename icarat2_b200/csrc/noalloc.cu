@@ -14,6 +14,7 @@
 // this file's module and commits the array on the device, so it belongs to
 // context creation, which allocates anyway, and not to the solve.
 #include "modal.cuh"
+#include "resident_cg.cuh"
 
 namespace icarat_b200
 {
@@ -66,7 +67,7 @@ void noalloc_resolve(icarat_ctx *c)
   const void *kernels[] = {(const void *)k_cg_init,          (const void *)k_cg_spmv,
                            (const void *)k_cg_update_jacobi, (const void *)k_cg_pupdate,
                            (const void *)k_inv_diag,         (const void *)k_scatter_free,
-                           (const void *)k_gather_free};
+                           (const void *)k_gather_free,      resident_kernel()};
   for(const void *k : kernels)
   {
     cudaFuncAttributes a;
@@ -124,7 +125,10 @@ static int solve_noalloc(icarat_ctx *c, const icarat_solve_opts *opts, const dou
   k_cg_init<<<c->red_blocks, kRedThreads, 0, c->stream>>>(n, b, invd, x, r, z, p,
                                                           partials, s, o.rtol, o.maxit, 1);
   ICK(cudaGetLastError());
-  const int chunk = o.chunk > 0 ? o.chunk : 16;
+  // the ordinary solve's route: resident where the grid fits the SMs
+  const ResidentPlan res = resident_plan(g, c->sm_count);
+  IREQUIRE(resident_work(res) <= kNaPartials, ICARAT_ERR_UNSUPPORTED, "too many SMs");
+  const int chunk = o.chunk > 0 ? o.chunk : (res.blocks > 0 ? kResidentChunk : 16);
   CgScalars hs{};
   const long max_chunks = (long)(o.maxit + 1 + chunk - 1) / chunk + 1;
   for(long ch = 0; ch < max_chunks; ch++)
@@ -133,7 +137,9 @@ static int solve_noalloc(icarat_ctx *c, const icarat_solve_opts *opts, const dou
     ICK(cudaStreamSynchronize(c->stream));
     if(hs.done)
       break;
-    for(int k = 0; k < chunk; k++)
+    if(res.blocks > 0)
+      resident_cg(c->stream, res, g, c->kh, c->d_E, invd, x, r, z, Ap, p, partials, s, chunk);
+    for(int k = 0; k < chunk && res.blocks == 0; k++)
     {
       note_launch(3);
       k_cg_spmv<<<nb_spmv, ModalCfg<double>::threads, smem, c->stream>>>(
@@ -154,6 +160,8 @@ static int solve_noalloc(icarat_ctx *c, const icarat_solve_opts *opts, const dou
   ICK(cudaMemcpyAsync(&hs, s, sizeof(CgScalars), cudaMemcpyDeviceToHost, c->stream));
   ICK(cudaStreamSynchronize(c->stream));
   const int status = hs.done ? hs.status : ICARAT_WARN_MAXITER;
+  IREQUIRE(status != ICARAT_ERR_CUDA, ICARAT_ERR_CUDA,
+           "a bounded wait of the resident CG ran out");
   if(info)
   {
     info->iterations = hs.iter;

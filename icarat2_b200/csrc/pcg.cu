@@ -17,6 +17,7 @@
 #include <tuple>
 
 #include "modal.cuh"
+#include "resident_cg.cuh"
 
 namespace icarat_b200
 {
@@ -390,6 +391,20 @@ void release_graphs(icarat_ctx *c)
   c->graphs.clear();
 }
 
+// the solve's result from the scalars last copied to the host
+static int cg_report(icarat_ctx *c, icarat_solve_info *info)
+{
+  const CgScalars &s = *c->h_cg;
+  IREQUIRE(s.status != ICARAT_ERR_CUDA, ICARAT_ERR_CUDA,
+           "a bounded wait of the resident CG ran out");
+  info->iterations = s.iter;
+  info->rel_residual = s.bnorm > 0 ? s.rnorm / s.bnorm : 0.0;
+  info->status = s.done ? s.status : ICARAT_WARN_MAXITER;
+  info->refreshes = 0;
+  info->learned_iterations = 0;
+  return info->status;
+}
+
 int solve_full(icarat_ctx *c, const icarat_solve_opts *o, const double *d_b,
                double *d_x, icarat_solve_info *info)
 {
@@ -447,6 +462,27 @@ int solve_full(icarat_ctx *c, const icarat_solve_opts *o, const double *d_b,
                                                           c->d_partials, c->d_cg, 1);
     ICK(cudaMemcpyAsync(c->d_p, c->d_z, sizeof(double) * n,
                         cudaMemcpyDeviceToDevice, c->stream));
+  }
+  // Jacobi-PCG of a grid that fits the SMs runs without launches per
+  // iteration; the host looks in every kResidentChunk iterations
+  const ResidentPlan res = method == ICARAT_SOLVER_JACOBI_PCG && !use_dmma(c, g)
+                               ? resident_plan(g, c->sm_count)
+                               : ResidentPlan{};
+  if(res.blocks > 0)
+  {
+    const int n_it = o->chunk > 0 ? o->chunk : kResidentChunk;
+    const long max_launches = (long)(o->maxit + 1 + n_it - 1) / n_it + 1;
+    for(long k = 0; k < max_launches; k++)
+    {
+      resident_cg(c->stream, res, g, c->kh, c->d_E, c->d_invd, d_x, c->d_r, c->d_z, c->d_Ap,
+                  c->d_p, c->d_partials, c->d_cg, n_it);
+      ICK(cudaMemcpyAsync(c->h_cg, c->d_cg, sizeof(CgScalars), cudaMemcpyDeviceToHost,
+                          c->stream));
+      ICK(cudaStreamSynchronize(c->stream));
+      if(c->h_cg->done)
+        break;
+    }
+    return cg_report(c, info);
   }
   const auto key =
       std::make_tuple(method + 4096 * (c->fp64_tc + 1), levels + 32 * c->coarse.cur, smooth,
@@ -508,13 +544,7 @@ int solve_full(icarat_ctx *c, const icarat_solve_opts *o, const double *d_b,
   ICK(cudaMemcpyAsync(c->h_cg, c->d_cg, sizeof(CgScalars),
                       cudaMemcpyDeviceToHost, c->stream));
   ICK(cudaStreamSynchronize(c->stream));
-  const CgScalars &s = *c->h_cg;
-  info->iterations = s.iter;
-  info->rel_residual = s.bnorm > 0 ? s.rnorm / s.bnorm : 0.0;
-  info->status = s.done ? s.status : ICARAT_WARN_MAXITER;
-  info->refreshes = 0;
-  info->learned_iterations = 0;
-  return info->status;
+  return cg_report(c, info);
 }
 
 } // namespace icarat_b200
