@@ -508,6 +508,17 @@ long conv3_tc_packed_size(int cin, int cout);
 void conv3_tc_pack(const uint16_t *W, int cin, int cout, uint16_t *wpk, cudaStream_t st);
 void conv3_tc_fwd(int X, int Y, int Z, long V, const uint16_t *x, int cin, const uint16_t *wpk,
                   const float *bias, int cout, uint16_t *y, int *err, cudaStream_t st);
+// net_mma.cu: its backward convolutions (BF16 bits, FP32 gradients)
+int conv3_split_blocks(long V);
+int conv3_wgrad_splits(int X, int Y, int Z, int cin, int cout);
+void conv3_split(long V, const float *dy, const uint16_t *ymask, int C, uint16_t *g3,
+                 double *part, float *db, cudaStream_t st);
+void conv3_wgrad(int X, int Y, int Z, const uint16_t *x, int cin, const uint16_t *g3, int cout,
+                 uint16_t *xcl, float *part, int splits, cudaStream_t st);
+void conv3_dgrad_pack(const uint16_t *wt, int cin, int cout, uint16_t *wpk, cudaStream_t st);
+void conv3_dgrad(int X, int Y, int Z, const uint16_t *g3, int cout, const uint16_t *wpk, int cin,
+                 float *dx, cudaStream_t st);
+void sum_parts(int blocks, int C, const double *part, float *out, cudaStream_t st);
 // dmma_stencil.cu
 bool dmma_fits(const GridDev &g);
 void launch_ku_dmma(icarat_ctx *c, int op, DmArgs a, cudaStream_t st);

@@ -20,14 +20,9 @@
 //
 // Kernels: the forward 3x3x3 convolutions run on the tensor cores
 // (k_conv3_tc in net_tc.cu: implicit GEMM, tcgen05, FP32 accumulation in
-// TMEM); the backward pass on the CUDA cores (FP32 FMA on BF16 operands):
-//   k_conv3        one voxel x 16 output channels per thread, the weights of
-//                  a 16-input-channel chunk staged in shared memory: the
-//                  data gradient (input: ReLU-masked FP32 output gradient,
-//                  weights transposed and flipped)
-//   k_conv3_wgrad  per 256-voxel chunk and 16 output channels, every
-//                  (input channel, tap) pair summed over the chunk; chunks
-//                  reduced in a fixed order (k_chunk_reduce)
+// TMEM), the backward ones in net_mma.cu (three-part BF16 split of the FP32
+// gradient); the rest here:
+//   k_chunk_reduce  weight-gradient partials summed in a fixed order
 //   pooling, nearest upsampling into a channel slice, the 1x1 head, the
 //   relative squared error and Adam.
 #include <cuda_bf16.h>
@@ -64,152 +59,6 @@ struct Dims
 
 __device__ __forceinline__ float bfv(bf16 v) { return __bfloat162float(v); }
 
-// y[co][v] (co in [16 blockIdx.y, +16)) = sum_ci sum_tap W[co][ci][tap] x[ci][v + tap]
-// (+ bias, relu, BF16 out) or plain FP32 out.  MASK: the input is an FP32
-// gradient taken where the (BF16) tensor xmask > 0.
-template <typename TI, bool MASK, bool OUT_BF16>
-__global__ void __launch_bounds__(128)
-    k_conv3(Dims d, const TI *__restrict__ x, const bf16 *__restrict__ xmask, int cin,
-            const bf16 *__restrict__ W, const float *__restrict__ bias, int cout,
-            bf16 *__restrict__ yb, float *__restrict__ yf, int relu)
-{
-  __shared__ float Ws[16][27][16]; // [ci in chunk][tap][co in tile]
-  const int co0 = blockIdx.y * 16;
-  const long v = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  const bool valid = v < d.V;
-  const int vx = valid ? (int)(v % d.X) : 0;
-  const int vy = valid ? (int)((v / d.X) % d.Y) : 0;
-  const int vz = valid ? (int)(v / ((long)d.X * d.Y)) : 0;
-  unsigned inb = 0; // bit tap: neighbour inside the grid
-#pragma unroll
-  for(int tap = 0; tap < 27; tap++)
-  {
-    const int xx = vx + tap % 3 - 1, yy = vy + (tap / 3) % 3 - 1, zz = vz + tap / 9 - 1;
-    if(valid && xx >= 0 && xx < d.X && yy >= 0 && yy < d.Y && zz >= 0 && zz < d.Z)
-      inb |= 1u << tap;
-  }
-  float acc[16];
-#pragma unroll
-  for(int q = 0; q < 16; q++)
-    acc[q] = 0.0f;
-  for(int ci0 = 0; ci0 < cin; ci0 += 16)
-  {
-    const int nc = min(16, cin - ci0);
-    __syncthreads();
-    for(int q = threadIdx.x; q < 16 * 27 * 16; q += blockDim.x)
-    {
-      const int co = q % 16, tap = (q / 16) % 27, ci = q / (16 * 27);
-      Ws[ci][tap][co] = (ci < nc && co0 + co < cout)
-                            ? bfv(W[((long)(co0 + co) * cin + ci0 + ci) * 27 + tap])
-                            : 0.0f;
-    }
-    __syncthreads();
-    for(int ci = 0; ci < nc; ci++)
-    {
-      const TI *xc = x + (long)(ci0 + ci) * d.V;
-      const bf16 *mc = MASK ? xmask + (long)(ci0 + ci) * d.V : nullptr;
-#pragma unroll
-      for(int tap = 0; tap < 27; tap++)
-      {
-        if(!((inb >> tap) & 1u))
-          continue;
-        const long off = v + (tap % 3 - 1) + (long)((tap / 3) % 3 - 1) * d.X +
-                         (long)(tap / 9 - 1) * d.X * d.Y;
-        float xv;
-        if constexpr(MASK)
-          xv = bfv(mc[off]) > 0.0f ? (float)xc[off] : 0.0f;
-        else
-          xv = (float)xc[off];
-#pragma unroll
-        for(int q = 0; q < 16; q++)
-          acc[q] = fmaf(xv, Ws[ci][tap][q], acc[q]);
-      }
-    }
-  }
-  if(!valid)
-    return;
-#pragma unroll
-  for(int q = 0; q < 16; q++)
-  {
-    const int co = co0 + q;
-    if(co >= cout)
-      break;
-    float y = acc[q] + (bias ? bias[co] : 0.0f);
-    if(relu)
-      y = fmaxf(y, 0.0f);
-    if constexpr(OUT_BF16)
-      yb[(long)co * d.V + v] = __float2bfloat16_rn(y);
-    else
-      yf[(long)co * d.V + v] = y;
-  }
-}
-
-__device__ __forceinline__ float load_bf_or_f(const bf16 *p) { return bfv(*p); }
-__device__ __forceinline__ float load_bf_or_f(const float *p) { return *p; }
-
-// part[chunk][co][ci][tap] = sum over the chunk's voxels of dy[co][v] x[ci][v+tap],
-// dy taken where ymask > 0.
-__global__ void __launch_bounds__(128)
-    k_conv3_wgrad(Dims d, const bf16 *__restrict__ x, int cin, const float *__restrict__ dy,
-                  const bf16 *__restrict__ ymask, int cout, float *__restrict__ part)
-{
-  constexpr int CH = 256;
-  __shared__ float dys[16][CH];
-  __shared__ int vxyz[CH][3]; // coordinates of the chunk's voxels (one division each)
-  const int chunk = blockIdx.x, co0 = blockIdx.y * 16;
-  const long v0 = (long)chunk * CH;
-  for(int i = threadIdx.x; i < CH; i += blockDim.x)
-  {
-    const long v = v0 + i;
-    const int vx = (int)(v % d.X);
-    const long r = v / d.X;
-    vxyz[i][0] = vx;
-    vxyz[i][1] = (int)(r % d.Y);
-    vxyz[i][2] = (int)(r / d.Y);
-  }
-  for(int q = threadIdx.x; q < 16 * CH; q += blockDim.x)
-  {
-    const int co = q / CH, i = q % CH;
-    const long v = v0 + i;
-    float g = 0.0f;
-    if(v < d.V && co0 + co < cout)
-    {
-      const long id = (long)(co0 + co) * d.V + v;
-      g = bfv(ymask[id]) > 0.0f ? dy[id] : 0.0f;
-    }
-    dys[co][i] = g;
-  }
-  __syncthreads();
-  const int npair = cin * 27;
-  for(int p = threadIdx.x; p < npair; p += blockDim.x)
-  {
-    const int ci = p / 27, tap = p % 27;
-    const int ox = tap % 3 - 1, oy = (tap / 3) % 3 - 1, oz = tap / 9 - 1;
-    const bf16 *xc = x + (long)ci * d.V;
-    float acc[16];
-#pragma unroll
-    for(int q = 0; q < 16; q++)
-      acc[q] = 0.0f;
-    for(int i = 0; i < CH; i++)
-    {
-      const long v = v0 + i;
-      if(v >= d.V)
-        break;
-      const int xx = vxyz[i][0] + ox, yy = vxyz[i][1] + oy, zz = vxyz[i][2] + oz;
-      if(xx < 0 || xx >= d.X || yy < 0 || yy >= d.Y || zz < 0 || zz >= d.Z)
-        continue;
-      const float xv = bfv(xc[v + ox + (long)oy * d.X + (long)oz * d.X * d.Y]);
-#pragma unroll
-      for(int q = 0; q < 16; q++)
-        acc[q] = fmaf(xv, dys[q][i], acc[q]);
-    }
-#pragma unroll
-    for(int q = 0; q < 16; q++)
-      if(co0 + q < cout)
-        part[((long)chunk * cout + co0 + q) * npair + p] = acc[q];
-  }
-}
-
 // g[i] = sum_chunk part[chunk][i] (fixed order)
 __global__ void k_chunk_reduce(long n, int nchunks, const float *__restrict__ part,
                                float *__restrict__ g)
@@ -222,25 +71,6 @@ __global__ void k_chunk_reduce(long n, int nchunks, const float *__restrict__ pa
       s += part[(long)c * n + i];
     g[i] = s;
   }
-}
-
-// db[co] = sum_v dy[co][v] where ymask > 0 (ymask null: everywhere)
-__global__ void k_bias_grad(Dims d, const float *__restrict__ dy, const bf16 *__restrict__ ymask,
-                            float *__restrict__ db)
-{
-  __shared__ double sh[32];
-  const int co = blockIdx.x;
-  double s = 0.0;
-  for(long v = threadIdx.x; v < d.V; v += blockDim.x)
-  {
-    const long id = (long)co * d.V + v;
-    if(!ymask || bfv(ymask[id]) > 0.0f)
-      s += dy[id];
-  }
-  double a[1] = {s};
-  block_sum<1>(a, sh);
-  if(threadIdx.x == 0)
-    db[co] = (float)a[0];
 }
 
 // The grid transfers run one block per x-line (channel, z, y) of the grid
@@ -368,19 +198,26 @@ __global__ void k_head_back(Dims d, const float *__restrict__ dout, const bf16 *
   }
 }
 
-// dW[c][ci] = sum_v dout[c][v] x[ci][v]: one block per (c, ci)
-__global__ void k_head_wgrad(Dims d, const float *__restrict__ dout, const bf16 *__restrict__ x,
-                             float *__restrict__ dW)
+// the head's gradients, slice by slice of the voxels: part[slice][51] = dW[c][ci]
+// = sum_v dout[c][v] x[ci][v] (48 values), then db[c] = sum_v dout[c][v]
+constexpr int kHeadSlices = 32;
+__global__ void k_head_grads(Dims d, const float *__restrict__ dout, const bf16 *__restrict__ x,
+                             double *__restrict__ part)
 {
   __shared__ double sh[32];
-  const int c = blockIdx.x / 16, ci = blockIdx.x % 16;
+  const int q = blockIdx.x;
+  const int c = q < 48 ? q / 16 : q - 48;
   double s = 0.0;
-  for(long v = threadIdx.x; v < d.V; v += blockDim.x)
-    s += (double)dout[(long)c * d.V + v] * (double)bfv(x[(long)ci * d.V + v]);
+  for(long v = blockIdx.y * (long)blockDim.x + threadIdx.x; v < d.V;
+      v += (long)kHeadSlices * blockDim.x)
+  {
+    const double g = dout[(long)c * d.V + v];
+    s += q < 48 ? g * (double)bfv(x[(long)(q % 16) * d.V + v]) : g;
+  }
   double a[1] = {s};
   block_sum<1>(a, sh);
   if(threadIdx.x == 0)
-    dW[c * 16 + ci] = (float)a[0];
+    part[blockIdx.y * 51 + q] = a[0];
 }
 
 // Network input from a node vector (component-major, FP64 or FP32) scaled by
@@ -561,7 +398,8 @@ struct icarat_net
   long wpk_off[15] = {};
   int *tc_err = nullptr;
   long step = 0;
-  bool wdirty = true;
+  bool wdirty = true;     // wb, wt and wpk are older than w
+  bool wpd_dirty = true;  // wpd (training only) is older than wt
   // activations of the current padded grid
   int PX = 0, PY = 0, PZ = 0;
   Dims d[4];
@@ -572,7 +410,10 @@ struct icarat_net
   float *out = nullptr, *tgt = nullptr, *dout = nullptr;
   uint8_t *mask = nullptr;
   float *gA[4] = {}, *gB[4] = {}, *part = nullptr;
-  long part_n = 0;
+  // backward convolutions: the gradient's three parts and the layer's input,
+  // channel-last; per-block sums of the bias gradients; dgrad weights
+  bf16 *g3 = nullptr, *xcl = nullptr, *wpd = nullptr;
+  double *bpart = nullptr;
   double *lpart = nullptr, *h_lpart = nullptr;
   std::vector<void *> act;
 };
@@ -650,16 +491,23 @@ void ensure_grid(icarat_net *N, const icarat_ctx *c)
     N->gA[l] = F((long)maxc[l] * N->d[l].V);
     N->gB[l] = F((long)maxc[l] * N->d[l].V);
   }
-  // weight-gradient partials: the largest chunks x parameters of any layer
-  long pn = 0;
+  // backward work: the largest of any layer
+  long pn = 0, gn = 0, xn = 0, bn = 51 * kHeadSlices;
   const int lev[15] = {0, 0, 1, 1, 2, 2, 3, 3, 2, 2, 1, 1, 0, 0, 0};
   for(int l = 0; l < 14; l++)
   {
-    const long chunks = (N->d[lev[l]].V + 255) / 256;
-    pn = std::max(pn, chunks * (long)N->L[l].cin * N->L[l].cout * 27);
+    const Dims &d = N->d[lev[l]];
+    const long cin = N->L[l].cin, cout = N->L[l].cout;
+    const long splits = conv3_wgrad_splits(d.X, d.Y, d.Z, (int)cin, (int)cout);
+    pn = std::max(pn, splits * cin * cout * 27);
+    gn = std::max(gn, 3 * cout * d.V);
+    xn = std::max(xn, (cin + 15) / 16 * 16 * d.V);
+    bn = std::max(bn, conv3_split_blocks(d.V) * cout);
   }
   N->part = F(pn);
-  N->part_n = pn;
+  N->g3 = B(gn);
+  N->xcl = B(xn);
+  N->bpart = (double *)F(2 * bn);
   N->lpart = (double *)F(3 * 4096 * 2);
   N->PX = PX;
   N->PY = PY;
@@ -678,6 +526,7 @@ void refresh_weights(icarat_net *N, cudaStream_t st)
       conv3_tc_pack(reinterpret_cast<const uint16_t *>(N->wb + N->L[l].woff), N->L[l].cin,
                     N->L[l].cout, reinterpret_cast<uint16_t *>(N->wpk + N->wpk_off[l]), st);
   N->wdirty = false;
+  N->wpd_dirty = true;
 }
 
 // the tensor-core convolution reports a wait that ran out through a flag
@@ -744,21 +593,18 @@ void conv_back(icarat_net *N, cudaStream_t st, int li, int lvl, const bf16 *x, c
 {
   const NetLayer &Ly = N->L[li];
   const Dims &d = N->d[lvl];
-  const int chunks = (int)((d.V + 255) / 256);
-  note_launch(3);
-  k_conv3_wgrad<<<dim3(chunks, (Ly.cout + 15) / 16), 128, 0, st>>>(d, x, Ly.cin, dy, y, Ly.cout,
-                                                                     N->part);
+  uint16_t *g3 = reinterpret_cast<uint16_t *>(N->g3);
+  conv3_split(d.V, dy, reinterpret_cast<const uint16_t *>(y), Ly.cout, g3, N->bpart,
+              N->g + Ly.boff, st);
+  const int splits = conv3_wgrad_splits(d.X, d.Y, d.Z, Ly.cin, Ly.cout);
+  conv3_wgrad(d.X, d.Y, d.Z, reinterpret_cast<const uint16_t *>(x), Ly.cin, g3, Ly.cout,
+              reinterpret_cast<uint16_t *>(N->xcl), N->part, splits, st);
   const long nw = (long)Ly.cout * Ly.cin * 27;
-  k_chunk_reduce<<<nb(nw), 256, 0, st>>>(nw, chunks, N->part, N->g + Ly.woff);
-  k_bias_grad<<<Ly.cout, 256, 0, st>>>(d, dy, y, N->g + Ly.boff);
-  if(dx)
-  {
-    // dx[ci] = sum_co sum_tap W[co][ci][tap] dy_masked[co][v - tap]
-    dim3 grid((unsigned)((d.V + 127) / 128), (unsigned)((Ly.cin + 15) / 16));
-    note_launch();
-    k_conv3<float, true, false><<<grid, 128, 0, st>>>(d, dy, y, Ly.cout, N->wt + Ly.woff,
-                                                      nullptr, Ly.cin, nullptr, dx, 0);
-  }
+  note_launch();
+  k_chunk_reduce<<<nb(nw), 256, 0, st>>>(nw, splits, N->part, N->g + Ly.woff);
+  if(dx) // dx[ci] = sum_co sum_tap W[co][ci][tap] dy_masked[co][v - tap]
+    conv3_dgrad(d.X, d.Y, d.Z, g3, Ly.cout, reinterpret_cast<const uint16_t *>(N->wpd + Ly.woff),
+                Ly.cin, dx, st);
   ICK(cudaGetLastError());
 }
 
@@ -766,10 +612,17 @@ void backward(icarat_net *N, cudaStream_t st)
 {
   const Dims *d = N->d;
   const long V0 = d[0].V, V1 = d[1].V, V2 = d[2].V;
-  // head
-  note_launch(3);
-  k_head_wgrad<<<48, 256, 0, st>>>(d[0], N->dout, N->d0, N->g + N->L[14].woff);
-  k_bias_grad<<<3, 256, 0, st>>>(d[0], N->dout, nullptr, N->g + N->L[14].boff);
+  if(N->wpd_dirty)
+  {
+    for(int l = 1; l < 14; l++) // layer 0 has no data gradient
+      conv3_dgrad_pack(reinterpret_cast<const uint16_t *>(N->wt + N->L[l].woff), N->L[l].cin,
+                       N->L[l].cout, reinterpret_cast<uint16_t *>(N->wpd + N->L[l].woff), st);
+    N->wpd_dirty = false;
+  }
+  // head: weights and bias are neighbours in the flat vector
+  note_launch(2);
+  k_head_grads<<<dim3(51, kHeadSlices), 256, 0, st>>>(d[0], N->dout, N->d0, N->bpart);
+  sum_parts(kHeadSlices, 51, N->bpart, N->g + N->L[14].woff, st);
   k_head_back<<<nb(V0), 256, 0, st>>>(d[0], N->dout, N->wb + N->L[14].woff, N->gA[0]);
   // level 0 decoder: gA[0] = dD0 -> gB[0] = dE0 -> gA[0] = dC0 (48 ch)
   conv_back(N, st, 13, 0, N->e0, N->d0, N->gA[0], N->gB[0]);
@@ -889,6 +742,7 @@ int icarat_net_create(int device, unsigned long long seed, icarat_net **out)
     N->g = alloc_n<float>(o);
     N->wb = alloc_n<bf16>(o);
     N->wt = alloc_n<bf16>(o);
+    N->wpd = alloc_n<bf16>(o);
     long po = 0;
     for(int l = 0; l < 15; l++)
       if(N->L[l].k == 3)
@@ -923,7 +777,7 @@ int icarat_net_destroy(icarat_net *N)
   cudaDeviceSynchronize();
   free_acts(N);
   for(void *p : {(void *)N->w, (void *)N->m, (void *)N->v, (void *)N->g, (void *)N->wb,
-                 (void *)N->wt, (void *)N->wpk, (void *)N->tc_err})
+                 (void *)N->wt, (void *)N->wpk, (void *)N->wpd, (void *)N->tc_err})
     if(p)
       cudaFree(p);
   if(N->h_lpart)
