@@ -422,9 +422,10 @@ __global__ void k_transpose_lower(int n, const double *__restrict__ W,
 }
 
 // x[rowmap] = WT t (WT upper), one warp per row; rows are contiguous
+template <typename T>
 __global__ void k_trmv_upper(int n, const double *__restrict__ WT,
                              const double *__restrict__ t, const int *__restrict__ rowmap,
-                             double *__restrict__ x, const int *__restrict__ halt)
+                             T *__restrict__ x, const int *__restrict__ halt)
 {
   chain_wait();
   if(halted(halt))
@@ -437,7 +438,7 @@ __global__ void k_trmv_upper(int n, const double *__restrict__ WT,
     const int r = trmv_row(w, n);
     const double s = warp_row_dot(WT + (long)r * n, t, r, n, lane);
     if(lane == 0)
-      x[rowmap[r]] = s;
+      x[rowmap[r]] = (T)s;
   }
 }
 
@@ -525,14 +526,20 @@ void dense_spd_inverse_factor(cudaStream_t st, double *A, double *W, double *T, 
 
 // x[rowmap] = W^T W b[rowmap]  (WT = W^T from dense_spd_inverse_factor); both
 // products return at entry while *halt != 0 (halt null: never)
+template <typename T>
 void dense_spd_solve(cudaStream_t st, const double *W, const double *WT, int n,
-                     const double *v, double *t, const int *rowmap, double *x,
-                     const int *halt)
+                     const double *v, double *t, const int *rowmap, T *x, const int *halt)
 {
   note_launch(2);
   const int blocks = (n * 32 + 255) / 256;
   launch_chained(k_trmv_lower, blocks, 256, 0, st, n, W, v, t, halt);
-  launch_chained(k_trmv_upper, blocks, 256, 0, st, n, WT, t, rowmap, x, halt);
+  launch_chained(k_trmv_upper<T>, blocks, 256, 0, st, n, WT, t, rowmap, x, halt);
 }
+
+template void dense_spd_solve<double>(cudaStream_t, const double *, const double *, int,
+                                      const double *, double *, const int *, double *,
+                                      const int *);
+template void dense_spd_solve<float>(cudaStream_t, const double *, const double *, int,
+                                     const double *, double *, const int *, float *, const int *);
 
 } // namespace icarat_b200

@@ -166,6 +166,23 @@ struct MxScalars
   unsigned int counter;
 };
 
+// What the last smoothing step of a V-cycle needs to take the Krylov dot
+// products with it (its right-hand side is the Krylov residual).
+template <typename T> struct CycleDot;
+template <> struct CycleDot<double>
+{
+  CgScalars *s = nullptr;
+  double *partials = nullptr;
+  const double *Ap = nullptr; // not used by the CG
+};
+template <> struct CycleDot<float>
+{
+  MxScalars *s = nullptr;
+  double *partials = nullptr;
+  const float *Ap = nullptr; // null on the first iteration
+  int first = 0;
+};
+
 // the FP64 residual of the mixed-precision solvers is recomputed at least
 // every kRefreshEvery iterations: on ill-conditioned systems (floating solid
 // islands in a 1e-9 void) the FP32 recurrence residual can stall while the
@@ -559,9 +576,12 @@ void mg_level_apply(icarat_ctx *c, const icarat_solve_opts *o, int level, const 
 // solve's work, side stream included, ends with the solve)
 void mg_join(icarat_ctx *c);
 double mg_coarse_check(icarat_ctx *c, int levels, int *n_coarse);
-// z = M r by one V-cycle (z null: the result stays in the finest level's x)
-void mg_vcycle(icarat_ctx *c, const double *r, double *z, int smooth, bool first_done = false);
-void mg_vcycle_f32(icarat_ctx *c, const float *r, float *z, int smooth);
+// z = M r by one V-cycle, z in the finest level's x.  With dot set, true when
+// the last smoothing step also took z . r (and z . K p) and set the scalars.
+bool mg_vcycle(icarat_ctx *c, const double *r, int smooth, bool first_done = false,
+               const CycleDot<double> *dot = nullptr);
+bool mg_vcycle_f32(icarat_ctx *c, const float *r, int smooth,
+                   const CycleDot<float> *dot = nullptr);
 // the context's V-cycle stop flag (icarat_ctx::mg_halt) for one scope
 struct HaltScope
 {

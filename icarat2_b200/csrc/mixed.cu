@@ -472,11 +472,20 @@ static void enqueue_precondition(icarat_ctx *c, int smooth, int first)
   const int n = c->neq;
   // z stays in the finest level's x32 (read by z . r and the p update
   // before the next V-cycle overwrites it)
-  mg_vcycle_f32(c, c->f_r, nullptr, smooth);
+  CycleDot<float> dot;
+  dot.s = c->d_mx;
+  dot.partials = c->d_partials;
+  dot.Ap = first ? nullptr : c->f_Ap;
+  dot.first = first;
+  const bool done = mg_vcycle_f32(c, c->f_r, smooth, &dot);
   const float *z = c->mg[0].x32;
-  note_launch(2);
-  launch_chained(k_mx_zr, c->red_blocks, kRedThreads, 0, c->stream, n, z, c->f_r, c->f_Ap,
-                 c->d_partials, c->d_mx, first);
+  if(!done)
+  {
+    note_launch();
+    launch_chained(k_mx_zr, c->red_blocks, kRedThreads, 0, c->stream, n, z, c->f_r, c->f_Ap,
+                   c->d_partials, c->d_mx, first);
+  }
+  note_launch();
   launch_chained(k_mx_pupdate, c->red_blocks, kRedThreads, 0, c->stream, n, z, c->f_p,
                  c->d_mx, first);
 }

@@ -142,8 +142,8 @@ inline ModalPlan modal_launch(const GridDev &g, const void *kernel, int sms, int
   static std::mutex mu;
   static std::set<std::pair<int, const void *>> ready;
   smem = sizeof(ModalShared<T>);
-  if(smem > 48 * 1024)
   {
+    // (FP32: 46 KB, above the default limit with a kernel's static arrays)
     const auto key = std::make_pair(device_slot(), kernel);
     std::lock_guard<std::mutex> lock(mu);
     if(!ready.count(key))

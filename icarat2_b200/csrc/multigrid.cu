@@ -33,8 +33,9 @@ namespace icarat_b200
 {
 
 void dense_spd_inverse_factor(cudaStream_t st, double *A, double *W, double *T, int n, int bw);
+template <typename T>
 void dense_spd_solve(cudaStream_t st, const double *W, const double *WT, int n,
-                     const double *v, double *t, const int *rowmap, double *x,
+                     const double *v, double *t, const int *rowmap, T *x,
                      const int *halt = nullptr);
 
 // Galerkin coarse operators (galerkin.cu)
@@ -97,65 +98,134 @@ __global__ void k_cast(long n, const Tin *__restrict__ in, Tout *__restrict__ ou
 }
 
 // ---------------------------------------------------------------- transfers
-// coarse b = R r  (R = P^T, 27 fine nodes per coarse node, weights 1/2^d;
-// restrict_node / prolong_node in stencil.cuh)
-template <typename T>
+// Blocks are 32 x 4 node columns of one plane (no index divisions; the parity
+// of a row is uniform in its warp).  NC components per thread: all three on
+// large levels, one on levels below kSplitNodes nodes, where the sums are
+// latency and more threads shorten them (33 x 17 x 17 nodes: restriction 10.7
+// -> 6.7 us; 65 x 33 x 33 is faster with three, 9.6 against 11.1).  Every load
+// is issued unconditionally: a neighbour outside the grid is read as one inside
+// and left out of the sum.  Bound by memory on the finest level: 257 x 129 x
+// 129 nodes FP64, prolongation 62 -> 40 us (220 MB), restriction 32 -> 30.
+constexpr int kSplitNodes = 1 << 15;
+
+// coarse b = R r  (R = P^T, 27 fine nodes per coarse node, weights 1/2^d).
 // With xc set, also the coarse level's first Chebyshev step from zero
-// (k_cheb_first fused): dc = xc = inv_theta invd_c bc.
-__global__ void k_restrict(GridDev f, GridDev c, const T *__restrict__ rf,
-                           const uint8_t *__restrict__ fixc, T *__restrict__ bc,
-                           const T *__restrict__ invd_c, T inv_theta, T *__restrict__ xc,
-                           T *__restrict__ dc, const int *__restrict__ halt)
+// (k_cheb_first fused): xc = inv_theta invd_c bc.  With v set (coarsest level)
+// also the dense solve's right-hand side through its column map.
+template <typename T, int NC>
+__global__ void __launch_bounds__(128)
+    k_restrict(GridDev f, GridDev c, const T *__restrict__ rf, const uint8_t *__restrict__ fixc,
+               T *__restrict__ bc, const T *__restrict__ invd_c, T inv_theta, T *__restrict__ xc,
+               const int *__restrict__ colmap, double *__restrict__ v,
+               const int *__restrict__ halt)
 {
   chain_wait();
   if(halted(halt))
     return;
-  for(int n = blockIdx.x * blockDim.x + threadIdx.x; n < c.numnp;
-      n += gridDim.x * blockDim.x)
-  {
-    T s[3];
-    restrict_node<T, false>(f, c, rf, n, s);
-    const unsigned fx = fixc[n];
+  const int I = blockIdx.x * 32 + threadIdx.x, J = blockIdx.y * 4 + threadIdx.y;
+  const int K = NC == 3 ? blockIdx.z : blockIdx.z / 3, q0 = NC == 3 ? 0 : blockIdx.z % 3;
+  if(I >= c.NX || J >= c.NY)
+    return;
+  T s[NC];
 #pragma unroll
-    for(int q = 0; q < 3; q++)
-    {
-      const long id = (long)q * c.numnp + n;
-      const T bq = ((fx >> q) & 1u) ? T(0) : s[q];
-      bc[id] = bq;
-      if(xc)
+  for(int q = 0; q < NC; q++)
+    s[q] = T(0);
+  const int m0 = 2 * (I + J * f.NX + K * f.NX * f.NY);
+#pragma unroll
+  for(int dz = -1; dz <= 1; dz++)
+#pragma unroll
+    for(int dy = -1; dy <= 1; dy++)
+#pragma unroll
+      for(int dx = -1; dx <= 1; dx++)
       {
-        const T di = inv_theta * invd_c[id] * bq;
-        dc[id] = di;
-        xc[id] = di;
+        const int i = 2 * I + dx, j = 2 * J + dy, k = 2 * K + dz;
+        const bool in = i >= 0 && i < f.NX && j >= 0 && j < f.NY && k >= 0 && k < f.NZ;
+        const T w = T((dx ? 0.5 : 1.0) * (dy ? 0.5 : 1.0) * (dz ? 0.5 : 1.0));
+        const int m = in ? m0 + dx + dy * f.NX + dz * f.NX * f.NY : m0;
+#pragma unroll
+        for(int q = 0; q < NC; q++)
+        {
+          const T r = rf[(long)(q0 + q) * f.numnp + m];
+          s[q] += in ? w * r : T(0);
+        }
       }
+  const int n = I + J * c.NX + K * c.NX * c.NY;
+  const unsigned fx = fixc[n];
+#pragma unroll
+  for(int q = 0; q < NC; q++)
+  {
+    const int qc = q0 + q;
+    const long id = (long)qc * c.numnp + n;
+    const T bq = ((fx >> qc) & 1u) ? T(0) : s[q];
+    bc[id] = bq;
+    if(xc)
+      xc[id] = inv_theta * invd_c[id] * bq;
+    if(v)
+    {
+      const int col = colmap[3 * n + qc];
+      if(col >= 0)
+        v[col] = (double)bq;
     }
   }
 }
 
-// fine x += P xc (masked)
-template <typename T>
-__global__ void k_prolong_add(GridDev f, GridDev c, const T *__restrict__ xc,
-                              const uint8_t *__restrict__ fixf, T *__restrict__ xf,
-                              const int *__restrict__ halt)
+// fine xo = xf + P xc (masked; xo may be xf)
+template <typename T, int NC>
+__global__ void __launch_bounds__(128)
+    k_prolong_add(GridDev f, GridDev c, const T *__restrict__ xc, const uint8_t *__restrict__ fixf,
+                  const T *xf, T *xo, const int *__restrict__ halt)
 {
   chain_wait();
   if(halted(halt))
     return;
-  for(int n = blockIdx.x * blockDim.x + threadIdx.x; n < f.numnp;
-      n += gridDim.x * blockDim.x)
-  {
-    T s[3];
-    prolong_node<T, false>(f, c, xc, n, s);
-    const unsigned fx = fixf[n];
+  const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 4 + threadIdx.y;
+  const int k = NC == 3 ? blockIdx.z : blockIdx.z / 3, q0 = NC == 3 ? 0 : blockIdx.z % 3;
+  if(i >= f.NX || j >= f.NY)
+    return;
+  const int ox = i & 1, oy = j & 1, oz = k & 1;
+  const int m0 = (i >> 1) + (j >> 1) * c.NX + (k >> 1) * c.NX * c.NY;
+  const T w = (ox ? T(0.5) : T(1)) * (oy ? T(0.5) : T(1)) * (oz ? T(0.5) : T(1));
+  const int n = i + j * f.NX + k * f.NX * f.NY;
+  T x[NC], s[NC];
 #pragma unroll
-    for(int q = 0; q < 3; q++)
-      if(!((fx >> q) & 1u))
-        xf[(long)q * f.numnp + n] += s[q];
+  for(int q = 0; q < NC; q++)
+  {
+    x[q] = xf[(long)(q0 + q) * f.numnp + n];
+    s[q] = T(0);
+  }
+  const unsigned fx = fixf[n];
+#pragma unroll
+  for(int cz = 0; cz < 2; cz++)
+#pragma unroll
+    for(int cy = 0; cy < 2; cy++)
+    {
+      if((cz && !oz) || (cy && !oy)) // uniform in the warp
+        continue;
+      const int m = m0 + cy * c.NX + cz * c.NX * c.NY;
+#pragma unroll
+      for(int q = 0; q < NC; q++)
+      {
+        const T *src = xc + (long)(q0 + q) * c.numnp + m;
+        const T r0 = src[0], r1 = src[ox];
+        s[q] += w * r0;
+        s[q] += ox ? w * r1 : T(0);
+      }
+    }
+#pragma unroll
+  for(int q = 0; q < NC; q++)
+  {
+    const int qc = q0 + q;
+    xo[(long)qc * f.numnp + n] = ((fx >> qc) & 1u) ? x[q] : x[q] + s[q];
   }
 }
 
+static dim3 transfer_grid(const GridDev &g, int nc)
+{
+  return dim3((g.NX + 31) / 32, (g.NY + 3) / 4, nc == 3 ? g.NZ : 3 * g.NZ);
+}
+
 // ---------------------------------------------------------------- smoother
-// First Chebyshev step from x = 0: d = invd b / theta, x = d.
+// First Chebyshev step from x = 0: d = x = invd b / theta (d null: not kept).
 template <typename T>
 __global__ void k_cheb_first(int n, const T *__restrict__ b, const T *__restrict__ invd,
                              T inv_theta, T *__restrict__ x, T *__restrict__ d,
@@ -168,19 +238,39 @@ __global__ void k_cheb_first(int n, const T *__restrict__ b, const T *__restrict
       i += gridDim.x * blockDim.x)
   {
     const T di = inv_theta * invd[i] * b[i];
-    d[i] = di;
     x[i] = di;
+    if(d)
+      d[i] = di;
   }
+}
+
+// The Krylov scalars that z . b (b the Krylov residual) of a V-cycle's last
+// smoothing step gives: k_cg_zr and k_mx_zr of the separate pass.
+__device__ __forceinline__ void finish_dot(const CycleDot<double> &k, const double (&t)[1])
+{
+  CgScalars *s = k.s;
+  s->zr_new = t[0];
+  s->beta = t[0] / s->zr;
+  s->zr = t[0];
+}
+__device__ __forceinline__ void finish_dot(const CycleDot<float> &k, const double (&t)[2])
+{
+  MxScalars *s = k.s;
+  s->zr = t[0];
+  s->beta = k.first ? 0.0 : -t[1] / s->pAp;
 }
 
 // One Chebyshev step: r = b - K x, d = c1 d + c2 invd r, xo = x + d.
 // x and xo are distinct buffers (neighbours of x are read by other threads).
-template <typename T>
+// din null: d = x (the step after k_cheb_first) where c1 != 0; dout null: no
+// step follows that reads d.  DOT: the last step of the cycle, whose result z
+// the Krylov iteration takes with z . b (and z . K p where k.Ap is set).
+template <typename T, bool DOT>
 __global__ void __launch_bounds__(ModalCfg<T>::threads, ModalCfg<T>::blocks)
     k_cheb_step(GridDev g, ModalPlan m, KhParam<T> kh, const T *__restrict__ E,
                 const uint8_t *__restrict__ fix, const T *__restrict__ invd,
-                const T *__restrict__ b, const T *__restrict__ x, T *__restrict__ d,
-                T *__restrict__ xo, T c1, T c2, const int *__restrict__ halt)
+                const T *__restrict__ b, const T *__restrict__ x, const T *din, T *dout,
+                T *__restrict__ xo, T c1, T c2, const int *__restrict__ halt, CycleDot<T> k)
 {
   chain_wait();
   ModalShared<T> &ms = modal_shared<T>();
@@ -191,6 +281,14 @@ __global__ void __launch_bounds__(ModalCfg<T>::threads, ModalCfg<T>::blocks)
     ModalRhs<T> r;
     T invd[3], d[3];
   };
+  // z . b, and z . K p in FP32; summed per thread in shared memory (the FP64
+  // march has no registers left for them)
+  constexpr int ND = sizeof(T) == 4 ? 2 : 1;
+  __shared__ double sums[DOT ? ND : 1][DOT ? ModalCfg<T>::threads : 1];
+  if(DOT)
+#pragma unroll
+    for(int q = 0; q < ND; q++)
+      sums[DOT ? q : 0][DOT ? threadIdx.x : 0] = 0.0;
   modal_march(g, m, kh, E, x, ms,
               [&](int n) {
                 Pre pre;
@@ -200,25 +298,62 @@ __global__ void __launch_bounds__(ModalCfg<T>::threads, ModalCfg<T>::blocks)
                 {
                   const long id = (long)q * g.numnp + n;
                   pre.invd[q] = invd[id];
-                  pre.d[q] = c1 != T(0) ? d[id] : T(0);
+                  pre.d[q] = din ? din[id] : T(0);
                 }
                 return pre;
               },
               [&](int n, const T(&acc)[3], const T(&uc)[3], const Pre &pre)
               {
                 const unsigned f = pre.r.fix;
+                double dot[ND] = {};
 #pragma unroll
                 for(int q = 0; q < 3; q++)
                 {
                   const long id = (long)q * g.numnp + n;
                   T dn = 0;
                   if(!((f >> q) & 1u))
-                    dn = (c1 != T(0) ? c1 * pre.d[q] : T(0)) +
+                    dn = (c1 != T(0) ? c1 * (din ? pre.d[q] : uc[q]) : T(0)) +
                          c2 * pre.invd[q] * (pre.r.b[q] - acc[q]);
-                  d[id] = dn;
-                  xo[id] = uc[q] + dn;
+                  if(dout)
+                    dout[id] = dn;
+                  const T z = uc[q] + dn;
+                  xo[id] = z;
+                  if(DOT)
+                  {
+                    dot[0] += (double)z * (double)pre.r.b[q];
+                    if constexpr(ND == 2)
+                      if(k.Ap)
+                        dot[1] += (double)z * (double)k.Ap[id];
+                  }
                 }
+                if(DOT)
+#pragma unroll
+                  for(int q = 0; q < ND; q++)
+                    sums[DOT ? q : 0][DOT ? threadIdx.x : 0] += dot[q];
               });
+  if(DOT)
+  {
+    __shared__ double sh[32 * ND];
+    double dot[ND];
+#pragma unroll
+    for(int q = 0; q < ND; q++)
+      dot[q] = sums[DOT ? q : 0][DOT ? threadIdx.x : 0];
+    block_sum<ND>(dot, sh);
+    if(threadIdx.x == 0)
+#pragma unroll
+      for(int q = 0; q < ND; q++)
+        k.partials[q * gridDim.x + blockIdx.x] = dot[q];
+    if(last_block(&k.s->counter))
+    {
+      double t[ND];
+      sum_partials<ND>(k.partials, gridDim.x, t, sh);
+      if(threadIdx.x == 0)
+      {
+        finish_dot(k, t);
+        k.s->counter = 0;
+      }
+    }
+  }
 }
 
 // r = b - K x (constrained rows 0)
@@ -283,20 +418,6 @@ __global__ void k_coarse_assemble(GridDev g, KeParam ke, const double *__restric
               }
         }
   }
-}
-
-// free coarse components of b (any precision) into the dense solve's vector
-template <typename T>
-__global__ void k_coarse_gather(int nfree, const int *__restrict__ rowmap,
-                                const T *__restrict__ b, double *__restrict__ v,
-                                const int *__restrict__ halt)
-{
-  chain_wait();
-  if(halted(halt))
-    return;
-  for(int r = blockIdx.x * blockDim.x + threadIdx.x; r < nfree;
-      r += gridDim.x * blockDim.x)
-    v[r] = (double)b[rowmap[r]];
 }
 
 // ---------------------------------------------------------------- driver
@@ -562,6 +683,12 @@ static void allocate_levels(icarat_ctx *c, int levels)
   c->coarse.work[0] = dalloc((size_t)nf * nf);
   c->coarse.vin = dalloc(nf);
   c->coarse.vout = dalloc(nf);
+  // the dense solve writes the free components; the constrained ones stay 0
+  {
+    const MgLevel &C = c->mg[levels - 1];
+    ICK(cudaMemset(C.x, 0, sizeof(double) * 3 * C.g.numnp));
+    ICK(cudaMemset(C.x32, 0, sizeof(float) * 3 * C.g.numnp));
+  }
   c->mg_built_levels = levels;
 }
 
@@ -713,11 +840,14 @@ void mg_level_apply(icarat_ctx *c, const icarat_solve_opts *o, int level, const 
   MgLevel &L = c->mg[level];
   const size_t nv = 3 * (size_t)L.g.numnp;
   ICK(cudaMemcpyAsync(L.x, x, sizeof(double) * nv, cudaMemcpyHostToDevice, c->stream));
+  // the coarsest level's constrained components are 0 between solves
+  auto clear = [&] { ICK(cudaMemsetAsync(L.x, 0, sizeof(double) * nv, c->stream)); };
   if(level > 0 && c->mg_galerkin)
   {
     ICK(cudaMemsetAsync(L.b, 0, sizeof(double) * nv, c->stream));
     st_residual_launch<double>(c->stream, L.g, L.S, L.fix, L.b, L.x, L.t, nullptr);
     ICK(cudaMemcpyAsync(y, L.t, sizeof(double) * nv, cudaMemcpyDeviceToHost, c->stream));
+    clear();
     ICK(cudaStreamSynchronize(c->stream));
     for(size_t i = 0; i < nv; i++)
       y[i] = -y[i];
@@ -725,6 +855,7 @@ void mg_level_apply(icarat_ctx *c, const icarat_solve_opts *o, int level, const 
   }
   launch_apply_K(c, L.g, L.E, L.fix, L.x, L.t, nullptr);
   ICK(cudaMemcpyAsync(y, L.t, sizeof(double) * nv, cudaMemcpyDeviceToHost, c->stream));
+  clear();
   ICK(cudaStreamSynchronize(c->stream));
 }
 
@@ -859,14 +990,19 @@ template <typename T> static bool tc_level(icarat_ctx *c, int lvl)
          (c->mx_fine_op == ICARAT_OP_TC_BF16X3 || c->mx_fine_op == ICARAT_OP_TC_BF16);
 }
 
-// one Chebyshev step d = c1 d + c2 invd (b - K x), xo = x + d on level lvl
+// one Chebyshev step d = c1 d + c2 invd (b - K x), xo = x + d on level lvl;
+// d_is_x: the d of the step before is x; last: no step follows that reads d.
+// With dot set the step also takes the cycle's dot products where its kernel
+// does (dot cleared then).
 template <typename T>
 static void cheb_step(icarat_ctx *c, MgLevel &L, int lvl, const T *b, const T *x, T *d, T *xo,
-                      double c1, double c2)
+                      double c1, double c2, bool d_is_x, bool last, const CycleDot<T> **dot)
 {
   using B = LevelBuf<T>;
   if(tc_level<T>(c, lvl))
   {
+    if(d_is_x) // this operator reads d
+      ICK(cudaMemcpyAsync(d, x, sizeof(T) * 3 * L.g.numnp, cudaMemcpyDeviceToDevice, c->stream));
     TcArgs a;
     a.g = L.g;
     a.E = reinterpret_cast<const float *>(B::E(L));
@@ -885,6 +1021,9 @@ static void cheb_step(icarat_ctx *c, MgLevel &L, int lvl, const T *b, const T *x
   if constexpr(std::is_same<T, double>::value)
     if(use_dmma(c, L.g))
     {
+      if(d_is_x)
+        ICK(cudaMemcpyAsync(d, x, sizeof(T) * 3 * L.g.numnp, cudaMemcpyDeviceToDevice,
+                            c->stream));
       DmArgs a;
       a.g = L.g;
       a.E = B::E(L);
@@ -902,11 +1041,24 @@ static void cheb_step(icarat_ctx *c, MgLevel &L, int lvl, const T *b, const T *x
     }
   int blocks;
   size_t smem;
-  const ModalPlan m =
-      modal_launch<T>(L.g, (const void *)k_cheb_step<T>, c->sm_count, 1 << 30, blocks, smem);
+  const T *din = c1 != 0.0 && !d_is_x ? d : nullptr;
+  T *dout = last ? nullptr : d;
   note_launch();
-  launch_chained(k_cheb_step<T>, blocks, ModalCfg<T>::threads, smem, c->stream, L.g, m, B::kh(c),
-                 B::E(L), L.fix, B::invd(L), b, x, d, xo, T(c1), T(c2), c->mg_halt);
+  if(dot && *dot)
+  {
+    const ModalPlan m = modal_launch<T>(L.g, (const void *)k_cheb_step<T, true>, c->sm_count,
+                                        kMaxRedBlocks, blocks, smem);
+    launch_chained(k_cheb_step<T, true>, blocks, ModalCfg<T>::threads, smem, c->stream, L.g, m,
+                   B::kh(c), B::E(L), L.fix, B::invd(L), b, x, din, dout, xo, T(c1), T(c2),
+                   c->mg_halt, **dot);
+    *dot = nullptr;
+    return;
+  }
+  const ModalPlan m = modal_launch<T>(L.g, (const void *)k_cheb_step<T, false>, c->sm_count,
+                                      1 << 30, blocks, smem);
+  launch_chained(k_cheb_step<T, false>, blocks, ModalCfg<T>::threads, smem, c->stream, L.g, m,
+                 B::kh(c), B::E(L), L.fix, B::invd(L), b, x, din, dout, xo, T(c1), T(c2),
+                 c->mg_halt, CycleDot<T>{});
 }
 
 // r = b - K x on level lvl
@@ -955,13 +1107,16 @@ static void mg_residual(icarat_ctx *c, MgLevel &L, int lvl, const T *b, const T 
                  B::E(L), L.fix, b, x, r, c->mg_halt);
 }
 
-// Chebyshev smoothing of K x = b on level lvl, deg steps.  from_zero: x = 0
-// on entry (the first step needs no product).
+// Chebyshev smoothing of K x = b on level lvl, deg steps, from x (one of the
+// level's buffers x and t) to the buffer returned.  from_zero: x = 0 on entry
+// (the first step needs no product).
 template <typename T>
-static void smooth(icarat_ctx *c, MgLevel &L, int lvl, const T *b, int deg, bool from_zero,
-                   bool first_done = false)
+static T *smooth(icarat_ctx *c, MgLevel &L, int lvl, const T *b, int deg, T *x, bool from_zero,
+                 bool first_done, const CycleDot<T> **dot)
 {
   using B = LevelBuf<T>;
+  T *xo = x == B::x(L) ? B::t(L) : B::x(L), *d = B::r(L);
+  const int nv = 3 * L.g.numnp;
   if(lvl > 0 && c->mg_galerkin)
   {
     // the same Chebyshev sequence with the level's own bound: coefficients
@@ -969,123 +1124,111 @@ static void smooth(icarat_ctx *c, MgLevel &L, int lvl, const T *b, int deg, bool
     IREQUIRE(deg <= (kGalCoef + 1) / 2, ICARAT_ERR_ARG,
              "mg_smooth too large for the Galerkin coarse levels");
     const double *coef = c->gal_coef + (size_t)lvl * kGalCoef;
-    const int nv = 3 * L.g.numnp;
-    T *x = B::x(L), *xo = B::t(L), *d = B::r(L);
     if(from_zero)
       st_first_launch<T>(c->stream, nv, b, B::invd(L), coef, x, d, c->mg_halt);
-    else
-    {
-      st_cheb_launch<T>(c->stream, L.g, B::S(L), L.fix, B::invd(L), b, x, d, xo, coef, 0,
-                        c->mg_halt);
-      std::swap(x, xo);
-    }
-    for(int k = 1; k < deg; k++)
+    for(int k = from_zero ? 1 : 0; k < deg; k++)
     {
       st_cheb_launch<T>(c->stream, L.g, B::S(L), L.fix, B::invd(L), b, x, d, xo, coef, k,
                         c->mg_halt);
       std::swap(x, xo);
     }
-    if(x != B::x(L))
-      ICK(cudaMemcpyAsync(B::x(L), x, sizeof(T) * nv, cudaMemcpyDeviceToDevice, c->stream));
-    return;
+    return x;
   }
   const double lmax = c->lam_max_dk;
   const double lmin = 0.1 * lmax;
   const double theta = 0.5 * (lmax + lmin), delta = 0.5 * (lmax - lmin);
   const double sigma = theta / delta;
   double rho_old = 1.0 / sigma;
-  const int nv = 3 * L.g.numnp;
-  T *x = B::x(L), *xo = B::t(L), *d = B::r(L);
-  int k0 = 0;
+  // the tensor-core operators read d from memory, the march takes x for it
+  bool d_is_x = from_zero;
   if(from_zero)
   {
-    if(!first_done) // else the restriction that produced b took this step
+    if(!first_done) // else the kernel that produced b took this step
     {
+      bool keep = tc_level<T>(c, lvl);
+      if constexpr(std::is_same<T, double>::value)
+        keep = keep || use_dmma(c, L.g);
+      d_is_x = !keep;
       note_launch();
       launch_chained(k_cheb_first<T>, blocks_for(nv, 256), 256, 0, c->stream, nv, b,
-                     B::invd(L), T(1.0 / theta), x, d, c->mg_halt);
+                     B::invd(L), T(1.0 / theta), x, keep ? d : (T *)nullptr, c->mg_halt);
     }
-    k0 = 1;
   }
   else
   {
     // first step from the current x: d = invd (b - K x) / theta
-    cheb_step<T>(c, L, lvl, b, x, d, xo, 0.0, 1.0 / theta);
+    cheb_step<T>(c, L, lvl, b, x, d, xo, 0.0, 1.0 / theta, false, deg == 1,
+                 deg == 1 ? dot : nullptr);
     std::swap(x, xo);
-    k0 = 1;
   }
-  for(int k = k0; k < deg; k++)
+  for(int k = 1; k < deg; k++)
   {
     const double rho = 1.0 / (2.0 * sigma - rho_old);
-    cheb_step<T>(c, L, lvl, b, x, d, xo, rho * rho_old, 2.0 * rho / delta);
+    cheb_step<T>(c, L, lvl, b, x, d, xo, rho * rho_old, 2.0 * rho / delta, d_is_x && k == 1,
+                 k == deg - 1, k == deg - 1 ? dot : nullptr);
     std::swap(x, xo);
     rho_old = rho;
   }
-  if(x != B::x(L))
-    ICK(cudaMemcpyAsync(B::x(L), x, sizeof(T) * nv, cudaMemcpyDeviceToDevice, c->stream));
+  return x;
 }
 
+// One V-cycle from level l on; the result is in the level's x.  dot: the dot
+// products of the finest level's last step (cleared where they were taken).
 template <typename T>
-static void vcycle(icarat_ctx *c, int l, const T *b, int deg, bool first_done = false)
+static void vcycle(icarat_ctx *c, int l, const T *b, int deg, bool first_done,
+                   const CycleDot<T> **dot)
 {
   using B = LevelBuf<T>;
   MgLevel &L = c->mg[l];
   const int levels = (int)c->mg.size();
   if(l == levels - 1)
   {
+    // the restriction has left the right-hand side in vin
     const int n = c->coarse.n;
-    ICK(cudaMemsetAsync(L.x, 0, sizeof(double) * 3 * L.g.numnp, c->stream));
     if(n > 0)
-    {
-      note_launch();
-      launch_chained(k_coarse_gather<T>, blocks_for(n, 256), 256, 0, c->stream, n,
-                     c->coarse.map, b, c->coarse.vin, c->mg_halt);
-      dense_spd_solve(c->stream, c->coarse.W[c->coarse.cur], c->coarse.work[c->coarse.cur],
-                      n, c->coarse.vin, c->coarse.vout, c->coarse.map, L.x, c->mg_halt);
-    }
-    if(!std::is_same<T, double>::value)
-    {
-      note_launch();
-      launch_chained(k_cast<double, T>, blocks_for(3L * L.g.numnp, 256), 256, 0, c->stream,
-                     3L * L.g.numnp, L.x, B::x(L));
-    }
+      dense_spd_solve<T>(c->stream, c->coarse.W[c->coarse.cur], c->coarse.work[c->coarse.cur], n,
+                         c->coarse.vin, c->coarse.vout, c->coarse.map, B::x(L), c->mg_halt);
     return;
   }
   MgLevel &C = c->mg[l + 1];
-  smooth<T>(c, L, l, b, deg, true, first_done);
+  T *x = smooth<T>(c, L, l, b, deg, B::x(L), true, first_done, nullptr);
   // residual into r (smooth() used r as scratch; done with it now)
-  mg_residual<T>(c, L, l, b, B::x(L), B::r(L));
+  mg_residual<T>(c, L, l, b, x, B::r(L));
   // the coarse level's first smoothing step rides on the restriction when
   // that level is smoothed with the shared rediscretised bound
-  const bool fuse = l + 1 < levels - 1 && !c->mg_galerkin;
+  const bool coarsest = l + 1 == levels - 1;
+  const bool fuse = !coarsest && !c->mg_galerkin;
   const double lm = c->lam_max_dk, theta = 0.5 * (lm + 0.1 * lm);
   note_launch();
-  launch_chained(k_restrict<T>, blocks_for(C.g.numnp, 128), 128, 0, c->stream, L.g, C.g,
+  const bool split_c = C.g.numnp < kSplitNodes, split_f = L.g.numnp < kSplitNodes;
+  launch_chained(split_c ? k_restrict<T, 1> : k_restrict<T, 3>,
+                 transfer_grid(C.g, split_c ? 1 : 3), dim3(32, 4), 0, c->stream, L.g, C.g,
                  B::r(L), C.fix, B::b(C), B::invd(C), T(1.0 / theta),
-                 fuse ? B::x(C) : (T *)nullptr, B::r(C), c->mg_halt);
-  vcycle<T>(c, l + 1, B::b(C), deg, fuse);
+                 fuse ? B::x(C) : (T *)nullptr, c->coarse.map + c->coarse.n,
+                 coarsest ? c->coarse.vin : (double *)nullptr, c->mg_halt);
+  vcycle<T>(c, l + 1, B::b(C), deg, fuse, nullptr);
+  // into the buffer from which deg steps end in the level's x
+  T *to = deg % 2 == 0 ? B::x(L) : B::t(L);
   note_launch();
-  launch_chained(k_prolong_add<T>, blocks_for(L.g.numnp, 128), 128, 0, c->stream, L.g, C.g,
-                 B::x(C), L.fix, B::x(L), c->mg_halt);
-  smooth<T>(c, L, l, b, deg, false);
+  launch_chained(split_f ? k_prolong_add<T, 1> : k_prolong_add<T, 3>,
+                 transfer_grid(L.g, split_f ? 1 : 3), dim3(32, 4), 0, c->stream, L.g, C.g,
+                 B::x(C), L.fix, (const T *)x, to, c->mg_halt);
+  smooth<T>(c, L, l, b, deg, to, false, false, l == 0 ? dot : nullptr);
 }
 
-void mg_vcycle(icarat_ctx *c, const double *r, double *z, int deg, bool first_done)
+bool mg_vcycle(icarat_ctx *c, const double *r, int deg, bool first_done,
+               const CycleDot<double> *dot)
 {
-  vcycle<double>(c, 0, r, deg, first_done);
-  if(z)
-    ICK(cudaMemcpyAsync(z, c->mg[0].x, sizeof(double) * c->neq, cudaMemcpyDeviceToDevice,
-                        c->stream));
+  vcycle<double>(c, 0, r, deg, first_done, &dot);
   ICK(cudaGetLastError());
+  return dot == nullptr;
 }
 
-void mg_vcycle_f32(icarat_ctx *c, const float *r, float *z, int deg)
+bool mg_vcycle_f32(icarat_ctx *c, const float *r, int deg, const CycleDot<float> *dot)
 {
-  vcycle<float>(c, 0, r, deg);
-  if(z)
-    ICK(cudaMemcpyAsync(z, c->mg[0].x32, sizeof(float) * c->neq, cudaMemcpyDeviceToDevice,
-                        c->stream));
+  vcycle<float>(c, 0, r, deg, false, &dot);
   ICK(cudaGetLastError());
+  return dot == nullptr;
 }
 
 } // namespace icarat_b200

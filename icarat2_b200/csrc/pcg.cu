@@ -233,14 +233,14 @@ __global__ void k_cg_update_jacobi(int n, const double *__restrict__ invd,
 
 // MG: x += alpha p, r -= alpha Ap; ||r||, stop test (z comes from a V-cycle).
 // With x0 set, also the V-cycle's first Chebyshev step on the finest level
-// from zero (k_cheb_first fused): d0 = x0 = inv_theta invd0 r.
+// from zero (k_cheb_first fused): x0 = inv_theta invd0 r.
 __global__ void k_cg_update_r(int n, double *__restrict__ x,
                               double *__restrict__ r,
                               const double *__restrict__ p,
                               const double *__restrict__ Ap,
                               double *__restrict__ partials, CgScalars *s,
                               const double *__restrict__ invd0, double inv_theta,
-                              double *__restrict__ x0, double *__restrict__ d0)
+                              double *__restrict__ x0)
 {
   chain_wait();
   __shared__ double sh[32];
@@ -256,11 +256,7 @@ __global__ void k_cg_update_r(int n, double *__restrict__ x,
     r[i] = ri;
     rr += ri * ri;
     if(x0)
-    {
-      const double di = inv_theta * invd0[i] * ri;
-      d0[i] = di;
-      x0[i] = di;
-    }
+      x0[i] = inv_theta * invd0[i] * ri;
   }
   double v[1] = {rr};
   block_sum<1>(v, sh);
@@ -370,14 +366,20 @@ static void enqueue_iteration(icarat_ctx *c, int method, int smooth,
     MgLevel &L0 = c->mg[0];
     const double lm = c->lam_max_dk, theta = 0.5 * (lm + 0.1 * lm);
     launch_chained(k_cg_update_r, c->red_blocks, kRedThreads, 0, c->stream, n, x, c->d_r,
-                   c->d_p, c->d_Ap, c->d_partials, c->d_cg, L0.invd, 1.0 / theta, L0.x, L0.r);
+                   c->d_p, c->d_Ap, c->d_partials, c->d_cg, L0.invd, 1.0 / theta, L0.x);
     // z stays in the finest level's x (overwritten only by the next
     // iteration's update, after z . r and the p update have read it)
-    mg_vcycle(c, c->d_r, nullptr, smooth, true);
+    CycleDot<double> dot;
+    dot.s = c->d_cg;
+    dot.partials = c->d_partials;
+    const bool done = mg_vcycle(c, c->d_r, smooth, true, &dot);
     z = c->mg[0].x;
-    note_launch();
-    launch_chained(k_cg_zr, c->red_blocks, kRedThreads, 0, c->stream, n, z, c->d_r,
-                   c->d_partials, c->d_cg, 0);
+    if(!done)
+    {
+      note_launch();
+      launch_chained(k_cg_zr, c->red_blocks, kRedThreads, 0, c->stream, n, z, c->d_r,
+                     c->d_partials, c->d_cg, 0);
+    }
   }
   note_launch();
   launch_chained(k_cg_pupdate, c->red_blocks, kRedThreads, 0, c->stream, n, z, c->d_p,
@@ -456,12 +458,12 @@ int solve_full(icarat_ctx *c, const icarat_solve_opts *o, const double *d_b,
   if(method == ICARAT_SOLVER_MG_PCG)
   {
     // z0 = M r0, zr, p = z
-    mg_vcycle(c, c->d_r, c->d_z, smooth);
+    mg_vcycle(c, c->d_r, smooth);
+    const double *z0 = c->mg[0].x;
     note_launch();
-    k_cg_zr<<<c->red_blocks, kRedThreads, 0, c->stream>>>(n, c->d_z, c->d_r,
-                                                          c->d_partials, c->d_cg, 1);
-    ICK(cudaMemcpyAsync(c->d_p, c->d_z, sizeof(double) * n,
-                        cudaMemcpyDeviceToDevice, c->stream));
+    k_cg_zr<<<c->red_blocks, kRedThreads, 0, c->stream>>>(n, z0, c->d_r, c->d_partials, c->d_cg,
+                                                          1);
+    ICK(cudaMemcpyAsync(c->d_p, z0, sizeof(double) * n, cudaMemcpyDeviceToDevice, c->stream));
   }
   // Jacobi-PCG of a grid that fits the SMs runs without launches per
   // iteration; the host looks in every kResidentChunk iterations

@@ -103,7 +103,8 @@ typedef struct
   int mg_levels; /* multigrid levels incl. the finest (MG_PCG, MIXED_IR) */
   int mg_smooth; /* smoothing sweeps per level and direction (MG_PCG, MIXED_IR) */
   int chunk;     /* iterations per host convergence check (0 = default: 4 for
-                    MG_PCG and MIXED_IR, 16 for JACOBI_PCG); the iterations of
+                    MG_PCG and MIXED_IR, 16 for JACOBI_PCG, 512 where the
+                    grid fits the GPU's shared memory); the iterations of
                     a chunk past convergence return at entry and change nothing */
   double refresh; /* MIXED_IR: recompute the residual in FP64 once the FP32
                      recurrence has fallen by this factor (0 = 1e-2) */
