@@ -459,10 +459,13 @@ void apply_K_lowp(icarat_ctx *c, int op, const float *u, float *y)
 // Operators of the FP32 iterations unless the options name others.  The
 // smoother tolerates even the ~1e-3 relative error of the single-product
 // BF16 tensor-core operator (the preconditioner is applied inexactly anyway:
-// 15 iterations to 1e-6 at 256 x 128 x 128 with BF16, BF16 hi/lo and FP32
-// alike, BF16 the fastest); the Krylov product K p does not (an inexact K p
-// costs many more iterations), so it stays on the FP32 CUDA-core stencil.
-constexpr int kDefaultFineOp = ICARAT_OP_TC_BF16;
+// 13 iterations to 1e-6 at 256 x 128 x 128 with BF16, BF16 hi/lo and FP32
+// alike), but the FP32 parity-block march is the fastest of them at every
+// grid measured: a solve to 1e-10 takes 25.4 ms with it, 28.2 with BF16 and
+// 30.5 with BF16 hi/lo at 256 x 128 x 128, 6.7 / 7.4 / 8.1 at 128 x 64 x 64 and
+// 3.5 / 4.5 / 4.4 at 64 x 32 x 32.  The Krylov product K p needs FP32 (an
+// inexact K p costs many more iterations).
+constexpr int kDefaultFineOp = ICARAT_OP_FP32;
 constexpr int kDefaultKrylovOp = ICARAT_OP_FP32;
 
 // z = M r32, zr, beta, p update
