@@ -397,8 +397,14 @@ static int find_ball(const FilterState &F, std::vector<double> &cube)
 void filter_setup(icarat_ctx *c, double R)
 {
   IREQUIRE(R >= 0.0 && std::isfinite(R), ICARAT_ERR_ARG, "filter radius must be >= 0");
-  filter_free(c);
   FilterState &F = c->filt;
+  if(F.ready && F.radius == R)
+  {
+    // the same stencil on the same mesh (a loop started again): it stands
+    F.have_forward = false;
+    return;
+  }
+  filter_free(c);
   F.radius = R;
   F.rx = (int)std::ceil(R / c->hx);
   F.ry = (int)std::ceil(R / c->hy);
@@ -434,6 +440,7 @@ void filter_setup(icarat_ctx *c, double R)
   k_filter_recip<<<eblocks(c), 256, 0, c->stream>>>(c->nelx, F.d_aa, F.d_ra);
   ICK(cudaGetLastError());
   F.have_forward = false;
+  F.ready = true;
 }
 
 template <int D2> static BallWeights<D2> ball_weights(const FilterState &F)

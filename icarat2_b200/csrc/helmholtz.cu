@@ -553,8 +553,10 @@ void helm_free(icarat_ctx *c)
 void helm_setup(icarat_ctx *c, double R)
 {
   IREQUIRE(R >= 0.0 && std::isfinite(R), ICARAT_ERR_ARG, "filter radius must be >= 0");
-  helm_free(c);
   HelmState &H = c->helm;
+  if(H.ready && H.radius == R)
+    return; // the same operator on the same mesh: every buffer is a call's own
+  helm_free(c);
   H.radius = R;
   helm_element(c->hx, c->hy, c->hz, R, H.ke, H.nj, H.ns);
   double coef[kHelmClasses * 27];
@@ -579,6 +581,7 @@ void helm_setup(icarat_ctx *c, double R)
   k_helm_invd<<<blocks_for(n, kHelmThreads, 4 * c->sm_count), kHelmThreads, 0, c->stream>>>(
       hgrid(c), H.d_coef, H.d_invd);
   ICK(cudaGetLastError());
+  H.ready = true;
 }
 
 // grid of the streaming CG kernels: 8 blocks of 256 threads per SM (full

@@ -310,6 +310,7 @@ struct FilterState
   double *d_aa = nullptr;       // nelx sums of weights (dfilters_ds)
   double *d_ra = nullptr;       // nelx correctly rounded reciprocals 1 / aa
   bool have_forward = false;
+  bool ready = false; // set up for `radius`
 };
 
 // Helmholtz PDE filter: element matrix, the 27 x 27 node-class stencil
@@ -325,6 +326,7 @@ struct HelmState
   cudaGraphExec_t exec = nullptr; // kHelmChunk iterations
   double *d_oc = nullptr;         // 3 nelx: work of the OC volume functor
   double invd_cls[27] = {};       // Jacobi inverse diagonal per node class
+  bool ready = false;             // set up for `radius`
 };
 
 struct MmaDev;

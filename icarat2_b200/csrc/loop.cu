@@ -16,8 +16,8 @@ namespace icarat_b200
 
 int mma_update_device(icarat_mma *h, double *x, const double *dfdx, const double *gx,
                       const double *dgdx, const double *xmin, const double *xmax);
-void mma_create(int device, int n, int m, double a, double c, double d,
-                icarat_mma **out, cudaStream_t stream);
+void mma_renew(int device, int n, int m, double a, double c, double d, icarat_mma **h,
+               cudaStream_t stream);
 void mma_set_move(icarat_mma *h, double move);
 int mma_last_newton(const icarat_mma *h);
 void mma_state_io(icarat_mma *h, bool save, int *iter, double *low, double *upp,
@@ -98,11 +98,6 @@ int loop_init(icarat_ctx *c, const icarat_loop_opts *o, const double *x0)
                       &L.xmin, &L.xmax})
       *p = dalloc(n);
   }
-  if(L.mma)
-  {
-    icarat_mma_destroy(L.mma);
-    L.mma = nullptr;
-  }
   L.opts = *o;
   L.optstep = 0;
   L.V0 = 0.0;
@@ -126,8 +121,13 @@ int loop_init(icarat_ctx *c, const icarat_loop_opts *o, const double *x0)
     // MMASolver mma(nelx, 1) with SetMoveLimit (opt_mma_Helmholtz.cpp uses 0.2)
     // (on the kept elements of a selection: the reference's MMA has nelx of
     // the modified mesh variables)
-    mma_create(c->device, abi_nelx(c), 1, 0.0, 100000.0, 0.0, &L.mma, c->stream);
+    mma_renew(c->device, abi_nelx(c), 1, 0.0, 100000.0, 0.0, &L.mma, c->stream);
     mma_set_move(L.mma, o->move);
+  }
+  else
+  {
+    icarat_mma_destroy(L.mma);
+    L.mma = nullptr;
   }
   ICK(cudaStreamSynchronize(c->stream));
   L.init = true;

@@ -505,6 +505,48 @@ int mma_update_device(icarat_mma *h, double *x, const double *dfdx, const double
 }
 
 void mma_destroy(icarat_mma *h);
+void mma_create(int device, int n, int m, double a, double c, double d, icarat_mma **out,
+                cudaStream_t stream);
+
+// The state a new solver starts from.
+static void mma_reset(icarat_mma *h, double a, double c, double d)
+{
+  const int n = h->n, m = h->m;
+  h->iter = 0;
+  h->last_outer = h->last_newton = 0;
+  // MMASolver::MMASolver defaults (MMASolver.cpp:41-55)
+  h->xmamieps = 1.0e-5;
+  h->epsimin = std::sqrt((double)(n + m)) * 1e-9;
+  h->raa0 = 0.00001;
+  h->move = 0.15;
+  h->albefa = 0.2;
+  h->asyminit = 0.2;
+  h->asymdec = 0.7;
+  h->asyminc = 1.2;
+  for(int j = 0; j < kMmaMaxM; j++)
+  {
+    h->a[j] = a;
+    h->c[j] = c;
+    h->d[j] = d;
+  }
+  for(double *p : {h->low, h->upp, h->alpha, h->beta, h->p0, h->q0, h->xold1, h->xold2})
+    ICK(cudaMemsetAsync(p, 0, sizeof(double) * n, h->stream));
+}
+
+// *h as mma_create would make it, its buffers kept when it has n variables
+// and m constraints on the same stream
+void mma_renew(int device, int n, int m, double a, double c, double d, icarat_mma **h,
+               cudaStream_t stream)
+{
+  if(*h && (*h)->n == n && (*h)->m == m && (*h)->stream == stream && (*h)->device == device)
+  {
+    mma_reset(*h, a, c, d);
+    return;
+  }
+  mma_destroy(*h);
+  *h = nullptr;
+  mma_create(device, n, m, a, c, d, h, stream);
+}
 
 // stream: run on this stream (owned by the caller) or, when null, on a new one
 void mma_create(int device, int n, int m, double a, double c, double d,
@@ -526,28 +568,10 @@ void mma_create(int device, int n, int m, double a, double c, double d,
       ICK(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
     h->n = n;
     h->m = m;
-    h->iter = 0;
-    // MMASolver::MMASolver defaults (MMASolver.cpp:41-55)
-    h->xmamieps = 1.0e-5;
-    h->epsimin = std::sqrt((double)(n + m)) * 1e-9;
-    h->raa0 = 0.00001;
-    h->move = 0.15;
-    h->albefa = 0.2;
-    h->asyminit = 0.2;
-    h->asymdec = 0.7;
-    h->asyminc = 1.2;
-    for(int j = 0; j < kMmaMaxM; j++)
-    {
-      h->a[j] = a;
-      h->c[j] = c;
-      h->d[j] = d;
-    }
     for(double **p : {&h->low, &h->upp, &h->alpha, &h->beta, &h->p0, &h->q0,
                       &h->xold1, &h->xold2})
-    {
       *p = dalloc(n);
-      ICK(cudaMemset(*p, 0, sizeof(double) * n));
-    }
+    mma_reset(h, a, c, d);
     h->pij = dalloc((size_t)n * m);
     h->qij = dalloc((size_t)n * m);
     h->stage = dalloc((size_t)n * (4 + m) + kMmaMaxM);
