@@ -333,6 +333,19 @@ static int apply_K_impl(icarat_ctx *c, const double *u, double *y, bool host)
 {
   IREQUIRE(c->design_set, ICARAT_ERR_STATE, "set the design first");
   IREQUIRE(u && y, ICARAT_ERR_ARG, "null argument");
+  if(host)
+  {
+    ICK(cudaMemcpyAsync(c->d_v2, u, sizeof(double) * c->numeq, cudaMemcpyHostToDevice, c->stream));
+    if(apply_K_equations(c, c->d_v2, c->d_Ap))
+    {
+      ICK(cudaMemcpyAsync(y, c->d_Ap, sizeof(double) * c->numeq, cudaMemcpyDeviceToHost,
+                          c->stream));
+      ICK(cudaStreamSynchronize(c->stream));
+      return ICARAT_OK;
+    }
+  }
+  else if(apply_K_equations(c, u, y))
+    return ICARAT_OK;
   GridDev g{c->nx, c->ny, c->nz, c->NX, c->NY, c->NZ, c->numnp, c->nelx};
   to_full(c, u, c->d_v1, host);
   launch_apply_K(c, g, c->d_E, c->d_fix, c->d_v1, c->d_Ap, nullptr);

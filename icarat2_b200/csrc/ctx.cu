@@ -656,6 +656,32 @@ int icarat_ctx_create_sel_impl(const icarat_grid *grid, const icarat_material *m
                    cudaMemcpyHostToDevice));
     ICK(cudaMalloc(&c->d_fix, c->numnp));
     ICK(cudaMemcpy(c->d_fix, c->fix_h.data(), c->numnp, cudaMemcpyHostToDevice));
+    {
+      std::vector<int> base(c->numnp, 0);
+      bool consecutive = true;
+      for(long n = 0; n < c->numnp; n++)
+      {
+        int k = 0;
+        for(int q = 0; q < 3; q++)
+        {
+          const int eq = c->dof[3 * n + q];
+          const bool free = eq < c->numeq;
+          consecutive = consecutive && free == !((c->fix_h[n] >> q) & 1u);
+          if(!free)
+            continue;
+          if(k == 0)
+            base[n] = eq;
+          consecutive = consecutive && eq == base[n] + k;
+          k++;
+        }
+      }
+      if(consecutive)
+      {
+        ICK(cudaMalloc(&c->d_eqbase, sizeof(int) * (size_t)c->numnp));
+        ICK(cudaMemcpy(c->d_eqbase, base.data(), sizeof(int) * (size_t)c->numnp,
+                       cudaMemcpyHostToDevice));
+      }
+    }
     const size_t nv = (size_t)c->neq;
     c->d_fext = dalloc(nv);
     c->d_rhs = dalloc(nv);
@@ -731,6 +757,7 @@ int icarat_ctx_destroy_impl(icarat_ctx *c)
   dfree(c->d_sel_elem);
   dfree(c->d_sel_buf);
   dfree(c->d_free);
+  dfree(c->d_eqbase);
   dfree(c->d_fix);
   dfree(c->d_uD);
   for(double *p : {c->d_fext, c->d_rhs, c->d_u, c->d_invd, c->d_r, c->d_p,

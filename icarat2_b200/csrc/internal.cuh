@@ -383,6 +383,9 @@ struct icarat_ctx
   bool has_uD = false;
   // device
   int *d_free = nullptr;
+  // equation number of each node's first free component (null unless a node's
+  // equations are consecutive in component order, as countDOF numbers them)
+  int *d_eqbase = nullptr;
   uint8_t *d_fix = nullptr;
   double *d_uD = nullptr;
   double *d_fext = nullptr;
@@ -497,6 +500,9 @@ void dfree(void *p);
 void launch_apply_K(icarat_ctx *c, const GridDev &g, const double *E,
                     const uint8_t *fix, const double *u, double *y,
                     double *dot_partials);
+// y = K u on equation vectors (device); false where the fused form does not
+// apply (overlapping vectors, the tensor-core operator): nothing is done then
+bool apply_K_equations(icarat_ctx *c, const double *u, double *y);
 void launch_apply_K_f32(icarat_ctx *c, const GridDev &g, const float *E,
                         const uint8_t *fix, const float *u, float *y);
 void launch_diag(icarat_ctx *c, const GridDev &g, const double *E,

@@ -192,6 +192,46 @@ __device__ __forceinline__ ModalRhs<T> modal_rhs(const GridDev &g, const uint8_t
   return ModalRhs<T>{fix[n], {b[n], b[(long)g.numnp + n], b[2L * g.numnp + n]}};
 }
 
+// The march's input: a node vector (component-major), or an equation vector
+// of the ABI (free components only, node by node: node n's are at base[n],
+// in component order).  copy() starts the copies of node n for this thread's
+// staging slot q; next() is told, a layer ahead, which node comes next there.
+template <typename T> struct ModalNodes
+{
+  const T *u;
+  int numnp;
+  __device__ __forceinline__ void next(int, int, bool) {}
+  __device__ __forceinline__ void copy(int, int n, bool v, T *d0, T *d1, T *d2)
+  {
+    const T *src = u + (v ? n : 0);
+    modal_copy(d0, src, v);
+    modal_copy(d1, src + numnp, v);
+    modal_copy(d2, src + 2L * numnp, v);
+  }
+};
+struct ModalEquations
+{
+  const double *u;
+  const int *base;
+  const uint8_t *fix;
+  int at[2];
+  unsigned f[2];
+  __device__ __forceinline__ void next(int q, int n, bool v)
+  {
+    f[q] = v ? fix[n] : 7u;
+    at[q] = v ? base[n] : 0;
+  }
+  __device__ __forceinline__ void copy(int q, int, bool, double *d0, double *d1, double *d2)
+  {
+    const unsigned g = ~f[q];
+    const double *src = u + at[q];
+    const int o1 = g & 1, o2 = o1 + ((g >> 1) & 1);
+    modal_copy(d0, (g & 1) ? src : u, (g & 1) != 0);
+    modal_copy(d1, (g & 2) ? src + o1 : u, (g & 2) != 0);
+    modal_copy(d2, (g & 4) ? src + o2 : u, (g & 4) != 0);
+  }
+};
+
 // x and y sums and differences of the element's four nodes on one layer:
 // f[c][q], bit 0 of q the x difference, bit 1 the y difference
 template <typename T>
@@ -270,11 +310,10 @@ __device__ __forceinline__ void modal_element(const KhParam<T> &k, T E, const T 
 // barrier per layer: the forces of a layer and the epilogue's loads cross it,
 // and the layer is summed and emitted at the start of the next layer's turn
 // (two force buffers).
-template <typename T, typename L, typename F>
+template <typename T, typename S, typename L, typename F>
 __device__ __forceinline__ void modal_march(const GridDev &g, const ModalPlan &m,
-                                            const KhParam<T> &kh, const T *__restrict__ E,
-                                            const T *__restrict__ u, ModalShared<T> &sh, L &&load,
-                                            F &&emit)
+                                            const KhParam<T> &kh, const T *__restrict__ E, S src,
+                                            ModalShared<T> &sh, L &&load, F &&emit)
 {
   const int t = threadIdx.x;
   const int tx = t % m.W, ty = t / m.W;
@@ -311,11 +350,8 @@ __device__ __forceinline__ void modal_march(const GridDev &g, const ModalPlan &m
           const int e = t + q * ModalCfg<T>::threads;
           if(e < tile_nodes)
           {
-            const bool v = in && off[q] >= 0;
-            const T *src = u + (v ? off[q] + k * plane : 0);
-#pragma unroll
-            for(int c = 0; c < 3; c++)
-              modal_copy(&dst[c][e], src + (long)c * g.numnp, v);
+            src.copy(q, off[q] + k * plane, in && off[q] >= 0, &dst[0][e], &dst[1][e], &dst[2][e]);
+            src.next(q, off[q] + (k + 1) * plane, k + 1 >= 0 && k + 1 < g.NZ && off[q] >= 0);
           }
         }
       }
@@ -349,6 +385,9 @@ __device__ __forceinline__ void modal_march(const GridDev &g, const ModalPlan &m
     };
     if(item != (int)blockIdx.x)
       __syncthreads(); // the previous item's last layer has been read
+#pragma unroll
+    for(int q = 0; q < 2; q++)
+      src.next(q, off[q] + (k0 - 1) * plane, k0 >= 1 && off[q] >= 0);
 #pragma unroll
     for(int q = 0; q <= kModalAhead; q++)
       stage(k0 - 1 + q);
@@ -402,6 +441,15 @@ __device__ __forceinline__ void modal_march(const GridDev &g, const ModalPlan &m
     __syncthreads();
     finish(k1 - 1);
   }
+}
+
+// the same on a node vector u
+template <typename T, typename L, typename F>
+__device__ __forceinline__ void modal_march(const GridDev &g, const ModalPlan &m,
+                                            const KhParam<T> &kh, const T *__restrict__ E,
+                                            const T *u, ModalShared<T> &sh, L &&load, F &&emit)
+{
+  modal_march(g, m, kh, E, ModalNodes<T>{u, g.numnp}, sh, load, emit);
 }
 
 } // namespace icarat_b200

@@ -40,6 +40,54 @@ __global__ void __launch_bounds__(ModalCfg<double>::threads, ModalCfg<double>::b
   }
 }
 
+// y = K u on equation vectors (free components only) in one launch: the march
+// reads u through the nodes' first equation numbers and writes y the same
+// way.  With the scatter into a node vector before and the gather after it was
+// four launches (memset, scatter, product, gather) and twice the traffic.
+__global__ void __launch_bounds__(ModalCfg<double>::threads, ModalCfg<double>::blocks)
+    k_apply_K_eq(GridDev g, ModalPlan m, KhParam<double> kh, const double *__restrict__ E,
+                 const uint8_t *__restrict__ fix, const int *__restrict__ base,
+                 const double *__restrict__ u, double *__restrict__ y)
+{
+  ModalShared<double> &ms = modal_shared<double>();
+  ModalEquations src;
+  src.u = u;
+  src.base = base;
+  src.fix = fix;
+  struct Pre
+  {
+    unsigned f;
+    int at;
+  };
+  modal_march(g, m, kh, E, src, ms,
+              [&](int n) { return Pre{fix[n], base[n]}; },
+              [&](int, const double(&acc)[3], const double(&)[3], const Pre &pre)
+              {
+                double *out = y + pre.at;
+#pragma unroll
+                for(int q = 0; q < 3; q++)
+                  if(!((pre.f >> q) & 1u))
+                    *out++ = acc[q];
+              });
+}
+
+bool apply_K_equations(icarat_ctx *c, const double *u, double *y)
+{
+  const GridDev g{c->nx, c->ny, c->nz, c->NX, c->NY, c->NZ, c->numnp, c->nelx};
+  // blocks read u while others write y: they must not overlap
+  if(!c->d_eqbase || c->numeq == 0 || use_dmma(c, g) || (u < y + c->numeq && y < u + c->numeq))
+    return false;
+  int blocks;
+  size_t smem;
+  const ModalPlan m = modal_launch<double>(g, (const void *)k_apply_K_eq, c->sm_count, 1 << 30,
+                                           blocks, smem);
+  note_launch();
+  k_apply_K_eq<<<blocks, ModalCfg<double>::threads, smem, c->stream>>>(
+      g, m, c->kh, c->d_E, c->d_fix, c->d_eqbase, u, y);
+  ICK(cudaGetLastError());
+  return true;
+}
+
 // 1 / diag(K): d_(n,c) = sum_{e ∋ n} E_e Ke0[3a+c][3a+c]; 0 on constrained.
 __global__ void k_inv_diag(GridDev g, KeParam ke, const double *__restrict__ E,
                            const uint8_t *__restrict__ fix,

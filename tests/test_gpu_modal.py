@@ -45,3 +45,33 @@ def test_more_tiles_than_blocks(gpu):
     u = rng.standard_normal(G.numeq)
     ref = G.apply_K_op(u, gpu.OP_FP32)
     assert np.abs(G.apply_K(u) - ref).max() <= 1e-6 * np.abs(ref).max()
+
+
+def test_equation_vectors_partly_fixed_nodes(gpu, oracle):
+    """nodes with one, two or all components fixed on four faces, device
+    pointers, and the product in place (which keeps the scattered form)"""
+    import torch
+    nx, ny, nz = 21, 13, 17
+    faces = [((1, 1, 1), (0.0,) * 3, ((0.0, 0.0), (0.0, ny), (0.0, nz))),
+             ((0, 1, 0), (0.0,) * 3, ((0.0, nx), (0.0, 0.0), (0.0, nz))),
+             ((1, 0, 1), (0.0,) * 3, ((0.0, nx), (ny, ny), (0.0, nz))),
+             ((0, 0, 1), (0.0,) * 3, ((nx, nx), (0.0, ny), (0.0, 0.0)))]
+    loads = [((0.0, 0.0, -1.0), ((nx, nx), (6.0, 6.0), (9.0, 9.0)))]
+    P = oracle.Problem(nx, ny, nz, dirichlet=faces, loads=loads)
+    G = gpu.Context(nx, ny, nz, dirichlet=faces, loads=loads)
+    rng = np.random.default_rng(2)
+    rho, u = rng.uniform(0.05, 1.0, P.nelx), rng.standard_normal(P.numeq)
+    P.assemble(rho)
+    G.set_design(rho)
+    ref = P.apply_K(u)
+    d_u = torch.tensor(u, device="cuda")
+    d_y = torch.full_like(d_u, float("nan"))
+    torch.cuda.synchronize()
+    G.apply_K_dev(d_u.data_ptr(), d_y.data_ptr())
+    G.synchronize()
+    top = np.abs(ref).max()
+    assert np.abs(d_y.cpu().numpy() - ref).max() <= 1e-14 * top
+    assert np.abs(G.apply_K(u) - ref).max() <= 1e-14 * top
+    G.apply_K_dev(d_u.data_ptr(), d_u.data_ptr())
+    G.synchronize()
+    assert np.array_equal(d_u.cpu().numpy(), d_y.cpu().numpy())
