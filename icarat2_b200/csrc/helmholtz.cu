@@ -26,13 +26,6 @@
 namespace icarat_b200
 {
 
-// the CG start of pcg.cu
-__global__ void k_cg_init(int n, const double *__restrict__ b,
-                          const double *__restrict__ invd, double *__restrict__ x,
-                          double *__restrict__ r, double *__restrict__ z,
-                          double *__restrict__ p, double *__restrict__ partials,
-                          CgScalars *s, double tol, int maxit, int jacobi);
-
 namespace
 {
 
@@ -63,49 +56,94 @@ __device__ __forceinline__ int node_class(int i, int n)
   return i == 0 ? 0 : (i == n - 1 ? 2 : 1);
 }
 
-// F = sum over the node's elements of s_e nj[a] (/8 for the sensitivity
-// call), elements in ascending id like the reference's assembly
-__global__ void k_helm_rhs(HelmGrid g, HelmWeights w, const double *__restrict__ in,
-                           double *__restrict__ F, int sens)
+// Jacobi inverse diagonal per node class (27 values, 1 / centre coefficient
+// of the class row)
+struct HelmInvd
 {
+  double v[kHelmClasses];
+};
+
+__device__ __forceinline__ int helm_class(const HelmGrid &g, int n)
+{
+  const int i = n % g.NX, rest = n / g.NX, j = rest % g.NY, k = rest / g.NY;
+  return node_class(i, g.NX) + 3 * node_class(j, g.NY) + 9 * node_class(k, g.nz + 1);
+}
+
+// The CG's start: r = F = sum over the node's elements of s_e nj[a] (/8 for the
+// sensitivity call), elements in ascending id like the reference's assembly,
+// x = 0, z.r with z = D^-1 r, ||F|| and the loop's scalars (as k_cg_init of
+// pcg.cu sets them; beta = 0 makes the first direction z).
+__global__ void k_helm_start(HelmGrid g, HelmWeights w, HelmInvd iv, const double *__restrict__ in,
+                             double *__restrict__ x, double *__restrict__ r, int sens,
+                             double *__restrict__ partials, CgScalars *s, double tol, int maxit)
+{
+  __shared__ double sh[64];
+  double zr = 0.0, bb = 0.0;
   for(int n = blockIdx.x * blockDim.x + threadIdx.x; n < g.numnp;
       n += gridDim.x * blockDim.x)
   {
     const int i = n % g.NX, rest = n / g.NX, j = rest % g.NY, k = rest / g.NY;
+    // all eight loads first (an element outside is read as the node's own and
+    // left out)
+    const int e0 = min(i, g.nx - 1) + min(j, g.ny - 1) * g.nx + min(k, g.nz - 1) * g.nx * g.ny;
+    double se[8];
+    bool have[8];
+#pragma unroll
+    for(int q = 0; q < 8; q++) // ascending element id
+    {
+      const int ei = i - 1 + (q & 1), ej = j - 1 + ((q >> 1) & 1), ek = k - 1 + (q >> 2);
+      have[q] = ei >= 0 && ei < g.nx && ej >= 0 && ej < g.ny && ek >= 0 && ek < g.nz;
+      se[q] = __ldg(in + (have[q] ? ei + ej * g.nx + ek * g.nx * g.ny : e0));
+    }
     double f = 0.0;
-    for(int oz = -1; oz <= 0; oz++)
-      for(int oy = -1; oy <= 0; oy++)
-        for(int ox = -1; ox <= 0; ox++)
-        {
-          const int ei = i + ox, ej = j + oy, ek = k + oz;
-          if(ei < 0 || ei >= g.nx || ej < 0 || ej >= g.ny || ek < 0 || ek >= g.nz)
-            continue;
-          const int a = -ox - 2 * oy - 4 * oz;
-          double fe = __dmul_rn(__ldg(in + ei + (long)ej * g.nx + (long)ek * g.nx * g.ny),
-                                w.nj[a]);
-          if(sens)
-            fe = __ddiv_rn(fe, 8.0);
-          f = __dadd_rn(f, fe);
-        }
-    F[n] = f;
+#pragma unroll
+    for(int q = 0; q < 8; q++)
+    {
+      double fe = __dmul_rn(se[q], w.nj[7 - q]);
+      if(sens)
+        fe = __dmul_rn(fe, 0.125); // = fe / 8 in every case
+      f = have[q] ? __dadd_rn(f, fe) : f;
+    }
+    x[n] = 0.0;
+    r[n] = f;
+    const double z = f * iv.v[helm_class(g, n)];
+    zr += z * f;
+    bb += f * f;
   }
-}
-
-// inverse of the stencil's centre coefficient (the Jacobi preconditioner)
-__global__ void k_helm_invd(HelmGrid g, const double *__restrict__ coef,
-                            double *__restrict__ invd)
-{
-  for(int n = blockIdx.x * blockDim.x + threadIdx.x; n < g.numnp;
-      n += gridDim.x * blockDim.x)
+  double v[2] = {zr, bb};
+  block_sum<2>(v, sh);
+  if(threadIdx.x == 0)
   {
-    const int i = n % g.NX, rest = n / g.NX, j = rest % g.NY, k = rest / g.NY;
-    const int NZ = g.nz + 1;
-    const int cls = node_class(i, g.NX) + 3 * node_class(j, g.NY) + 9 * node_class(k, NZ);
-    invd[n] = 1.0 / coef[27 * cls + 13];
+    partials[blockIdx.x] = v[0];
+    partials[gridDim.x + blockIdx.x] = v[1];
+  }
+  if(last_block(&s->counter))
+  {
+    double t[2];
+    sum_partials<2>(partials, gridDim.x, t, sh);
+    if(threadIdx.x == 0)
+    {
+      s->zr = t[0];
+      s->beta = 0.0;
+      s->bnorm = sqrt(t[1]);
+      s->rnorm = s->bnorm;
+      s->tol = tol;
+      s->maxit = maxit;
+      s->iter = 0;
+      s->status = ICARAT_OK;
+      s->done = (t[1] == 0.0) ? 1 : 0;
+      if(!(t[1] == t[1]))
+      {
+        s->done = 1;
+        s->status = ICARAT_ERR_NAN;
+      }
+      s->counter = 0;
+    }
   }
 }
 
-// Ap = K p and alpha = zr / (p . Ap), by sum factorisation.
+// p = z + beta p (z = D^-1 r), Ap = K p and alpha = zr / (p . Ap), by sum
+// factorisation.
 //
 // With trilinear shape functions and exact 2-point Gauss rules the element
 // matrix is a tensor product, Ke = Mx (x) My (x) Mz + c (Sx (x) My (x) Mz +
@@ -116,190 +154,196 @@ __global__ void k_helm_invd(HelmGrid g, const double *__restrict__ coef,
 // through two in-plane sums per node, A = (mx my + c (sx my + mx sy)) p and
 // B = mx my p, and Ap(k) = sum_dz mz A(k+dz) + c sz B(k+dz).
 //
-// A block of 8 warps owns 32 x 8 kHelmRows node columns (a warp kHelmRows
-// rows of 32 nodes along x) and marches through kHelmTz planes, holding A
-// and B of planes k-1, k, k+1 in registers.  The planes of p come through
-// shared memory: a ring of kHelmDepth halo tiles filled by cp.async,
-// kHelmDepth - 1 planes ahead of the plane being reduced, so later planes
-// are in flight without holding registers.  Positions outside the box are
-// stored as 0 (their stencil weights are 0 as well).  Measured on the B200
-// at 257 x 129 x 129 nodes: about 50 us per launch, like a variant with a
-// one-plane register lookahead and one with two rows per thread; the limit
-// is dependent-latency (FP64 FMA chains, barriers), not DRAM.
-constexpr int kHelmTx = 32, kHelmWarps = 8, kHelmRows = 1, kHelmTz = 16, kHelmDepth = 4;
-constexpr int kHelmTy = kHelmWarps * kHelmRows;
+// A block of 8 warps owns 32 x 8 node columns and marches through kz planes,
+// holding A and B of planes k-1, k, k+1 in registers.  r and the old p come
+// through rings of halo tiles filled by cp.async kHelmAhead planes ahead; one
+// plane ahead of the sums the block forms the new p in a tile of its own (and
+// its owner stores it, into the other of two vectors: neighbours still read
+// the old one), so a plane costs one barrier and p costs no pass of its own.
+// Positions outside the box are stored as 0 (their stencil weights are 0 as
+// well).  Bound by memory (32 bytes per node) and the barrier per plane.
+// Measured on a B200 at 257 x 129 x 129 nodes: the product alone took 50 us and
+// the update of p another 24; this kernel takes 49.
+// Two rows per thread at two blocks per SM: one row 56 us, three blocks (80
+// registers) 48 there but slower on smaller grids, and a variant that spills
+// 80 bytes 95.
+constexpr int kHelmRows = 2, kHelmTx = 32, kHelmTy = kHelmRows * kHelmThreads / 32;
+constexpr int kHelmRing = 4, kHelmAhead = 2, kHelmBlocks = 2;
 constexpr int kHaloX = kHelmTx + 2, kHaloY = kHelmTy + 2, kHalo = kHaloX * kHaloY;
-constexpr int kStage = (kHalo + kHelmTx * kHelmWarps - 1) / (kHelmTx * kHelmWarps);
+constexpr int kStage = (kHalo + kHelmThreads - 1) / kHelmThreads;
 
-// 1-D stencils [axis][class][d + 1] and the diffusion coefficient c
+// 1-D stencils per axis: neighbour weights mo, so (a neighbour outside the box
+// is staged as 0, so they hold for every node) and centre weights md, sd of a
+// face node (twice that inside); the diffusion coefficient c
 struct HelmAxes
 {
-  double m[3][3][3], s[3][3][3];
+  double mo[3], so[3], md[3], sd[3];
   double c;
 };
 
-// 8-byte global -> shared copies (cp.async), one commit group per staged
-// plane, and a wait for all but the newest kHelmDepth - 1 groups
-__device__ __forceinline__ void cp_async8(double *dst, const double *src)
+// tiles of kHelmTx x kHelmTy columns and chunks of kz planes
+struct HelmPlan
 {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit()
-{
-  asm volatile("cp.async.commit_group;\n" ::: "memory");
-}
-__device__ __forceinline__ void cp_async_wait_ring()
-{
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(kHelmDepth - 1) : "memory");
-}
-
-// this thread's staged halo positions: in-plane offset (or -1 outside)
-struct HelmStage
-{
-  long off[kStage];
+  int tiles_x, tiles_y, kz, items;
 };
 
-// halo tile of plane kk (rows j0-1 .. j0+kHelmTy, columns i0-1 .. i0+32)
-// into buf; one commit group per call, empty when the plane is not needed
-__device__ __forceinline__ void helm_stage(double *buf, const double *__restrict__ p,
-                                          const HelmStage &st, int NZ, long plane, int kk,
-                                          bool needed)
+struct HelmShared
 {
-  if(needed)
-  {
-    const bool inz = kk >= 0 && kk < NZ;
-#pragma unroll
-    for(int q = 0; q < kStage; q++)
-    {
-      const int e = threadIdx.x + q * kHelmTx * kHelmWarps;
-      if(e < kHalo)
-      {
-        if(inz && st.off[q] >= 0)
-          cp_async8(buf + e, p + st.off[q] + kk * plane);
-        else
-          buf[e] = 0.0;
-      }
-    }
-  }
-  cp_async_commit();
+  double r[kHelmRing][kHalo], p[kHelmRing][kHalo], q[2][kHalo];
+};
+
+// 8-byte global -> shared copy, 0 where !valid
+__device__ __forceinline__ void cp_async8(double *dst, const double *src, bool valid)
+{
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  const int n = valid ? 8 : 0;
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src), "r"(n)
+               : "memory");
 }
 
-__global__ void __launch_bounds__(kHelmTx * kHelmWarps)
-    k_helm_spmv(HelmGrid g, HelmAxes ax, const double *__restrict__ p,
-                double *__restrict__ Ap, double *__restrict__ partials, CgScalars *s)
+__global__ void __launch_bounds__(kHelmThreads, kHelmBlocks)
+    k_helm_step(HelmGrid g, HelmPlan pl, const __grid_constant__ HelmAxes ax,
+                const __grid_constant__ HelmInvd iv, const double *__restrict__ r,
+                const double *__restrict__ p, double *__restrict__ pn, double *__restrict__ Ap,
+                double *__restrict__ partials, CgScalars *s)
 {
   chain_wait();
-  __shared__ double ring[kHelmDepth][kHalo];
-  __shared__ double sh[64];
+  extern __shared__ __align__(16) unsigned char helm_raw[];
+  HelmShared &S = *reinterpret_cast<HelmShared *>(helm_raw);
+  __shared__ double sh[32], s_iv[kHelmClasses];
   if(s->done)
     return;
+  if(threadIdx.x < kHelmClasses)
+    s_iv[threadIdx.x] = iv.v[threadIdx.x];
+  const double beta = s->beta;
   const int NZ = g.nz + 1;
-  const long plane = (long)g.NX * g.NY;
-  const int tiles_x = (g.NX + kHelmTx - 1) / kHelmTx, tiles_y = (g.NY + kHelmTy - 1) / kHelmTy;
-  const int tiles = tiles_x * tiles_y * ((NZ + kHelmTz - 1) / kHelmTz);
+  const int plane = g.NX * g.NY;
   const double c = ax.c;
   const int lx = threadIdx.x & 31, ly = (threadIdx.x >> 5) * kHelmRows;
   double dot = 0.0;
-  for(int t = blockIdx.x; t < tiles; t += gridDim.x)
+  for(int t = blockIdx.x; t < pl.items; t += gridDim.x)
   {
-    const int i0 = (t % tiles_x) * kHelmTx, j0 = (t / tiles_x % tiles_y) * kHelmTy;
-    const int k0 = t / (tiles_x * tiles_y) * kHelmTz;
-    const int k1 = min(k0 + kHelmTz, NZ);
-    const int i = i0 + lx;
-    HelmStage st;
+    const int i0 = t % pl.tiles_x * kHelmTx, j0 = t / pl.tiles_x % pl.tiles_y * kHelmTy;
+    const int k0 = t / (pl.tiles_x * pl.tiles_y) * pl.kz;
+    const int k1 = min(k0 + pl.kz, NZ);
+    const int i = i0 + lx, j = j0 + ly;
+    // this thread's staged cells: in-plane offset (-1 outside), class of x and
+    // y, whether the block owns the column
+    int off[kStage], cls[kStage];
+    bool own[kStage];
 #pragma unroll
     for(int q = 0; q < kStage; q++)
     {
-      const int e = threadIdx.x + q * kHelmTx * kHelmWarps;
-      const int x = i0 - 1 + e % kHaloX, y = j0 - 1 + e / kHaloX;
-      st.off[q] = (x >= 0 && x < g.NX && y >= 0 && y < g.NY) ? x + (long)y * g.NX : -1;
+      const int e = threadIdx.x + q * kHelmThreads;
+      const int hx = e % kHaloX, hy = e / kHaloX;
+      const int x = i0 - 1 + hx, y = j0 - 1 + hy;
+      const bool in = e < kHalo && x >= 0 && x < g.NX && y >= 0 && y < g.NY;
+      off[q] = in ? x + y * g.NX : -1;
+      cls[q] = in ? node_class(x, g.NX) + 3 * node_class(y, g.NY) : 0;
+      own[q] = in && hx > 0 && hx <= kHelmTx && hy > 0 && hy <= kHelmTy;
     }
-    double mx[3], sx[3], my[kHelmRows][3], sy[kHelmRows][3];
-    const int cx = node_class(min(i, g.NX - 1), g.NX);
-#pragma unroll
-    for(int d = 0; d < 3; d++)
-    {
-      mx[d] = ax.m[0][cx][d];
-      sx[d] = ax.s[0][cx][d];
-    }
-#pragma unroll
-    for(int r = 0; r < kHelmRows; r++)
-    {
-      const int cy = node_class(min(j0 + ly + r, g.NY - 1), g.NY);
-#pragma unroll
-      for(int d = 0; d < 3; d++)
+    auto stage = [&](int k) { // raw plane k into its ring slot
+      if(k <= k1)
       {
-        my[r][d] = ax.m[1][cy][d];
-        sy[r][d] = ax.s[1][cy][d];
-      }
-    }
-    // planes k0-1 .. k1 are reduced, plane m in ring slot (m - k0 + 1) % depth;
-    // the ring of the previous tile is no longer read past this barrier, and
-    // every copy of that tile has landed (its groups past plane k1 were empty)
-    __syncthreads();
+        const int slot = (k - k0 + 1) & (kHelmRing - 1);
+        const bool inz = k >= 0 && k < NZ;
 #pragma unroll
-    for(int q = 0; q < kHelmDepth; q++)
-      helm_stage(ring[q], p, st, NZ, plane, k0 - 1 + q, k0 - 1 + q <= k1);
-    double A0[kHelmRows], B0[kHelmRows], A1[kHelmRows], B1[kHelmRows], A2[kHelmRows],
-        B2[kHelmRows], P1[kHelmRows], P2[kHelmRows];
-    for(int m = k0 - 1; m <= k1; m++)
-    {
-      const int slot = (m - k0 + 1) % kHelmDepth;
-      cp_async_wait_ring();
-      __syncthreads();
-      {
-        const double *buf = ring[slot] + ly * kHaloX + lx;
-        double rm[kHelmRows + 2], rs[kHelmRows + 2];
-#pragma unroll
-        for(int q = 0; q < kHelmRows + 2; q++)
+        for(int q = 0; q < kStage; q++)
         {
-          const double vl = buf[q * kHaloX], v0 = buf[q * kHaloX + 1], vr = buf[q * kHaloX + 2];
-          rm[q] = mx[0] * vl + mx[1] * v0 + mx[2] * vr;
-          rs[q] = sx[0] * vl + sx[1] * v0 + sx[2] * vr;
-          if(q >= 1 && q <= kHelmRows)
-            P2[q - 1] = v0;
-        }
-#pragma unroll
-        for(int r = 0; r < kHelmRows; r++)
-        {
-          const double pm = my[r][0] * rm[r] + my[r][1] * rm[r + 1] + my[r][2] * rm[r + 2];
-          const double ps = my[r][0] * rs[r] + my[r][1] * rs[r + 1] + my[r][2] * rs[r + 2] +
-                            sy[r][0] * rm[r] + sy[r][1] * rm[r + 1] + sy[r][2] * rm[r + 2];
-          A2[r] = pm + c * ps;
-          B2[r] = pm;
-        }
-      }
-      __syncthreads(); // every thread has read the slot: refill it
-      helm_stage(ring[slot], p, st, NZ, plane, m + kHelmDepth, m + kHelmDepth <= k1);
-      if(m >= k0 + 1)
-      {
-        // output plane k = m - 1 from planes k-1, k, k+1
-        const int k = m - 1;
-        const int cz = node_class(k, NZ);
-        const double mz0 = ax.m[2][cz][0], mz1 = ax.m[2][cz][1], mz2 = ax.m[2][cz][2];
-        const double sz0 = ax.s[2][cz][0], sz1 = ax.s[2][cz][1], sz2 = ax.s[2][cz][2];
-#pragma unroll
-        for(int r = 0; r < kHelmRows; r++)
-        {
-          const double y = mz0 * A0[r] + mz1 * A1[r] + mz2 * A2[r] +
-                           c * (sz0 * B0[r] + sz1 * B1[r] + sz2 * B2[r]);
-          const int j = j0 + ly + r;
-          if(i < g.NX && j < g.NY)
+          const int e = threadIdx.x + q * kHelmThreads;
+          if(e < kHalo)
           {
-            Ap[i + (long)j * g.NX + (long)k * plane] = y;
-            dot += P1[r] * y;
+            const bool v = inz && off[q] >= 0;
+            const int n = v ? off[q] + k * plane : 0;
+            cp_async8(&S.r[slot][e], r + n, v);
+            cp_async8(&S.p[slot][e], p + n, v);
           }
         }
       }
+      asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    auto combine = [&](int k) { // new p of plane k
+      if(k > k1)
+        return;
+      const int slot = (k - k0 + 1) & (kHelmRing - 1);
+      const int cz = 9 * node_class(min(max(k, 0), NZ - 1), NZ);
+      const bool mine = k >= k0 && k < k1;
 #pragma unroll
-      for(int r = 0; r < kHelmRows; r++)
+      for(int q = 0; q < kStage; q++)
       {
-        A0[r] = A1[r];
-        B0[r] = B1[r];
-        A1[r] = A2[r];
-        B1[r] = B2[r];
-        P1[r] = P2[r];
+        const int e = threadIdx.x + q * kHelmThreads;
+        if(e < kHalo)
+        {
+          const double z = S.r[slot][e] * s_iv[cls[q] + cz];
+          const double v = beta == 0.0 ? z : fma(beta, S.p[slot][e], z);
+          S.q[(k - k0) & 1][e] = v;
+          if(mine && own[q])
+            pn[off[q] + k * plane] = v;
+        }
+      }
+    };
+    // centre weights of this thread's nodes
+    const double ex = node_class(min(i, g.NX - 1), g.NX) == 1 ? 2.0 : 1.0;
+    const double mx = ex * ax.md[0], sx = ex * ax.sd[0];
+    double my[kHelmRows], sy[kHelmRows];
+#pragma unroll
+    for(int q = 0; q < kHelmRows; q++)
+    {
+      const double ey = node_class(min(j + q, g.NY - 1), g.NY) == 1 ? 2.0 : 1.0;
+      my[q] = ey * ax.md[1];
+      sy[q] = ey * ax.sd[1];
+    }
+    __syncthreads(); // the previous item's tiles have been read, s_iv is set
+#pragma unroll
+    for(int q = 0; q <= kHelmAhead; q++)
+      stage(k0 - 1 + q);
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(kHelmAhead) : "memory");
+    __syncthreads();
+    combine(k0 - 1);
+    // per row: L = this plane's share of either neighbour plane's K p, done =
+    // the output plane's sum but for the plane above, its p
+    double L[kHelmRows] = {}, done[kHelmRows] = {}, pc[kHelmRows] = {};
+    for(int m = k0 - 1; m <= k1; m++)
+    {
+      // raw plane m + 1 has landed and the new p of plane m is complete
+      asm volatile("cp.async.wait_group %0;\n" ::"n"(kHelmAhead - 1) : "memory");
+      __syncthreads();
+      stage(m + 1 + kHelmAhead);
+      combine(m + 1);
+      const double *buf = S.q[(m - k0) & 1] + ly * kHaloX + lx;
+      double rm[kHelmRows + 2], rs[kHelmRows + 2], pn0[kHelmRows];
+#pragma unroll
+      for(int q = 0; q < kHelmRows + 2; q++)
+      {
+        const double v0 = buf[q * kHaloX + 1], t = buf[q * kHaloX] + buf[q * kHaloX + 2];
+        rm[q] = fma(ax.mo[0], t, mx * v0);
+        rs[q] = fma(ax.so[0], t, sx * v0);
+        if(q >= 1 && q <= kHelmRows)
+          pn0[q - 1] = v0;
+      }
+      const double ez = node_class(min(max(m, 0), NZ - 1), NZ) == 1 ? 2.0 : 1.0;
+      const double mz = ez * ax.md[2], sz = ez * ax.sd[2] * ax.c, so = ax.so[2] * ax.c;
+#pragma unroll
+      for(int q = 0; q < kHelmRows; q++)
+      {
+        const double tm = rm[q] + rm[q + 2], ts = rs[q] + rs[q + 2];
+        const double B = fma(ax.mo[1], tm, my[q] * rm[q + 1]);
+        const double D = fma(ax.so[1], tm, sy[q] * rm[q + 1]) +
+                         fma(ax.mo[1], ts, my[q] * rs[q + 1]);
+        const double A = fma(ax.c, D, B);
+        const double up = fma(so, B, ax.mo[2] * A);
+        if(m >= k0 + 1)
+        {
+          const double y = done[q] + up;
+          if(i < g.NX && j + q < g.NY)
+          {
+            Ap[i + (j + q) * g.NX + (m - 1) * plane] = y;
+            dot += pc[q] * y;
+          }
+        }
+        done[q] = L[q] + fma(sz, B, mz * A);
+        L[q] = up;
+        pc[q] = pn0[q];
       }
     }
   }
@@ -320,24 +364,9 @@ __global__ void __launch_bounds__(kHelmTx * kHelmWarps)
   }
 }
 
-// Jacobi inverse diagonal per node class (27 values, 1 / centre coefficient
-// of the class row)
-struct HelmInvd
-{
-  double v[kHelmClasses];
-};
-
-__device__ __forceinline__ int helm_class(const HelmGrid &g, int n)
-{
-  const int i = n % g.NX, rest = n / g.NX, j = rest % g.NY, k = rest / g.NY;
-  return node_class(i, g.NX) + 3 * node_class(j, g.NY) + 9 * node_class(k, g.nz + 1);
-}
-
 // The Jacobi CG update of k_cg_update_jacobi (x += alpha p, r -= alpha Ap,
 // z = D^-1 r, beta, stop test) with D^-1 taken from the node's class instead
-// of a vector and z not stored: k_helm_pupdate forms it again from r, with
-// the same operations, so the iterates are those of the generic kernels on
-// 16 bytes per node less.
+// of a vector and z not stored: the next k_helm_step forms it again from r.
 __global__ void k_helm_update(HelmGrid g, HelmInvd iv, double *__restrict__ x,
                               double *__restrict__ r, const double *__restrict__ p,
                               const double *__restrict__ Ap, double *__restrict__ partials,
@@ -381,19 +410,6 @@ __global__ void k_helm_update(HelmGrid g, HelmInvd iv, double *__restrict__ x,
   }
 }
 
-// p = z + beta p with z = D^-1 r
-__global__ void k_helm_pupdate(HelmGrid g, HelmInvd iv, const double *__restrict__ r,
-                               double *__restrict__ p, const CgScalars *s)
-{
-  chain_wait();
-  if(s->done)
-    return;
-  const double beta = s->beta;
-  for(int n = blockIdx.x * blockDim.x + threadIdx.x; n < g.numnp;
-      n += gridDim.x * blockDim.x)
-    p[n] = beta * p[n] + r[n] * iv.v[helm_class(g, n)];
-}
-
 // out_e = sum_a ns[a] val[node_a] (/8 for the density call)
 __global__ void k_helm_out(HelmGrid g, HelmWeights w, const double *__restrict__ val,
                            double *__restrict__ out, int sens)
@@ -411,7 +427,7 @@ __global__ void k_helm_out(HelmGrid g, HelmWeights w, const double *__restrict__
       const long m = n0 + (a & 1) + ((a >> 1) & 1) * (long)g.NX + ((a >> 2) & 1) * plane;
       s = __dadd_rn(s, __dmul_rn(w.ns[a], __ldg(val + m)));
     }
-    out[e] = sens ? s : __ddiv_rn(s, 8.0);
+    out[e] = sens ? s : __dmul_rn(s, 0.125); // = s / 8 in every case
   }
 }
 
@@ -523,16 +539,10 @@ static HelmAxes helm_axes(const icarat_ctx *c)
   const double h[3] = {c->hx, c->hy, c->hz};
   for(int d = 0; d < 3; d++)
   {
-    const double md = h[d] / 3.0, mo = h[d] / 6.0, sd = 1.0 / h[d], so = -1.0 / h[d];
-    // class 0: only the element above; 1: both; 2: only the element below
-    const double m[3][3] = {{0.0, md, mo}, {mo, md + md, mo}, {mo, md, 0.0}};
-    const double s[3][3] = {{0.0, sd, so}, {so, sd + sd, so}, {so, sd, 0.0}};
-    for(int k = 0; k < 3; k++)
-      for(int q = 0; q < 3; q++)
-      {
-        a.m[d][k][q] = m[k][q];
-        a.s[d][k][q] = s[k][q];
-      }
+    a.mo[d] = h[d] / 6.0;
+    a.md[d] = h[d] / 3.0;
+    a.so[d] = -1.0 / h[d];
+    a.sd[d] = 1.0 / h[d];
   }
   a.c = std::pow(c->helm.radius / (2.0 * std::sqrt(3.0)), 2);
   return a;
@@ -543,8 +553,7 @@ void helm_free(icarat_ctx *c)
   HelmState &H = c->helm;
   if(H.exec)
     cudaGraphExecDestroy(H.exec);
-  for(double *p : {H.d_coef, H.d_invd, H.d_F, H.d_val, H.d_r, H.d_z, H.d_p, H.d_Ap,
-                   H.d_partials, H.d_oc})
+  for(double *p : {H.d_val, H.d_r, H.d_p[0], H.d_p[1], H.d_Ap, H.d_partials, H.d_oc})
     dfree(p);
   dfree(H.d_cg);
   H = HelmState{};
@@ -564,23 +573,17 @@ void helm_setup(icarat_ctx *c, double R)
   for(int q = 0; q < kHelmClasses; q++)
     H.invd_cls[q] = 1.0 / coef[27 * q + 13];
   const size_t n = (size_t)c->numnp;
-  H.d_coef = dalloc(kHelmClasses * 27);
-  ICK(cudaMemcpy(H.d_coef, coef, sizeof(coef), cudaMemcpyHostToDevice));
-  H.d_invd = dalloc(n);
-  H.d_F = dalloc(n);
   H.d_val = dalloc(n);
   H.d_r = dalloc(n);
-  H.d_z = dalloc(n);
-  H.d_p = dalloc(n);
+  H.d_p[0] = dalloc(n);
+  H.d_p[1] = dalloc(n);
   H.d_Ap = dalloc(n);
   H.d_partials = dalloc((size_t)kMaxRedBlocks * 2);
   H.d_oc = dalloc(3 * (size_t)c->nelx);
   ICK(cudaMalloc(&H.d_cg, sizeof(CgScalars)));
   ICK(cudaMemsetAsync(H.d_cg, 0, sizeof(CgScalars), c->stream));
-  note_launch();
-  k_helm_invd<<<blocks_for(n, kHelmThreads, 4 * c->sm_count), kHelmThreads, 0, c->stream>>>(
-      hgrid(c), H.d_coef, H.d_invd);
-  ICK(cudaGetLastError());
+  ICK(cudaFuncSetAttribute(k_helm_step, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)sizeof(HelmShared)));
   H.ready = true;
 }
 
@@ -588,27 +591,53 @@ void helm_setup(icarat_ctx *c, double R)
 // occupancy; 4 per SM left them at 3-4 TB/s on the B200)
 static int helm_red_blocks(const icarat_ctx *c)
 {
-  return 8 * c->sm_count < kMaxRedBlocks ? 8 * c->sm_count : kMaxRedBlocks;
+  const int need = (c->numnp + 511) / 512;
+  const int most = 8 * c->sm_count < kMaxRedBlocks ? 8 * c->sm_count : kMaxRedBlocks;
+  return need < 1 ? 1 : (need < most ? need : most);
 }
 
-static void helm_iteration(icarat_ctx *c)
+// Planes per item for the least of waves x (planes + start-up): two planes of
+// halo are formed again per chunk and kHelmBlocks blocks fit an SM.
+static HelmPlan helm_plan(const icarat_ctx *c)
 {
-  HelmState &H = c->helm;
-  const int n = c->numnp;
-  const int rb = helm_red_blocks(c);
-  const long tiles = (long)((c->NX + kHelmTx - 1) / kHelmTx) *
-                    ((c->NY + kHelmTy - 1) / kHelmTy) * ((c->NZ + kHelmTz - 1) / kHelmTz);
-  note_launch(3);
-  launch_chained(k_helm_spmv, blocks_for(tiles, 1, kMaxRedBlocks), kHelmTx * kHelmWarps, 0,
-                 c->stream, hgrid(c), helm_axes(c), H.d_p, H.d_Ap, H.d_partials, H.d_cg);
+  HelmPlan p{(c->NX + kHelmTx - 1) / kHelmTx, (c->NY + kHelmTy - 1) / kHelmTy, c->NZ, 0};
+  const long tiles = (long)p.tiles_x * p.tiles_y, slots = (long)kHelmBlocks * c->sm_count;
+  double best = 0.0;
+  for(int kz = 1; kz <= c->NZ; kz++)
+  {
+    const long items = tiles * ((c->NZ + kz - 1) / kz);
+    const double cost = (double)((items + slots - 1) / slots) * (kz + 4.0);
+    if(best == 0.0 || cost <= best)
+    {
+      best = cost;
+      p.kz = kz;
+    }
+  }
+  p.items = (int)(tiles * ((c->NZ + p.kz - 1) / p.kz));
+  return p;
+}
+
+static HelmInvd helm_invd(const icarat_ctx *c)
+{
   HelmInvd iv;
   for(int q = 0; q < kHelmClasses; q++)
-    iv.v[q] = H.invd_cls[q];
-  (void)n;
-  launch_chained(k_helm_update, rb, kRedThreads, 0, c->stream, hgrid(c), iv, H.d_val, H.d_r,
-                 H.d_p, H.d_Ap, H.d_partials, H.d_cg);
-  launch_chained(k_helm_pupdate, rb, kRedThreads, 0, c->stream, hgrid(c), iv, H.d_r, H.d_p,
-                 H.d_cg);
+    iv.v[q] = c->helm.invd_cls[q];
+  return iv;
+}
+
+// iteration k of a chunk: the directions alternate between the two vectors
+static void helm_iteration(icarat_ctx *c, int k)
+{
+  HelmState &H = c->helm;
+  const HelmPlan pl = helm_plan(c);
+  const HelmInvd iv = helm_invd(c);
+  const int blocks = pl.items < kMaxRedBlocks ? pl.items : kMaxRedBlocks;
+  double *from = H.d_p[k & 1], *to = H.d_p[1 - (k & 1)];
+  note_launch(2);
+  launch_chained(k_helm_step, blocks, kHelmThreads, sizeof(HelmShared), c->stream, hgrid(c), pl,
+                 helm_axes(c), iv, H.d_r, from, to, H.d_Ap, H.d_partials, H.d_cg);
+  launch_chained(k_helm_update, helm_red_blocks(c), kRedThreads, 0, c->stream, hgrid(c), iv,
+                 H.d_val, H.d_r, to, H.d_Ap, H.d_partials, H.d_cg);
   ICK(cudaGetLastError());
 }
 
@@ -618,26 +647,22 @@ int helm_filter(icarat_ctx *c, const double *in, double *out, bool is_sens, doub
                 int maxit, icarat_solve_info *info)
 {
   HelmState &H = c->helm;
-  IREQUIRE(H.d_coef != nullptr, ICARAT_ERR_STATE, "Helmholtz filter not set up");
+  IREQUIRE(H.ready, ICARAT_ERR_STATE, "Helmholtz filter not set up");
   IREQUIRE(std::isfinite(rtol), ICARAT_ERR_ARG, "rtol must be finite");
   if(rtol <= 0.0)
     rtol = 1.0e-10;
   if(maxit <= 0)
     maxit = 10000;
-  const int n = c->numnp;
-  const int eb = blocks_for(n, kHelmThreads, 4 * c->sm_count);
   HelmWeights w;
   for(int a = 0; a < 8; a++)
   {
     w.nj[a] = H.nj[a];
     w.ns[a] = H.ns[a];
   }
-  note_launch(2);
-  k_helm_rhs<<<eb, kHelmThreads, 0, c->stream>>>(hgrid(c), w, in, H.d_F, is_sens ? 1 : 0);
-  ICK(cudaGetLastError());
-  k_cg_init<<<helm_red_blocks(c), kRedThreads, 0, c->stream>>>(n, H.d_F, H.d_invd, H.d_val,
-                                                          H.d_r, H.d_z, H.d_p, H.d_partials,
-                                                          H.d_cg, rtol, maxit, 1);
+  note_launch();
+  k_helm_start<<<helm_red_blocks(c), kRedThreads, 0, c->stream>>>(
+      hgrid(c), w, helm_invd(c), in, H.d_val, H.d_r, is_sens ? 1 : 0, H.d_partials, H.d_cg, rtol,
+      maxit);
   ICK(cudaGetLastError());
   if(!H.exec)
   {
@@ -647,7 +672,7 @@ int helm_filter(icarat_ctx *c, const double *in, double *out, bool is_sens, doub
     try
     {
       for(int k = 0; k < kHelmChunk; k++)
-        helm_iteration(c);
+        helm_iteration(c, k);
     }
     catch(...)
     {
@@ -669,7 +694,7 @@ int helm_filter(icarat_ctx *c, const double *in, double *out, bool is_sens, doub
     if(c->h_cg->done)
       break;
     ICK(cudaGraphLaunch(H.exec, c->stream));
-    note_launch(3 * kHelmChunk);
+    note_launch(2 * kHelmChunk);
   }
   note_launch();
   k_helm_out<<<blocks_for(c->nelx, kHelmThreads, 4 * c->sm_count), kHelmThreads, 0,

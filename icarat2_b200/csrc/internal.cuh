@@ -319,9 +319,8 @@ struct HelmState
 {
   double radius = 0.0;
   double ke[64] = {}, nj[8] = {}, ns[8] = {};
-  double *d_coef = nullptr;
-  double *d_invd = nullptr, *d_F = nullptr, *d_val = nullptr, *d_r = nullptr,
-         *d_z = nullptr, *d_p = nullptr, *d_Ap = nullptr, *d_partials = nullptr;
+  double *d_val = nullptr, *d_r = nullptr, *d_p[2] = {}, *d_Ap = nullptr,
+         *d_partials = nullptr;
   CgScalars *d_cg = nullptr;
   cudaGraphExec_t exec = nullptr; // kHelmChunk iterations
   double *d_oc = nullptr;         // 3 nelx: work of the OC volume functor

@@ -336,7 +336,7 @@ int oc_update_helm_dev(icarat_ctx *c, double *x, const double *dfdx, double g,
                        const icarat_oc_opts *o, int *steps, double *fil, double *thr,
                        const double *vol)
 {
-  IREQUIRE(c->helm.d_coef != nullptr, ICARAT_ERR_STATE,
+  IREQUIRE(c->helm.ready, ICARAT_ERR_STATE,
            "the Helmholtz OC volume functor needs the Helmholtz filter set up");
   IREQUIRE(o->maxiter >= 0 && o->lambda_max + o->lambda_min > 0, ICARAT_ERR_ARG,
            "bad OC parameters");
