@@ -784,7 +784,8 @@ static void batch_mg_tables(icarat_batch *B, int L, int tile)
       V.b = G.b32;
     }
     M.W = c->coarse.W[c->coarse.cur];
-    M.WT = c->coarse.work[c->coarse.cur];
+    M.WT = c->coarse.U[c->coarse.cur];
+    M.rows = c->coarse.tree.rows;
     M.map = c->coarse.map;
     M.cmap = c->coarse.map + M.nc;
     M.v = B->d_y + yoff;

@@ -132,12 +132,13 @@ struct BmLevel
 };
 
 // the multigrid hierarchy of one design: levels, the coarsest level's dense
-// solve x = W^T (W b) (W = L^-1 of the coarse Cholesky factor, FP64, row
-// major, and its transpose), and the Chebyshev coefficients of its smoother
+// solve x = W^T (W b) (W = L^-1 of the coarse Cholesky factor, FP64, and its
+// transpose, by the rows that hold entries), and the Chebyshev coefficients of its smoother
 struct BmDesign
 {
   BmLevel lv[kBmMaxLevels];
   const double *W, *WT;
+  CoarseRows rows;
   const int *map;  // coarse unknown -> index of the coarsest level's node vectors
   const int *cmap; // node-major index 3 n + q of the coarsest level -> unknown (-1: fixed)
   double *v;       // the coarsest right-hand side gathered to the unknowns

@@ -1,225 +1,64 @@
-// Dense FP64 linear algebra for the coarsest multigrid level, on the FP64
-// tensor cores (mma.sync m8n8k4 f64, the DMMA path of sm_100a).
+// Direct solver of the coarsest multigrid level in FP64.
 //
 // The coarsest operator A (n x n SPD, n = free DOFs of the coarsest grid)
 // changes with every design, so each design computes W = L^-1 of its
 // Cholesky factor A = L L^T, and every V-cycle solves A x = b as
 // x = W^T (W b) with two triangular matrix-vector products.
-//   1. right-looking blocked Cholesky, block 64: per block k the diagonal
-//      block is factored and inverted in registers (k_potrf64, which also
-//      stores W_kk = L_kk^-1), the panel becomes L_ik = A_ik W_kk^T and the
-//      trailing matrix takes A -= L_ik L_jk^T (lower tiles), both as GEMMs
-//      limited to the matrix's band (the caller orders the unknowns so that
-//      the band is narrow);
-//   2. W by triangular inversion in doubling steps: with L = [L11 0; L21 L22],
-//      W21 = -W22 (L21 W11), two batched GEMMs per block size over the band
-//      of L21.
-// Matrices are row-major with leading dimension n.
-#include <type_traits>
+//
+// Order: nested dissection by node planes across the longest axis.  A node
+// couples to the planes either side only, so a plane separates what lies
+// left and right of it; the planes are split D times by middle planes, and the
+// tree of 2^D leaves and 2^D - 1 separators is numbered in postorder.  Row r
+// of W is then zero outside its node's subtree (one contiguous range), and
+// nodes of one height do not depend on one another.  At 17 x 9 x 9 nodes
+// (3,888 unknowns, D = 3) W holds 23 MB instead of the 60 MB of the plane
+// order's dense triangle, so W and W^T stay in L2 between V-cycles, and the
+// chain of 64-column steps is 20 instead of 61 long: the set-up takes 1.07 ms
+// (3.58 before), the two products of a V-cycle 20 us (43).  At 9 x 5 x 5
+// (600 unknowns, D = 2, 7 steps instead of 10) the set-up takes 0.28 ms (0.60).
+//
+// Factorization, heights from the leaves up, all nodes of a height together:
+// the matrix [A | I] is eliminated 64 columns at a time.  A node's panel
+// holds its columns for its own rows and for the rows of the (at most two)
+// separators its subtree touches.  Per step
+//   scaling (k_coarse_scale): D = W_kk^-1 .. the 64 x 64 diagonal block's
+//     inverse factor W_kk, then L_ik = A_ik W_kk^T down the panel and
+//     E_k = W_kk E_k along the rows of the identity side, which is row block
+//     k of W, done (stored with its transpose);
+//   update (k_coarse_update): A_ij -= L_ik L_jk^T in the panel and in the
+//     separators' own panels, E_i -= L_ik E_k for every later row i.
+// Each tile is one 64 x 64 x 64 product on the FP64 units: mma.sync m8n8k4 f64
+// takes 17 us for one on a whole SM here, scalar FMAs 2.1.  A separator receives from the
+// subtree on each of its sides: the right one adds into an accumulator of its
+// own (no two tiles of a launch share a target) that k_coarse_add joins.
+#include <algorithm>
+#include <cstring>
 
+#include "coarse.cuh"
 #include "internal.cuh"
 
 namespace icarat_b200
 {
 
-__device__ __forceinline__ void dmma884(double (&d)[2], double a, double b)
+namespace
 {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, "
-               "{%0,%1};\n"
-               : "+d"(d[0]), "+d"(d[1])
-               : "d"(a), "d"(b));
-}
+constexpr int kB = 64;  // block size
+constexpr int kLd = 66; // row of a staged tile: 4 banks apart, so that 16-byte reads of 16 rows
+                        // (two steps of k) take two passes over the banks, the fewest
+constexpr int kTile = kB * kLd;
+constexpr size_t kScaleSmem = 3 * kTile * sizeof(double);
+constexpr size_t kUpdateSmem = 2 * kTile * sizeof(double);
+constexpr int kLongRow = 1024; // rows of W longer than this take a block of their own
 
-// C(i,j) = alpha sum_k op(A)(i,k) op(B)(k,j) + beta C(i,j) for i < M, j < N.
-// op(A)(i,k) = ta ? A[k lda + i] : A[i lda + k]; op(B)(k,j) = tb ? B[j ldb + k]
-// : B[k ldb + j].  lower != 0: only tiles / elements with j <= i.
-struct GemmArgs
-{
-  int M, N, K;
-  double alpha, beta;
-  const double *A;
-  long lda;
-  int ta;
-  const double *B;
-  long ldb;
-  int tb;
-  double *C;
-  long ldc;
-  int lower;
-  int a_lower; // op(A)(i,k) = 0 for k > i: K ends at the tile's last row
-  int b_lower; // op(B)(k,j) = 0 for k < j: K starts at the tile's first column
-  // batch (grid z): product z uses A + z za, B + z zb, C + z zc; with
-  // rows0 > 0 it has at most rows0 - z rows_step rows (and, with k_clip, at
-  // most that many terms)
-  long za, zb, zc;
-  int rows0, rows_step, k_clip;
-};
-
-// Element t of a 64 x 16 A chunk / 16 x 64 B chunk, ordered so that the
-// stored (contiguous) axis runs across consecutive threads.
-__device__ __forceinline__ void gemm_a_idx(int ta, int t, int &r, int &c)
-{
-  if(ta)
-  {
-    c = t >> 6;
-    r = t & 63;
-  }
-  else
-  {
-    r = t >> 4;
-    c = t & 15;
-  }
-}
-__device__ __forceinline__ void gemm_b_idx(int tb, int t, int &kr, int &jc)
-{
-  if(tb)
-  {
-    jc = t >> 4;
-    kr = t & 15;
-  }
-  else
-  {
-    kr = t >> 6;
-    jc = t & 63;
-  }
-}
-
-// 64 x 64 tile per CTA, 4 warps of 32 x 32, K staged by 16 in shared memory;
-// the next chunk is fetched into registers while the current one is used.
-__global__ void __launch_bounds__(128) k_gemm_f64(GemmArgs g)
-{
-  chain_wait();
-  const int tm = blockIdx.y, tn = blockIdx.x;
-  if(g.lower && tn > tm)
-    return;
-  if(blockIdx.z > 0)
-  {
-    g.A += blockIdx.z * g.za;
-    g.B += blockIdx.z * g.zb;
-    g.C += blockIdx.z * g.zc;
-  }
-  if(g.rows0 > 0)
-  {
-    const int rows = g.rows0 - (int)blockIdx.z * g.rows_step;
-    g.M = min(g.M, rows);
-    if(g.k_clip)
-      g.K = min(g.K, rows);
-  }
-  if(tm * 64 >= g.M)
-    return;
-  __shared__ double As[64][16 + 2];
-  __shared__ double Bs[16][64 + 2];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int wm = warp >> 1, wn = warp & 1;
-  double acc[4][4][2];
-#pragma unroll
-  for(int a = 0; a < 4; a++)
-#pragma unroll
-    for(int b = 0; b < 4; b++)
-      acc[a][b][0] = acc[a][b][1] = 0.0;
-  const int i0 = tm * 64, j0 = tn * 64;
-  const int kb = g.b_lower ? (j0 & ~15) : 0;
-  const int ke = g.a_lower ? min(g.K, i0 + 64) : g.K;
-  double ra[8], rb[8];
-  auto fetch = [&](int k0)
-  {
-#pragma unroll
-    for(int u = 0; u < 8; u++)
-    {
-      const int t = threadIdx.x + 128 * u;
-      int r, c, kr, jc;
-      gemm_a_idx(g.ta, t, r, c);
-      gemm_b_idx(g.tb, t, kr, jc);
-      const int gi = i0 + r, gk = k0 + c;
-      ra[u] = (gi < g.M && gk < g.K)
-                  ? (g.ta ? g.A[(long)gk * g.lda + gi] : g.A[(long)gi * g.lda + gk])
-                  : 0.0;
-      const int bk = k0 + kr, bj = j0 + jc;
-      rb[u] = (bk < g.K && bj < g.N)
-                  ? (g.tb ? g.B[(long)bj * g.ldb + bk] : g.B[(long)bk * g.ldb + bj])
-                  : 0.0;
-    }
-  };
-  if(kb < ke)
-    fetch(kb);
-  for(int k0 = kb; k0 < ke; k0 += 16)
-  {
-#pragma unroll
-    for(int u = 0; u < 8; u++)
-    {
-      const int t = threadIdx.x + 128 * u;
-      int r, c, kr, jc;
-      gemm_a_idx(g.ta, t, r, c);
-      gemm_b_idx(g.tb, t, kr, jc);
-      As[r][c] = ra[u];
-      Bs[kr][jc] = rb[u];
-    }
-    __syncthreads();
-    if(k0 + 16 < ke)
-      fetch(k0 + 16);
-#pragma unroll
-    for(int kk = 0; kk < 16; kk += 4)
-    {
-      double a[4], b[4];
-#pragma unroll
-      for(int mt = 0; mt < 4; mt++)
-        a[mt] = As[wm * 32 + mt * 8 + (lane >> 2)][kk + (lane & 3)];
-#pragma unroll
-      for(int nt = 0; nt < 4; nt++)
-        b[nt] = Bs[kk + (lane & 3)][wn * 32 + nt * 8 + (lane >> 2)];
-#pragma unroll
-      for(int mt = 0; mt < 4; mt++)
-#pragma unroll
-        for(int nt = 0; nt < 4; nt++)
-          dmma884(acc[mt][nt], a[mt], b[nt]);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for(int mt = 0; mt < 4; mt++)
-#pragma unroll
-    for(int nt = 0; nt < 4; nt++)
-#pragma unroll
-      for(int q = 0; q < 2; q++)
-      {
-        const int i = i0 + wm * 32 + mt * 8 + (lane >> 2);
-        const int j = j0 + wn * 32 + nt * 8 + 2 * (lane & 3) + q;
-        if(i < g.M && j < g.N && (!g.lower || j <= i))
-        {
-          double *c = g.C + (long)i * g.ldc + j;
-          const double v = g.alpha * acc[mt][nt][q];
-          *c = (g.beta != 0.0) ? v + g.beta * *c : v;
-        }
-      }
-}
-
-// Factor the 64 x 64 diagonal block at k0, write L_kk into A (zeros above the
-// diagonal) and W_kk = L_kk^-1 into W.  Rows / columns past n are padded with
-// the identity.
-//
-// The block lives in registers: thread (ty, tx) of a 16 x 16 grid holds rows
-// 4ty..4ty+3 and columns 4tx..4tx+3 of the block (a) and of the inverse being
-// built (e).  Elimination is right-looking in the unscaled form: step j
-// subtracts m_rj = a_rj / a_jj times row j from every row r > j, both in a
-// (a_rc -= m_rj a_cj, lower part) and in e, which starts as the identity
-// (e_rc -= m_rj e_jc, c <= j), so that e ends as the inverse of the unit
-// lower factor; the square roots of the pivots scale both at the end
-// (L_rc = a_rc / sqrt(a_cc), W_rc = e_rc / sqrt(a_rr)).  Column j of a, row
-// j of e and 1 / a_jj are final after step j - 1: their owners publish them
-// to shared memory at the end of that step (the pivot's owner updates it
-// and starts its reciprocal before its other updates), double-buffered, so
-// each step needs a single barrier.
-constexpr int kPotrfSmem = (4 * 64 + 2 * 64 + 2) * sizeof(double);
-
-// 1 / x and 1 / sqrt(x) for x > 0 by Newton's method from an FP32 seed
-// (y <- y (2 - x y), and y <- y (3/2 - x y^2 / 2)): each step doubles the
-// correct digits, so two steps take the seed's ~2^-22 past double precision
-// (x must lie in the normal FP32 range).  Inline FMAs only: an out-of-line
-// divide or square root inside the loops below would save the
-// register-resident block to the stack at every call.
+// 1 / x and 1 / sqrt(x) for x > 0 by Newton's method from the hardware's
+// approximations (y <- y (2 - x y), and y <- y (3/2 - x y^2 / 2)): each step
+// doubles the correct digits, so two steps take a seed of ~2^-20 past double
+// precision.  Inline FMAs only: an out-of-line divide or square root would save
+// the register-resident rows to the stack.
 __device__ __forceinline__ double recip_newton(double x)
 {
-  double y = (double)__fdividef(1.0f, (float)x);
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
 #pragma unroll
   for(int it = 0; it < 2; it++)
     y = y * fma(-x, y, 2.0);
@@ -228,318 +67,646 @@ __device__ __forceinline__ double recip_newton(double x)
 
 __device__ __forceinline__ double rsqrt_newton(double x)
 {
-  double y = (double)rsqrtf((float)x);
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
 #pragma unroll
   for(int it = 0; it < 2; it++)
     y = y * fma(-0.5 * x, y * y, 1.5);
   return y;
 }
 
-__global__ void __launch_bounds__(256) k_potrf64(double *A, double *W, int n, int k0)
+// Inverse of the 16 x 16 Cholesky factor of the block at S (lower part) into W
+// (zeros above its diagonal), by one warp: lanes 0-15 hold the rows of the
+// block (symmetric), lanes 16-31 the rows of the identity side.  Step j
+// subtracts m_r = a_rj / a_jj times row j from the rows r > j of both sides;
+// the pivots' square roots scale the inverse at the end.  What lies left of
+// the pivot on the block's side is not used again and may hold anything.
+__device__ __forceinline__ void factor16(const double *S, double *W, int lane)
 {
-  chain_wait();
-  extern __shared__ double potrf_smem[];
-  double(*colbuf)[64] = reinterpret_cast<double(*)[64]>(potrf_smem); // [2][64] column j of a
-  double(*rowbuf)[64] = colbuf + 2;                                  // [2][64] row j of e
-  double *isq = potrf_smem + 4 * 64;                                  // 1 / sqrt(pivot)
-  double *sq = isq + 64;                                              // sqrt(pivot)
-  double *invbuf = sq + 64;                                           // [2] 1 / a_jj
-  const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
-  const int m = min(64, n - k0);
-  double a[4][4], e[4][4];
+  const int r = lane & 15;
+  const bool block = lane < 16;
+  double x[16], piv = 1.0;
 #pragma unroll
-  for(int i = 0; i < 4; i++)
+  for(int c = 0; c < 16; c++)
+    x[c] = block ? S[max(r, c) * kLd + min(r, c)] : (r == c ? 1.0 : 0.0);
+  double p = __shfl_sync(0xffffffffu, x[0], 0);
+  double inv = recip_newton(p);
 #pragma unroll
-    for(int q = 0; q < 4; q++)
-    {
-      const int r = 4 * ty + i, c = 4 * tx + q;
-      a[i][q] = (r < m && c < m) ? A[(long)(k0 + r) * n + k0 + c] : (r == c ? 1.0 : 0.0);
-      e[i][q] = (r == c) ? 1.0 : 0.0;
-    }
-  if(tx == 0)
-#pragma unroll
-    for(int i = 0; i < 4; i++)
-      colbuf[0][4 * ty + i] = a[i][0];
-  if(ty == 0)
-#pragma unroll
-    for(int q = 0; q < 4; q++)
-      rowbuf[0][4 * tx + q] = e[0][q];
-  if(t == 0)
-    invbuf[0] = recip_newton(a[0][0]);
-  __syncthreads();
-  auto step = [&](auto qc, int j)
+  for(int j = 0; j < 16; j++)
   {
-    constexpr int Q = decltype(qc)::value; // j & 3
-    constexpr int Q1 = (Q + 1) & 3;        // (j + 1) & 3
-    const double *cj = colbuf[j & 1];
-    const double *ej = rowbuf[j & 1];
-    const double inv = invbuf[j & 1];
-    // multipliers zero outside the rows / columns that step j updates, so
-    // that every update below is unconditional: rows r > j of a (columns
-    // c > j; the entries above the diagonal follow the symmetric update and
-    // are never output) and of e (row j of e is zero past column j)
-    double fr[4], fc[4], er[4];
+    const double col = __shfl_sync(0xffffffffu, x[j], r);
+    const double m = r > j ? -col * inv : 0.0;
+    const double mb = block ? m : 0.0;
+    if(r == j)
+      piv = p;
+    if(j < 15) // the next pivot first: its reciprocal is the longest chain
+    {
+      x[j + 1] = fma(mb, __shfl_sync(0xffffffffu, x[j + 1], j), x[j + 1]);
+      p = __shfl_sync(0xffffffffu, x[j + 1], j + 1);
+      inv = recip_newton(p);
+    }
+#pragma unroll
+    for(int c = 0; c < 16; c++)
+      if(c != j + 1)
+      {
+        const double v = __shfl_sync(0xffffffffu, x[c], c > j ? j : 16 + j);
+        x[c] = fma(c > j ? mb : m, v, x[c]);
+      }
+  }
+  if(!block)
+  {
+    const double y = rsqrt_newton(piv);
+#pragma unroll
+    for(int c = 0; c < 16; c++)
+      W[r * kLd + c] = c <= r ? x[c] * y : 0.0;
+  }
+}
+
+// Step `C / 16` of factor64: columns [C, C + 16).
+__device__ __forceinline__ void factor64_step(int C, double *S, double *W)
+{
+  const int NB = (kB - 16 - C) / 16; // 16-row blocks below
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  double *Wd = W + C * kLd + C;
+  if(threadIdx.x < 32)
+    factor16(S + C * kLd + C, Wd, threadIdx.x);
+  __syncthreads();
+  // 48 vectors x of 16: the rows of S below (L_i = S_i W_d^T) and the columns of
+  // W left of the block (E = W_d E); W_d x in place
+  double out[3] = {0.0, 0.0, 0.0};
+#pragma unroll 4
+  for(int k = 0; k < 16; k++)
+  {
+    const double w = Wd[tx * kLd + k];
+#pragma unroll
+    for(int u = 0; u < 3; u++)
+      out[u] = fma(w, u < NB ? S[(C + 16 + 16 * u + ty) * kLd + C + k]
+                             : W[(C + k) * kLd + 16 * (u - NB) + ty], out[u]);
+  }
+  __syncthreads();
+#pragma unroll
+  for(int u = 0; u < 3; u++)
+    if(u < NB)
+      S[(C + 16 + 16 * u + ty) * kLd + C + tx] = out[u];
+    else
+      W[(C + tx) * kLd + 16 * (u - NB) + ty] = out[u];
+  __syncthreads();
+  if(NB == 0)
+    return;
+  // the rows below, 64 columns in all: S_ij -= L_i L_j^T (j <= i), E_i -= L_i E
+  double acc[3][4] = {};
+#pragma unroll 4
+  for(int k = 0; k < 16; k++)
+  {
+    double b[4];
+#pragma unroll
+    for(int q = 0; q < 4; q++)
+      b[q] = q < NB ? S[(C + 16 + 16 * q + tx) * kLd + C + k]
+                    : W[(C + k) * kLd + 16 * (q - NB) + tx];
+#pragma unroll
+    for(int i = 0; i < 3; i++)
+      if(i < NB)
+      {
+        const double a = S[(C + 16 + 16 * i + ty) * kLd + C + k];
+#pragma unroll
+        for(int q = 0; q < 4; q++)
+          acc[i][q] = fma(a, b[q], acc[i][q]);
+      }
+  }
+#pragma unroll
+  for(int i = 0; i < 3; i++)
+#pragma unroll
+    for(int q = 0; q < 4; q++)
+    {
+      const int row = C + 16 + 16 * i + ty;
+      if(i < NB && q < NB && q <= i)
+        S[row * kLd + C + 16 + 16 * q + tx] -= acc[i][q];
+      else if(i < NB && q >= NB)
+        W[row * kLd + 16 * (q - NB) + tx] -= acc[i][q];
+    }
+  __syncthreads();
+}
+
+// W (64 x 64, zero on entry) = inverse Cholesky factor of the block S (lower
+// part; overwritten), 256 threads: [S | W] eliminated 16 columns at a time, as
+// the whole matrix is by 64.  16 columns are what one warp holds in registers;
+// the rest of a step is small products over all threads.
+__device__ void factor64(double *S, double *W)
+{
+#pragma unroll 1
+  for(int c = 0; c < kB; c += 16)
+    factor64_step(c, S, W);
+}
+
+// stage rows x cols (<= 64 x 64, row length ld) as a 64 x 64 tile, zeros past
+// the end
+__device__ __forceinline__ void stage_tile(double *T, const double *g, int ld, int rows, int cols)
+{
+  const int c = threadIdx.x & 63;
+  double v[16];
+#pragma unroll
+  for(int u = 0; u < 16; u++)
+  {
+    const int r = (threadIdx.x >> 6) + 4 * u;
+    v[u] = (r < rows && c < cols) ? g[(long)r * ld + c] : 0.0;
+  }
+#pragma unroll
+  for(int u = 0; u < 16; u++)
+    T[((threadIdx.x >> 6) + 4 * u) * kLd + c] = v[u];
+}
+
+// 64 x 64 product of two staged tiles, A B (BT false) or A B^T: thread
+// (ty, tx) of 16 x 16 has rows ty + 16 i and columns tx + 16 q, two steps of k
+// at a time.  A warp reads 12 passes of shared memory for 64 FMA cycles.
+template <bool BT>
+__device__ __forceinline__ void tile_product(double (&acc)[4][4], const double *A,
+                                             const double *B)
+{
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+#pragma unroll 4
+  for(int k = 0; k < kB; k += 2)
+  {
+    double2 a[4], b[4];
 #pragma unroll
     for(int i = 0; i < 4; i++)
-    {
-      fr[i] = (4 * ty + i > j) ? cj[4 * ty + i] * inv : 0.0; // m_rj
-      fc[i] = (4 * tx + i > j) ? cj[4 * tx + i] : 0.0;       // a_cj
-      er[i] = ej[4 * tx + i];                                // e_jc
-    }
-    const int j1 = j + 1;
-    // the next pivot's reciprocal, computed by every thread without a branch
-    // (only the pivot's owner publishes it) so that its latency hides behind
-    // the independent updates below
-    const bool pivot_owner = (tx == (j1 >> 2)) && (ty == (j1 >> 2)) && j1 < 64;
-    const double inv_next = recip_newton(fma(-fr[Q1], fc[Q1], a[Q1][Q1]));
+      a[i] = *reinterpret_cast<const double2 *>(A + (ty + 16 * i) * kLd + k);
+#pragma unroll
+    for(int q = 0; q < 4; q++)
+      b[q] = BT ? *reinterpret_cast<const double2 *>(B + (tx + 16 * q) * kLd + k)
+                : make_double2(B[k * kLd + tx + 16 * q], B[(k + 1) * kLd + tx + 16 * q]);
 #pragma unroll
     for(int i = 0; i < 4; i++)
 #pragma unroll
       for(int q = 0; q < 4; q++)
-      {
-        a[i][q] = fma(-fr[i], fc[q], a[i][q]);
-        e[i][q] = fma(-fr[i], er[q], e[i][q]);
-      }
-    if(j1 < 64)
-    {
-      if(tx == (j1 >> 2))
-#pragma unroll
-        for(int i = 0; i < 4; i++)
-          colbuf[j1 & 1][4 * ty + i] = a[i][Q1];
-      if(ty == (j1 >> 2))
-#pragma unroll
-        for(int q = 0; q < 4; q++)
-          rowbuf[j1 & 1][4 * tx + q] = e[Q1][q];
-      if(pivot_owner)
-        invbuf[j1 & 1] = inv_next;
-    }
-    __syncthreads();
-  };
-  for(int j = 0; j < 64; j += 4)
-  {
-    step(std::integral_constant<int, 0>{}, j);
-    step(std::integral_constant<int, 1>{}, j + 1);
-    step(std::integral_constant<int, 2>{}, j + 2);
-    step(std::integral_constant<int, 3>{}, j + 3);
+        acc[i][q] = fma(a[i].y, b[q].y, fma(a[i].x, b[q].x, acc[i][q]));
   }
-  // ---- scaling by the square roots of the pivots
-  if(tx == ty)
-#pragma unroll
-    for(int i = 0; i < 4; i++)
-    {
-      const double y = rsqrt_newton(a[i][i]);
-      isq[4 * ty + i] = y;
-      sq[4 * ty + i] = a[i][i] * y;
-    }
-  __syncthreads();
+}
+
+// f(row, column, value) for each element of a thread's share
+template <typename F> __device__ __forceinline__ void tile_each(const double (&acc)[4][4], F f)
+{
 #pragma unroll
   for(int i = 0; i < 4; i++)
 #pragma unroll
     for(int q = 0; q < 4; q++)
+      f((int)(threadIdx.x >> 4) + 16 * i, (int)(threadIdx.x & 15) + 16 * q, acc[i][q]);
+}
+
+// the 64 x kw block T of row block k0 of node X's part of W, columns from
+// global unknown c: into W, and transposed into W^T (rows: the columns here)
+__device__ __forceinline__ void store_inverse(const CoarseNode &X, const CoarseNode *nodes,
+                                              const int *node_of, int k0, int kw, int c, int cols,
+                                              const double *T, double *W, double *U)
+{
+  const int x = threadIdx.x & 63;
+  for(int y = threadIdx.x >> 6; y < kw; y += 4)
+    if(x < cols)
+      W[X.W + (long)(k0 + y) * X.S + (c - X.lo) + x] = T[y * kLd + x];
+  for(int y = threadIdx.x >> 6; y < cols; y += 4)
+    if(x < kw)
     {
-      const int r = 4 * ty + i, c = 4 * tx + q;
-      if(r < m && c < m)
-      {
-        A[(long)(k0 + r) * n + k0 + c] = r > c ? a[i][q] * isq[c] : (r == c ? sq[c] : 0.0);
-        W[(long)(k0 + r) * n + k0 + c] = (c <= r) ? e[i][q] * isq[r] : 0.0;
-      }
+      const CoarseNode &Y = nodes[node_of[c + y]];
+      U[Y.U + (long)(c + y - Y.s) * Y.C + (Y.C - X.C) + k0 + x] = T[x * kLd + y];
     }
 }
+} // namespace
 
-// The row a warp takes in the triangular products: even warps the short
-// rows from the top, odd warps the long ones from the bottom, so every pair
-// of neighbouring warps reads n + 1 coefficients and the blocks stay balanced.
-__device__ __forceinline__ int trmv_row(int warp, int n)
-{
-  return (warp & 1) ? n - 1 - (warp >> 1) : (warp >> 1);
-}
-
-// sum over q in [q0, q1) of row[q] v[q] by one warp: eight independent
-// partial sums per lane (eight coefficient loads in flight), summed in a
-// fixed order, then across the warp
-__device__ __forceinline__ double warp_row_dot(const double *__restrict__ row,
-                                               const double *__restrict__ v, int q0, int q1,
-                                               int lane)
-{
-  double s[8];
-#pragma unroll
-  for(int u = 0; u < 8; u++)
-    s[u] = 0.0;
-  int q = q0 + lane;
-  for(; q + 224 < q1; q += 256)
-#pragma unroll
-    for(int u = 0; u < 8; u++)
-      s[u] = fma(row[q + 32 * u], v[q + 32 * u], s[u]);
-  for(; q < q1; q += 32)
-    s[0] = fma(row[q], v[q], s[0]);
-  double a = ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
-  for(int o = 16; o > 0; o >>= 1)
-    a += __shfl_down_sync(0xffffffffu, a, o);
-  return a;
-}
-
-// t = W v (W lower triangular), one warp per row
-__global__ void k_trmv_lower(int n, const double *__restrict__ W,
-                             const double *__restrict__ v, double *__restrict__ t,
-                             const int *__restrict__ halt)
+// panels of the nodes of one height += their second accumulators
+__global__ void k_coarse_add(const CoarseNode *__restrict__ nodes, int height,
+                             double *__restrict__ P)
 {
   chain_wait();
-  if(halted(halt))
+  const CoarseNode X = nodes[blockIdx.y];
+  if(X.height != height)
     return;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  const int nw = (gridDim.x * blockDim.x) >> 5;
-  for(int w = warp; w < n; w += nw)
-  {
-    const int r = trmv_row(w, n);
-    const double s = warp_row_dot(W + (long)r * n, v, 0, r + 1, lane);
-    if(lane == 0)
-      t[r] = s;
-  }
+  const int total = X.m * X.m;
+  for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x)
+    P[X.P + i] += P[X.Q + i];
 }
 
-// WT = W^T (W lower -> WT upper), 32 x 32 tiles through shared memory
-__global__ void k_transpose_lower(int n, const double *__restrict__ W,
-                                  double *__restrict__ WT)
+// One step's scaling: every block factors its node's diagonal block itself,
+// which saves a launch and a round trip through memory.  The pivots' serial
+// chain bounds it (about 24 us of latency; the product after it takes 3).
+__global__ void __launch_bounds__(256)
+    k_coarse_scale(const CoarseNode *__restrict__ nodes, const int *__restrict__ node_of,
+                   const CoarseScaleTile *__restrict__ tiles, double *P, double *W, double *U)
 {
   chain_wait();
-  __shared__ double tile[32][33];
-  const int bi = blockIdx.y * 32, bj = blockIdx.x * 32; // source tile rows / cols
-  if(bj > bi + 31)
-    return; // entirely above the diagonal: zero in W and in WT below
-  for(int r = threadIdx.y; r < 32; r += blockDim.y)
-  {
-    const int i = bi + r, j = bj + threadIdx.x;
-    tile[r][threadIdx.x] = (i < n && j < n && j <= i) ? W[(long)i * n + j] : 0.0;
-  }
+  extern __shared__ double coarse_smem[];
+  double *S = coarse_smem, *Wk = S + kTile, *T = Wk + kTile;
+  const CoarseScaleTile tile = tiles[blockIdx.x];
+  const CoarseNode X = nodes[tile.node];
+  const int k0 = tile.k0, kw = min(kB, X.m - k0);
+  stage_tile(S, P + X.P + (long)k0 * X.m + k0, X.m, kw, kw);
+  for(int i = threadIdx.x; i < kTile; i += 256)
+    Wk[i] = 0.0;
+  const int rows = min(kB, X.m + X.ml + X.mr - tile.first);       // of a panel tile
+  const int cols = min(kB, X.s + k0 - X.lo - tile.first);         // of an inverse tile
+  double *panel = P + X.P + (long)tile.first * X.m + k0;
+  if(tile.kind == kTilePanel)
+    stage_tile(T, panel, X.m, rows, kw);
+  else if(tile.kind == kTileInverse)
+    stage_tile(T, W + X.W + (long)k0 * X.S + tile.first, X.S, kw, cols);
   __syncthreads();
-  for(int r = threadIdx.y; r < 32; r += blockDim.y)
+  if((int)threadIdx.x >= kw && threadIdx.x < kB) // identity past the last column
+    S[threadIdx.x * kLd + threadIdx.x] = 1.0;
+  __syncthreads();
+  factor64(S, Wk);
+  if(tile.kind == kTileDiag)
   {
-    const int i = bj + r, j = bi + threadIdx.x; // WT[i][j] = W[j][i]
-    if(i < n && j < n)
-      WT[(long)i * n + j] = tile[threadIdx.x][r];
+    store_inverse(X, nodes, node_of, k0, kw, X.s + k0, kw, Wk, W, U);
+    return;
   }
+  double acc[4][4] = {};
+  if(tile.kind == kTilePanel)
+  {
+    tile_product<true>(acc, T, Wk);
+    tile_each(acc,
+              [&](int i, int j, double v)
+              {
+                if(i < rows && j < kw)
+                  panel[(long)i * X.m + j] = v;
+              });
+    return;
+  }
+  tile_product<false>(acc, Wk, T);
+  tile_each(acc, [&](int i, int j, double v) { S[i * kLd + j] = v; });
+  __syncthreads();
+  store_inverse(X, nodes, node_of, k0, kw, X.lo + tile.first, cols, S, W, U);
 }
 
-// x[rowmap] = WT t (WT upper), one warp per row; rows are contiguous
-template <typename T>
-__global__ void k_trmv_upper(int n, const double *__restrict__ WT,
-                             const double *__restrict__ t, const int *__restrict__ rowmap,
-                             T *__restrict__ x, const int *__restrict__ halt)
+// One step's updates.
+__global__ void __launch_bounds__(256)
+    k_coarse_update(const CoarseUpdateTile *__restrict__ tiles, double *P, double *W)
+{
+  chain_wait();
+  extern __shared__ double coarse_smem[];
+  double *A = coarse_smem, *B = A + kTile;
+  const CoarseUpdateTile g = tiles[blockIdx.x];
+  stage_tile(A, P + g.a, g.lda, g.M, g.K);
+  if(g.from_w)
+    stage_tile(B, W + g.b, g.ldb, g.K, g.N);
+  else
+    stage_tile(B, P + g.b, g.ldb, g.N, g.K);
+  __syncthreads();
+  double acc[4][4] = {};
+  if(g.from_w)
+    tile_product<false>(acc, A, B);
+  else
+    tile_product<true>(acc, A, B);
+  double *C = (g.to_w ? W : P) + g.c;
+  tile_each(acc,
+            [&](int i, int j, double v)
+            {
+              if(i < g.M && j < g.N && (!g.lower || j <= i))
+                C[(long)i * g.ldc + j] -= v;
+            });
+}
+
+// t = W v, blocks of 8 warps: a row each, or one long row together
+__global__ void __launch_bounds__(256)
+    k_coarse_lower(int n, CoarseRows R, const int *__restrict__ items,
+                   const double *__restrict__ W, const double *v, double *__restrict__ t,
+                   const int *__restrict__ halt)
 {
   chain_wait();
   if(halted(halt))
     return;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  const int nw = (gridDim.x * blockDim.x) >> 5;
-  for(int w = warp; w < n; w += nw)
+  __shared__ double part[8];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int item = items[blockIdx.x];
+  if(item >= 0) // up to the next item's first row
   {
-    const int r = trmv_row(w, n);
-    const double s = warp_row_dot(WT + (long)r * n, t, r, n, lane);
-    if(lane == 0)
-      x[rowmap[r]] = (T)s;
-  }
-}
-
-
-static void gemm(cudaStream_t st, int M, int N, int K, double alpha, const double *A,
-                 long lda, int ta, const double *B, long ldb, int tb, double beta,
-                 double *C, long ldc, int lower, int a_lower = 0, int b_lower = 0)
-{
-  if(M <= 0 || N <= 0 || K <= 0)
-    return;
-  GemmArgs g{M,   N,  K,  alpha, beta, A,     lda,    ta,
-             B,   ldb, tb, C,    ldc,  lower, a_lower, b_lower, 0, 0, 0, 0, 0, 0};
-  dim3 grid((N + 63) / 64, (M + 63) / 64);
-  note_launch();
-  launch_chained(k_gemm_f64, grid, 128, 0, st, g);
-}
-
-// W = L^-1 from the diagonal blocks W_kk by doubling: at block size s every
-// pair of neighbouring inverted blocks [o, o + s), [o + s, o + 2s) (o a
-// multiple of 2s; the second may be short or absent) becomes one, with
-// L = [L11 0; L21 L22], W21 = -W22 L21 W11.  All pairs of one size go in one
-// batched launch per product.  L has lower bandwidth bw, so L21 is zero
-// outside its top-right min(bw, s2) x min(bw, s) corner:
-//   T = L21[0:r, s-k:s] W11[s-k:s, :]   (r x s; the other rows are zero)
-//   W21 = -W22[:, 0:r] T                (columns past each row of the lower
-//                                        triangular W22 skipped)
-// T holds one r x s slab per pair.
-static void trinv_banded(cudaStream_t st, const double *L, double *W, double *T, int n,
-                         int bw)
-{
-  for(int s = 64; s < n; s *= 2)
-  {
-    const int pairs = (n - s + 2 * s - 1) / (2 * s); // pairs whose second block exists
-    const int k = std::min(bw, s);
-    const int r = std::min(bw, s);
-    const long step = 2L * s * n + 2L * s;           // from pair z to pair z + 1
-    const long tslab = (long)r * s;
-    note_launch(2);
-    // T_z = L21 W11 (rows clipped to the short second block of the last pair)
-    GemmArgs g1{r, s, k, 1.0, 0.0, L + (long)s * n + s - k, n, 0, W + (long)(s - k) * n, n, 0,
-                T, s, 0, 0, 0, step, step, tslab, n - s, 2 * s, 0};
-    launch_chained(k_gemm_f64, dim3((s + 63) / 64, (r + 63) / 64, pairs), 128, 0, st, g1);
-    // W21_z = -W22 T_z (K clipped like the rows: W22 has s2 columns)
-    GemmArgs g2{s, s, r, -1.0, 0.0, W + (long)s * n + s, n, 0, T, s, 0, W + (long)s * n, n,
-                0, 1, 0, step, tslab, step, n - s, 2 * s, 1};
-    launch_chained(k_gemm_f64, dim3((s + 63) / 64, (s + 63) / 64, pairs), 128, 0, st, g2);
-  }
-}
-
-// A (lower part, lower bandwidth bw) -> L in place; W <- L^-1 (upper part
-// zero); T: n x n scratch, which ends up holding W^T (upper part; rows
-// contiguous for the transposed product of every solve).  The Cholesky
-// factor keeps the band, so block column k updates only the bw rows below
-// its diagonal block; W = L^-1 is dense.
-void dense_spd_inverse_factor(cudaStream_t st, double *A, double *W, double *T, int n, int bw)
-{
-  ICK(cudaFuncSetAttribute(k_potrf64, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           kPotrfSmem));
-  ICK(cudaMemsetAsync(W, 0, sizeof(double) * (size_t)n * n, st));
-  bw = std::max(1, std::min(bw, n));
-  const int nb = (n + 63) / 64;
-  for(int k = 0; k < nb; k++)
-  {
-    const int k0 = k * 64;
-    note_launch();
-    launch_chained(k_potrf64, 1, 256, kPotrfSmem, st, A, W, n, k0);
-    const int rest = std::min(n - k0 - 64, bw);
-    if(rest > 0)
+    const int next = items[blockIdx.x + 1], r = item + warp;
+    if(r < (next >= 0 ? next : -next - 1))
     {
-      double *panel = A + (long)(k0 + 64) * n + k0;
-      // L_ik = A_ik W_kk^T (in place: each CTA reads its own rows first)
-      gemm(st, rest, 64, 64, 1.0, panel, n, 0, W + (long)k0 * n + k0, n, 1, 0.0, panel, n,
-           0);
-      // A22 -= L_i L_j^T on the lower tiles of the band
-      gemm(st, rest, rest, 64, -1.0, panel, n, 0, panel, n, 1, 1.0,
-           A + (long)(k0 + 64) * n + k0 + 64, n, 1);
+      const double s = coarse_warp_sum(coarse_dot(W + R.wofs[r], v, R.lo[r], r + 1, lane, 0.0));
+      if(lane == 0)
+        t[r] = s;
+    }
+    return;
+  }
+  const int r = -item - 1, lo = R.lo[r], per = ((r + 1 - lo + 7) / 8 + 31) & ~31;
+  const int j0 = lo + warp * per, j1 = min(r + 1, j0 + per);
+  const double s = coarse_warp_sum(coarse_dot(W + R.wofs[r], v, j0, j1, lane, 0.0));
+  if(lane == 0)
+    part[warp] = s;
+  __syncthreads();
+  if(threadIdx.x == 0)
+    t[r] = ((part[0] + part[1]) + (part[2] + part[3])) +
+           ((part[4] + part[5]) + (part[6] + part[7]));
+}
+
+// x[rowmap] = W^T t, one warp per row
+template <typename T>
+__global__ void __launch_bounds__(256)
+    k_coarse_upper(int n, CoarseRows R, const double *__restrict__ WT, const double *t,
+                   const int *__restrict__ rowmap, T *__restrict__ x,
+                   const int *__restrict__ halt)
+{
+  chain_wait();
+  if(halted(halt))
+    return;
+  const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if(r >= n)
+    return;
+  const double s = coarse_upper_row(R, WT, t, r, lane);
+  if(lane == 0)
+    x[rowmap[r]] = (T)s;
+}
+
+// ---------------------------------------------------------------- the tree
+namespace
+{
+struct TreeBuilder
+{
+  const std::vector<int> &pf; // first unknown of each plane
+  std::vector<int> &order;
+  std::vector<CoarseNode> nodes;
+  std::vector<int> parent;
+
+  // planes [p0, p1), `depth` levels of separators below; returns the root
+  int build(int p0, int p1, int depth)
+  {
+    const int lo = (int)order.size();
+    int kid[2] = {-1, -1}, s0 = p0, s1 = p1;
+    if(depth > 0)
+    {
+      s0 = p0 + (p1 - p0) / 2;
+      s1 = s0 + 1;
+      kid[0] = build(p0, s0, depth - 1);
+      kid[1] = build(s1, p1, depth - 1);
+    }
+    CoarseNode X{};
+    X.s = (int)order.size();
+    for(int i = pf[s0]; i < pf[s1]; i++)
+      order.push_back(i);
+    X.m = (int)order.size() - X.s;
+    X.lo = lo;
+    X.S = X.s + X.m - lo;
+    X.left = X.right = -1;
+    X.height = depth;
+    const int id = (int)nodes.size();
+    nodes.push_back(X);
+    parent.push_back(-1);
+    if(depth > 0)
+    {
+      parent[kid[0]] = parent[kid[1]] = id;
+      border(kid[0], false, id);
+      border(kid[1], true, id);
+    }
+    return id;
+  }
+  // separator `sep` lies left (right) of the subtree of x: of x itself and of
+  // the nodes down its left (right) edge
+  void border(int x, bool left, int sep)
+  {
+    for(;;)
+    {
+      (left ? nodes[x].left : nodes[x].right) = sep;
+      if(nodes[x].height == 0)
+        return;
+      // children of x in postorder: the right one is x - 1, the left one
+      // ends before the right one's subtree
+      const int right_kid = x - 1;
+      const int left_kid = right_kid - ((2 << nodes[right_kid].height) - 1);
+      x = left ? left_kid : right_kid;
     }
   }
-  trinv_banded(st, A, W, T, n, bw);
-  note_launch();
-  launch_chained(k_transpose_lower, dim3((n + 31) / 32, (n + 31) / 32), dim3(32, 8), 0, st, n,
-                 (const double *)W, T);
+};
+
+// the tree's tables, in one device allocation
+struct TablePacker
+{
+  std::vector<char> bytes;
+  template <typename T> size_t add(const std::vector<T> &v)
+  {
+    const size_t at = (bytes.size() + 15) & ~size_t(15);
+    bytes.resize(at + v.size() * sizeof(T));
+    if(!v.empty())
+      memcpy(bytes.data() + at, v.data(), v.size() * sizeof(T));
+    return at;
+  }
+};
+} // namespace
+
+void coarse_tree_free(CoarseTree &t)
+{
+  cudaFree(t.tables);
+  t = CoarseTree{};
+}
+
+void coarse_tree_build(CoarseTree &t, const std::vector<int> &pf, std::vector<int> &order)
+{
+  const int planes = (int)pf.size() - 1;
+  t.n = pf[planes];
+  int widest = 1;
+  for(int p = 0; p < planes; p++)
+    widest = std::max(widest, pf[p + 1] - pf[p]);
+  // depth: split while every leaf keeps a plane and the chain of 64-column
+  // steps (a leaf's and one separator's per level) does not grow
+  auto steps = [&](int d)
+  {
+    const int leaf = (planes - ((1 << d) - 1) + (1 << d) - 1) >> d; // planes of the largest
+    return (leaf * widest + kB - 1) / kB + d * ((widest + kB - 1) / kB);
+  };
+  int depth = 0;
+  while(depth < kCoarseDepth && planes >= (4 << depth) - 1 && steps(depth + 1) <= steps(depth))
+    depth++;
+  order.clear();
+  TreeBuilder b{pf, order, {}, {}};
+  if(t.n > 0)
+    b.build(0, planes, depth);
+  std::vector<CoarseNode> &N = b.nodes;
+  const int nn = (int)N.size();
+  t.nnodes = nn;
+  std::vector<int2> chain((size_t)kCoarseChain * nn, make_int2(0, 0));
+  for(int i = nn - 1; i >= 0; i--) // ancestors come after their descendants
+  {
+    CoarseNode &X = N[i];
+    X.ml = X.left >= 0 ? N[X.left].m : 0;
+    X.mr = X.right >= 0 ? N[X.right].m : 0;
+    X.C = X.m + (b.parent[i] >= 0 ? N[b.parent[i]].C : 0);
+    int k = 0;
+    for(int y = i; y >= 0; y = b.parent[y])
+      chain[(size_t)kCoarseChain * i + k++] = make_int2(N[y].s, N[y].m);
+  }
+  for(CoarseNode &X : N)
+  {
+    X.P = t.nP;
+    t.nP += (long)(X.m + X.ml + X.mr) * X.m;
+    X.Q = -1;
+    if(X.height > 0)
+    {
+      X.Q = t.nP;
+      t.nP += (long)X.m * X.m;
+    }
+    X.W = t.nW;
+    t.nW += (long)X.m * X.S;
+    X.U = t.nU;
+    t.nU += (long)X.m * X.C;
+  }
+  std::vector<long> wofs(t.n), uofs(t.n);
+  std::vector<int> lo(t.n), node(t.n), items;
+  for(int i = 0; i < nn; i++)
+    for(int q = 0; q < N[i].m; q++)
+    {
+      const CoarseNode &X = N[i];
+      const int r = X.s + q;
+      wofs[r] = X.W + (long)q * X.S - X.lo;
+      uofs[r] = X.U + (long)q * X.C + q;
+      lo[r] = X.lo;
+      node[r] = i;
+    }
+  for(int r = 0; r < t.n;)
+    if(r + 1 - lo[r] > kLongRow)
+      items.push_back(-(r++) - 1);
+    else
+    {
+      items.push_back(r);
+      for(int k = 0; k < 8 && r < t.n && r + 1 - lo[r] <= kLongRow; k++)
+        r++;
+    }
+  t.nitems = (int)items.size();
+  items.push_back(t.n); // ends the last item
+  // launch tables
+  std::vector<CoarseScaleTile> scale;
+  std::vector<CoarseUpdateTile> upd;
+  auto product = [&](long a, int lda, long bo, int ldb, bool from_w, long c, int ldc, bool to_w,
+                     int M, int Nc, int K, bool lower)
+  {
+    for(int i = 0; i < M; i += kB)
+      for(int j = 0; j < Nc && (!lower || j <= i); j += kB)
+        upd.push_back({a + (long)i * lda, from_w ? bo + j : bo + (long)j * ldb,
+                       c + (long)i * ldc + j, lda, ldb, ldc, (short)std::min(kB, M - i),
+                       (short)std::min(kB, Nc - j), (short)K, (short)from_w,
+                       (short)(lower && i == j), (short)to_w});
+  };
+  // row of separator y in the panel of x
+  auto panel_row = [&](int x, int y) { return N[x].m + (y == N[x].left ? 0 : N[x].ml); };
+  for(int h = 0; h <= depth && nn > 0; h++)
+  {
+    int most = 0;
+    for(const CoarseNode &X : N)
+      if(X.height == h)
+        most = std::max(most, X.m);
+    for(int k0 = 0; k0 < most; k0 += kB)
+    {
+      CoarseStep st{};
+      st.join = k0 == 0 ? h : 0;
+      st.scale0 = (int)scale.size();
+      st.upd0 = (int)upd.size();
+      for(int x = 0; x < nn; x++)
+      {
+        const CoarseNode &X = N[x];
+        if(X.height != h || k0 >= X.m)
+          continue;
+        const int kw = std::min(kB, X.m - k0), next = k0 + kw, rows = X.m + X.ml + X.mr;
+        const int before = X.s + k0 - X.lo, done = before + kw; // columns of the inverse side
+        scale.push_back({x, k0, kTileDiag, 0});
+        for(int r = next; r < rows; r += kB)
+          scale.push_back({x, k0, kTilePanel, r});
+        for(int c = 0; c < before; c += kB)
+          scale.push_back({x, k0, kTileInverse, c});
+        auto L = [&](int row) { return X.P + (long)row * X.m + k0; };
+        // own columns: the lower triangle of the node, all of the border rows
+        product(L(next), X.m, L(next), X.m, false, X.P + (long)next * X.m + next, X.m, false,
+                X.m - next, X.m - next, kw, true);
+        product(L(X.m), X.m, L(next), X.m, false, X.P + (long)X.m * X.m + next, X.m, false,
+                X.ml + X.mr, X.m - next, kw, false);
+        // rows of the inverse side
+        const long Ek = X.W + (long)k0 * X.S;
+        product(L(next), X.m, Ek, X.S, true, X.W + (long)next * X.S, X.S, true, X.m - next, done,
+                kw, false);
+        for(int y : {X.left, X.right})
+          if(y >= 0)
+          {
+            const CoarseNode &Y = N[y];
+            product(L(panel_row(x, y)), X.m, Ek, X.S, true, Y.W + (X.lo - Y.lo), Y.S, true, Y.m,
+                    done, kw, false);
+            product(L(panel_row(x, y)), X.m, L(panel_row(x, y)), X.m, false,
+                    y == X.left ? Y.Q : Y.P, Y.m, false, Y.m, Y.m, kw, true);
+          }
+        if(X.left >= 0 && X.right >= 0)
+        {
+          // the deeper separator's panel holds the rows of the other
+          const int d = N[X.left].height < N[X.right].height ? X.left : X.right;
+          const int u = d == X.left ? X.right : X.left;
+          product(L(panel_row(x, u)), X.m, L(panel_row(x, d)), X.m, false,
+                  N[d].P + (long)panel_row(d, u) * N[d].m, N[d].m, false, N[u].m, N[d].m, kw,
+                  false);
+        }
+      }
+      st.scales = (int)scale.size() - st.scale0;
+      st.upds = (int)upd.size() - st.upd0;
+      t.steps.push_back(st);
+    }
+  }
+  TablePacker pk;
+  const size_t at[9] = {pk.add(N),    pk.add(scale), pk.add(upd),  pk.add(items), pk.add(wofs),
+                        pk.add(uofs), pk.add(lo),    pk.add(node), pk.add(chain)};
+  const cudaError_t e = cudaMalloc(&t.tables, pk.bytes.size() + 1);
+  if(e != cudaSuccess)
+    throw Error{ICARAT_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e)};
+  ICK(cudaMemcpy(t.tables, pk.bytes.data(), pk.bytes.size(), cudaMemcpyHostToDevice));
+  t.nodes = reinterpret_cast<CoarseNode *>(t.tables + at[0]);
+  t.scale = reinterpret_cast<CoarseScaleTile *>(t.tables + at[1]);
+  t.upd = reinterpret_cast<CoarseUpdateTile *>(t.tables + at[2]);
+  t.items = reinterpret_cast<int *>(t.tables + at[3]);
+  t.rows.wofs = reinterpret_cast<long *>(t.tables + at[4]);
+  t.rows.uofs = reinterpret_cast<long *>(t.tables + at[5]);
+  t.rows.lo = reinterpret_cast<int *>(t.tables + at[6]);
+  t.rows.node = reinterpret_cast<int *>(t.tables + at[7]);
+  t.rows.chain = reinterpret_cast<int2 *>(t.tables + at[8]);
+}
+
+// W = L^-1 and W^T (in U) of the matrix in the panels P (which it overwrites)
+void coarse_factor(cudaStream_t st, const CoarseTree &t, double *P, double *W, double *U)
+{
+  ICK(cudaFuncSetAttribute(k_coarse_scale, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)kScaleSmem));
+  ICK(cudaFuncSetAttribute(k_coarse_update, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)kUpdateSmem));
+  ICK(cudaMemsetAsync(W, 0, sizeof(double) * t.nW, st));
+  for(const CoarseStep &s : t.steps)
+  {
+    if(s.join > 0)
+    {
+      note_launch();
+      launch_chained(k_coarse_add, dim3(16, t.nnodes), 256, 0, st,
+                     (const CoarseNode *)t.nodes, s.join, P);
+    }
+    note_launch();
+    launch_chained(k_coarse_scale, s.scales, 256, kScaleSmem, st, (const CoarseNode *)t.nodes,
+                   t.rows.node, (const CoarseScaleTile *)t.scale + s.scale0, P, W, U);
+    if(s.upds > 0)
+    {
+      note_launch();
+      launch_chained(k_coarse_update, s.upds, 256, kUpdateSmem, st,
+                     (const CoarseUpdateTile *)t.upd + s.upd0, P, W);
+    }
+  }
   ICK(cudaGetLastError());
 }
 
-// x[rowmap] = W^T W b[rowmap]  (WT = W^T from dense_spd_inverse_factor); both
-// products return at entry while *halt != 0 (halt null: never)
+// x[rowmap] = W^T W v; both products return at entry while *halt != 0 (halt
+// null: never)
 template <typename T>
-void dense_spd_solve(cudaStream_t st, const double *W, const double *WT, int n,
-                     const double *v, double *t, const int *rowmap, T *x, const int *halt)
+void coarse_solve(cudaStream_t st, const CoarseTree &t, const double *W, const double *U,
+                  const double *v, double *y, const int *rowmap, T *x, const int *halt)
 {
   note_launch(2);
-  const int blocks = (n * 32 + 255) / 256;
-  launch_chained(k_trmv_lower, blocks, 256, 0, st, n, W, v, t, halt);
-  launch_chained(k_trmv_upper<T>, blocks, 256, 0, st, n, WT, t, rowmap, x, halt);
+  launch_chained(k_coarse_lower, t.nitems, 256, 0, st, t.n, t.rows, (const int *)t.items, W, v,
+                 y, halt);
+  launch_chained(k_coarse_upper<T>, (t.n * 32 + 255) / 256, 256, 0, st, t.n, t.rows, U,
+                 (const double *)y, rowmap, x, halt);
 }
 
-template void dense_spd_solve<double>(cudaStream_t, const double *, const double *, int,
-                                      const double *, double *, const int *, double *,
-                                      const int *);
-template void dense_spd_solve<float>(cudaStream_t, const double *, const double *, int,
-                                     const double *, double *, const int *, float *, const int *);
+template void coarse_solve<double>(cudaStream_t, const CoarseTree &, const double *,
+                                   const double *, const double *, double *, const int *,
+                                   double *, const int *);
+template void coarse_solve<float>(cudaStream_t, const CoarseTree &, const double *,
+                                  const double *, const double *, double *, const int *, float *,
+                                  const int *);
 
 } // namespace icarat_b200

@@ -454,32 +454,33 @@ int st_blocks(int numnp)
   return (numnp + kStNodes - 1) / kStNodes;
 }
 
-// dense coarsest matrix from the coarsest level's stencil (thread per free
-// row; entries of constrained columns are skipped)
+// coarsest matrix from the coarsest level's stencil into the panels of its
+// factorization, lower part (thread per free row and neighbour node; entries of
+// constrained columns are skipped)
 __global__ void k_coarse_assemble_st(GridDev g, const double *__restrict__ S,
+                                     const CoarseNode *__restrict__ nodes,
+                                     const int *__restrict__ node,
                                      const int *__restrict__ rowmap,
                                      const int *__restrict__ colmap, int nfree,
-                                     double *__restrict__ A)
+                                     double *__restrict__ P)
 {
-  for(int r = blockIdx.x * blockDim.x + threadIdx.x; r < nfree; r += gridDim.x * blockDim.x)
+  const long total = 27L * nfree;
+  for(long id = blockIdx.x * (long)blockDim.x + threadIdx.x; id < total;
+      id += (long)gridDim.x * blockDim.x)
   {
+    const int r = (int)(id / 27), o = (int)(id % 27);
     const int full = rowmap[r];
     const int c = full / g.numnp, n = full % g.numnp;
-    const int X = n % g.NX, Y = (n / g.NX) % g.NY, Z = n / (g.NX * g.NY);
-    double *row = A + (long)r * nfree;
-    for(int o = 0; o < 27; o++)
+    const int X2 = n % g.NX + o % 3 - 1, Y2 = (n / g.NX) % g.NY + (o / 3) % 3 - 1;
+    const int Z2 = n / (g.NX * g.NY) + o / 9 - 1;
+    if(X2 < 0 || X2 >= g.NX || Y2 < 0 || Y2 >= g.NY || Z2 < 0 || Z2 >= g.NZ)
+      continue;
+    const int m = X2 + Y2 * g.NX + Z2 * g.NX * g.NY;
+    for(int d = 0; d < 3; d++)
     {
-      const int ox = o % 3 - 1, oy = (o / 3) % 3 - 1, oz = o / 9 - 1;
-      const int X2 = X + ox, Y2 = Y + oy, Z2 = Z + oz;
-      if(X2 < 0 || X2 >= g.NX || Y2 < 0 || Y2 >= g.NY || Z2 < 0 || Z2 >= g.NZ)
-        continue;
-      const int m = X2 + Y2 * g.NX + Z2 * g.NX * g.NY;
-      for(int d = 0; d < 3; d++)
-      {
-        const int col = colmap[3L * m + d];
-        if(col >= 0)
-          row[col] = st_coef(S, g.numnp, n, m, o, c, d);
-      }
+      const int col = colmap[3L * m + d];
+      if(col >= 0 && col <= r)
+        P[coarse_entry(nodes, node, r, col)] = st_coef(S, g.numnp, n, m, o, c, d);
     }
   }
 }

@@ -20,6 +20,7 @@
 #include <vector>
 
 #include "../../include/icarat_gpu.h"
+#include "coarse.cuh"
 
 namespace icarat_b200
 {
@@ -276,12 +277,12 @@ struct MgLevel
 struct CoarseSolver
 {
   int n = 0;              // free DOFs of the coarsest level
-  int bw = 0;             // lower bandwidth of the dense matrix in that order
-  int *map = nullptr;     // n -> full index on the coarsest grid
+  CoarseTree tree;        // their order, and the launches that factor and solve
+  int *map = nullptr;     // n -> full index on the coarsest grid; node-major index -> n or -1
   // two factor buffers (the second only once a lagged set-up needs it):
-  double *A[2] = {nullptr, nullptr};    // n x n dense SPD matrix -> its Cholesky factor L
-  double *W[2] = {nullptr, nullptr};    // n x n, L^-1
-  double *work[2] = {nullptr, nullptr}; // n x n scratch of the inversion, then W^T
+  double *P[2] = {nullptr, nullptr}; // panels of the SPD matrix -> of its Cholesky factor L
+  double *W[2] = {nullptr, nullptr}; // L^-1
+  double *U[2] = {nullptr, nullptr}; // its transpose
   double *vin = nullptr, *vout = nullptr;
   int cur = 0;        // buffer the V-cycle reads
   int pending = -1;   // buffer being factored on the side stream (-1: none)

@@ -13,9 +13,8 @@
 // a symmetric positive definite preconditioner.  The coarsest level is solved
 // exactly: W = L^-1 of the Cholesky factor of its dense matrix is rebuilt on
 // the GPU for every design (dense.cu) and each V-cycle applies W^T W.  The
-// dense unknowns are ordered by node planes across the longest axis, which
-// makes the matrix banded (about 3 plane sizes wide) and the factorization
-// work proportional to the band.
+// unknowns are ordered by nested dissection in node planes across the longest
+// axis.
 //
 // The V-cycle exists in FP64 (preconditioner of the FP64 solver) and in FP32
 // (inner solver of the mixed-precision solver); the coarsest solve is FP64 in
@@ -32,11 +31,12 @@
 namespace icarat_b200
 {
 
-void dense_spd_inverse_factor(cudaStream_t st, double *A, double *W, double *T, int n, int bw);
+// dense.cu
+void coarse_factor(cudaStream_t st, const CoarseTree &t, double *P, double *W, double *U);
 template <typename T>
-void dense_spd_solve(cudaStream_t st, const double *W, const double *WT, int n,
-                     const double *v, double *t, const int *rowmap, T *x,
-                     const int *halt = nullptr);
+void coarse_solve(cudaStream_t st, const CoarseTree &t, const double *W, const double *U,
+                  const double *v, double *y, const int *rowmap, T *x,
+                  const int *halt = nullptr);
 
 // Galerkin coarse operators (galerkin.cu)
 __global__ void k_gal_cells_free(GridDev f, GridDev c, const double *__restrict__ E,
@@ -63,9 +63,11 @@ template <typename T>
 void st_residual_launch(cudaStream_t st, const GridDev &g, const T *S, const uint8_t *fix,
                         const T *b, const T *x, T *r, const int *halt);
 __global__ void k_coarse_assemble_st(GridDev g, const double *__restrict__ S,
+                                     const CoarseNode *__restrict__ nodes,
+                                     const int *__restrict__ node,
                                      const int *__restrict__ rowmap,
                                      const int *__restrict__ colmap, int nfree,
-                                     double *__restrict__ A);
+                                     double *__restrict__ P);
 
 // ---------------------------------------------------------------- level data
 __global__ void k_coarsen_E(GridDev f, GridDev c, const double *__restrict__ Ef,
@@ -380,43 +382,52 @@ __global__ void __launch_bounds__(ModalCfg<T>::threads, ModalCfg<T>::blocks)
 }
 
 // ---------------------------------------------------------------- coarse
-// Dense coarse matrix, one thread per free row (fixed summation order).
+// Coarse matrix into the panels of its factorization, one thread per free row
+// and neighbour node (fixed summation order), lower part.  A thread per row
+// walked its eight elements one after another: 71 us on 9 x 5 x 5 nodes,
+// where ten blocks held all rows.
 __global__ void k_coarse_assemble(GridDev g, KeParam ke, const double *__restrict__ E,
-                                  const int *__restrict__ rowmap,
+                                  const CoarseNode *__restrict__ nodes,
+                                  const int *__restrict__ node, const int *__restrict__ rowmap,
                                   const int *__restrict__ colmap, int nfree,
-                                  double *__restrict__ A)
+                                  double *__restrict__ P)
 {
-  for(int r = blockIdx.x * blockDim.x + threadIdx.x; r < nfree;
-      r += gridDim.x * blockDim.x)
+  const long total = 27L * nfree;
+  for(long id = blockIdx.x * (long)blockDim.x + threadIdx.x; id < total;
+      id += (long)gridDim.x * blockDim.x)
   {
-    double *row = A + (long)r * nfree; // zeroed by the caller
-    const int full = rowmap[r];        // component-major index c * numnp + n
+    const int r = (int)(id / 27), o = (int)(id % 27);
+    const int full = rowmap[r]; // component-major index c * numnp + n
     const int n = full % g.numnp, c = full / g.numnp;
     const int i = n % g.NX, j = (n / g.NX) % g.NY, k = n / (g.NX * g.NY);
+    const int dx = o % 3 - 1, dy = (o / 3) % 3 - 1, dz = o / 9 - 1;
+    if(i + dx < 0 || i + dx >= g.NX || j + dy < 0 || j + dy >= g.NY || k + dz < 0 ||
+       k + dz >= g.NZ)
+      continue;
+    double sum[3] = {0.0, 0.0, 0.0};
     for(int sz = 0; sz < 2; sz++)
       for(int sy = 0; sy < 2; sy++)
         for(int sx = 0; sx < 2; sx++)
         {
           const int ei = i - 1 + sx, ej = j - 1 + sy, ek = k - 1 + sz;
-          if(ei < 0 || ei >= g.nx || ej < 0 || ej >= g.ny || ek < 0 || ek >= g.nz)
+          const int bx = dx + 1 - sx, by = dy + 1 - sy, bz = dz + 1 - sz;
+          if((unsigned)ei >= (unsigned)g.nx || (unsigned)ej >= (unsigned)g.ny ||
+             (unsigned)ek >= (unsigned)g.nz || ((bx | by | bz) & ~1))
             continue;
           const double e = E[ei + (long)ej * g.nx + (long)ek * g.nx * g.ny];
-          const int a = local_node(1 - sx, 1 - sy, 1 - sz);
-          for(int bz = 0; bz < 2; bz++)
-            for(int by = 0; by < 2; by++)
-              for(int bx = 0; bx < 2; bx++)
-              {
-                const int b = local_node(bx, by, bz);
-                const long m = (ei + bx) + (long)(ej + by) * g.NX +
-                               (long)(ek + bz) * g.NX * g.NY;
-                for(int d = 0; d < 3; d++)
-                {
-                  const int col = colmap[3 * m + d];
-                  if(col >= 0)
-                    row[col] += e * ke.k[(3 * a + c) * 24 + 3 * b + d];
-                }
-              }
+          const int a = local_node(1 - sx, 1 - sy, 1 - sz), b = local_node(bx, by, bz);
+#pragma unroll
+          for(int d = 0; d < 3; d++)
+            sum[d] += e * ke.k[(3 * a + c) * 24 + 3 * b + d];
         }
+    const long m = n + dx + (long)dy * g.NX + (long)dz * g.NX * g.NY;
+#pragma unroll
+    for(int d = 0; d < 3; d++)
+    {
+      const int col = colmap[3 * m + d];
+      if(col >= 0 && col <= r)
+        P[coarse_entry(nodes, node, r, col)] = sum[d];
+    }
   }
 }
 
@@ -498,9 +509,9 @@ void mg_free(icarat_ctx *c)
       cudaGraphExecDestroy(C.factor[b]);
     if(C.ev_factor[b])
       cudaEventDestroy(C.ev_factor[b]);
-    dfree(C.A[b]);
+    dfree(C.P[b]);
     dfree(C.W[b]);
-    dfree(C.work[b]);
+    dfree(C.U[b]);
   }
   if(C.levels)
     cudaGraphExecDestroy(C.levels);
@@ -508,6 +519,7 @@ void mg_free(icarat_ctx *c)
     cudaEventDestroy(C.ev_levels);
   if(C.side)
     cudaStreamDestroy(C.side);
+  coarse_tree_free(C.tree);
   dfree(C.map);
   dfree(C.vin);
   dfree(C.vout);
@@ -522,6 +534,13 @@ static float *falloc(size_t n)
   if(e != cudaSuccess)
     throw Error{ICARAT_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e)};
   return static_cast<float *>(p);
+}
+
+static void allocate_factor(CoarseSolver &C, int b)
+{
+  C.P[b] = dalloc(C.tree.nP);
+  C.W[b] = dalloc(C.tree.nW);
+  C.U[b] = dalloc(C.tree.nU);
 }
 
 static void allocate_levels(icarat_ctx *c, int levels)
@@ -624,17 +643,19 @@ static void allocate_levels(icarat_ctx *c, int levels)
     fix.swap(fc);
     gf = gc;
   }
-  // dense coarse system: unknowns ordered by node planes across the longest
-  // axis (nodes within a plane, then the 3 components), so that the matrix
-  // is banded (a node couples to the planes either side only) with the
-  // narrowest band
+  // coarse system: its unknowns by node planes across the longest axis (a node
+  // couples to the planes either side only; nodes within a plane, then the 3
+  // components), which the tree's order rearranges
   GridDev gc = c->mg[levels - 1].g;
-  std::vector<int> rowmap, colmap(3 * (size_t)gc.numnp, -1);
+  std::vector<int> full, node3; // of each unknown in the order of the planes
+  std::vector<int> plane_first;
   const int ext[3] = {gc.NX, gc.NY, gc.NZ};
   int ax[3] = {0, 1, 2}; // slowest .. fastest
   std::stable_sort(ax, ax + 3, [&](int p, int q) { return ext[p] > ext[q]; });
   int id[3];
   for(id[ax[0]] = 0; id[ax[0]] < ext[ax[0]]; id[ax[0]]++)
+  {
+    const size_t first = full.size();
     for(id[ax[1]] = 0; id[ax[1]] < ext[ax[1]]; id[ax[1]]++)
       for(id[ax[2]] = 0; id[ax[2]] < ext[ax[2]]; id[ax[2]]++)
       {
@@ -642,45 +663,29 @@ static void allocate_levels(icarat_ctx *c, int levels)
         for(int q = 0; q < 3; q++)
           if(!((fix[n] >> q) & 1u))
           {
-            colmap[3 * (size_t)n + q] = (int)rowmap.size(); // node-major lookup table
-            rowmap.push_back(q * gc.numnp + n);             // component-major vector index
+            full.push_back(q * gc.numnp + n); // component-major vector index
+            node3.push_back(3 * n + q);       // node-major lookup index
           }
       }
-  const int nf = (int)rowmap.size();
-  int bw = 0; // largest index distance of two coupled unknowns
-  for(int n = 0; n < gc.numnp; n++)
-  {
-    const int I = n % gc.NX, J = (n / gc.NX) % gc.NY, K = n / (gc.NX * gc.NY);
-    for(int dk = -1; dk <= 1; dk++)
-      for(int dj = -1; dj <= 1; dj++)
-        for(int di = -1; di <= 1; di++)
-        {
-          const int i2 = I + di, j2 = J + dj, k2 = K + dk;
-          if(i2 < 0 || j2 < 0 || k2 < 0 || i2 >= gc.NX || j2 >= gc.NY || k2 >= gc.NZ)
-            continue;
-          const int n2 = i2 + gc.NX * (j2 + gc.NY * k2);
-          for(int q = 0; q < 3; q++)
-            for(int q2 = 0; q2 < 3; q2++)
-            {
-              const int u = colmap[3 * (size_t)n + q], v = colmap[3 * (size_t)n2 + q2];
-              if(u >= 0 && v >= 0)
-                bw = std::max(bw, std::abs(u - v));
-            }
-        }
+    if(full.size() > first) // a plane without free unknowns is none
+      plane_first.push_back((int)first);
   }
-  c->coarse.bw = bw;
+  const int nf = (int)full.size();
+  plane_first.push_back(nf);
   IREQUIRE((double)nf * nf * 8.0 * 3 < 6.0e9, ICARAT_ERR_UNSUPPORTED,
            "coarsest multigrid level too large for the dense solve; add levels");
   c->coarse.n = nf;
-  ICK(cudaMalloc(&c->coarse.map, sizeof(int) * (rowmap.size() + colmap.size() + 1)));
-  if(nf > 0)
-    ICK(cudaMemcpy(c->coarse.map, rowmap.data(), sizeof(int) * nf,
-                   cudaMemcpyHostToDevice));
-  ICK(cudaMemcpy(c->coarse.map + nf, colmap.data(), sizeof(int) * colmap.size(),
-                 cudaMemcpyHostToDevice));
-  c->coarse.A[0] = dalloc((size_t)nf * nf);
-  c->coarse.W[0] = dalloc((size_t)nf * nf);
-  c->coarse.work[0] = dalloc((size_t)nf * nf);
+  std::vector<int> order;
+  coarse_tree_build(c->coarse.tree, plane_first, order);
+  std::vector<int> map(nf + 3 * (size_t)gc.numnp, -1);
+  for(int i = 0; i < nf; i++)
+  {
+    map[i] = full[order[i]];
+    map[nf + (size_t)node3[order[i]]] = i;
+  }
+  ICK(cudaMalloc(&c->coarse.map, sizeof(int) * (map.size() + 1)));
+  ICK(cudaMemcpy(c->coarse.map, map.data(), sizeof(int) * map.size(), cudaMemcpyHostToDevice));
+  allocate_factor(c->coarse, 0);
   c->coarse.vin = dalloc(nf);
   c->coarse.vout = dalloc(nf);
   // the dense solve writes the free components; the constrained ones stay 0
@@ -762,18 +767,17 @@ static void enqueue_factor(icarat_ctx *c, int b, cudaStream_t st)
   const int n = c->coarse.n;
   if(n == 0)
     return;
-  ICK(cudaMemsetAsync(c->coarse.A[b], 0, sizeof(double) * (size_t)n * n, st));
+  CoarseSolver &D = c->coarse;
+  ICK(cudaMemsetAsync(D.P[b], 0, sizeof(double) * D.tree.nP, st));
   note_launch();
   if(c->mg_galerkin)
-    k_coarse_assemble_st<<<blocks_for(n, 64), 64, 0, st>>>(C.g, C.S, c->coarse.map,
-                                                           c->coarse.map + n, n,
-                                                           c->coarse.A[b]);
+    k_coarse_assemble_st<<<blocks_for(27L * n, 256), 256, 0, st>>>(
+        C.g, C.S, D.tree.nodes, D.tree.rows.node, D.map, D.map + n, n, D.P[b]);
   else
-    k_coarse_assemble<<<blocks_for(n, 64), 64, 0, st>>>(C.g, c->ke0, C.E, c->coarse.map,
-                                                       c->coarse.map + n, n, c->coarse.A[b]);
+    k_coarse_assemble<<<blocks_for(27L * n, 256), 256, 0, st>>>(
+        C.g, c->ke0, C.E, D.tree.nodes, D.tree.rows.node, D.map, D.map + n, n, D.P[b]);
   ICK(cudaGetLastError());
-  dense_spd_inverse_factor(st, c->coarse.A[b], c->coarse.W[b], c->coarse.work[b], n,
-                           c->coarse.bw);
+  coarse_factor(st, D.tree, D.P[b], D.W[b], D.U[b]);
 }
 
 // ||b - K_c x|| / ||b|| of the coarsest dense solve for a fixed right-hand
@@ -797,8 +801,8 @@ double mg_coarse_check(icarat_ctx *c, int levels, int *n_coarse)
   ICK(cudaMemcpy(rowmap.data(), c->coarse.map, sizeof(int) * n, cudaMemcpyDeviceToHost));
   ICK(cudaMemcpy(c->coarse.vin, b.data(), sizeof(double) * n, cudaMemcpyHostToDevice));
   ICK(cudaMemsetAsync(C.x, 0, sizeof(double) * nv, c->stream));
-  dense_spd_solve(c->stream, c->coarse.W[c->coarse.cur], c->coarse.work[c->coarse.cur], n,
-                  c->coarse.vin, c->coarse.vout, c->coarse.map, C.x);
+  coarse_solve(c->stream, c->coarse.tree, c->coarse.W[c->coarse.cur], c->coarse.U[c->coarse.cur],
+               c->coarse.vin, c->coarse.vout, c->coarse.map, C.x);
   if(c->mg_galerkin)
   {
     // A x with the stencil: the residual of b = 0 is -A x
@@ -949,13 +953,8 @@ void mg_setup(icarat_ctx *c, int levels, bool lag)
     return;
   }
   const int nb = 1 - C.cur;
-  if(!C.A[nb])
-  {
-    const size_t nn = (size_t)C.n * C.n;
-    C.A[nb] = dalloc(nn);
-    C.W[nb] = dalloc(nn);
-    C.work[nb] = dalloc(nn);
-  }
+  if(!C.P[nb])
+    allocate_factor(C, nb);
   if(!C.side)
   {
     ICK(cudaStreamCreateWithFlags(&C.side, cudaStreamNonBlocking));
@@ -1186,8 +1185,8 @@ static void vcycle(icarat_ctx *c, int l, const T *b, int deg, bool first_done,
     // the restriction has left the right-hand side in vin
     const int n = c->coarse.n;
     if(n > 0)
-      dense_spd_solve<T>(c->stream, c->coarse.W[c->coarse.cur], c->coarse.work[c->coarse.cur], n,
-                         c->coarse.vin, c->coarse.vout, c->coarse.map, B::x(L), c->mg_halt);
+      coarse_solve<T>(c->stream, c->coarse.tree, c->coarse.W[c->coarse.cur],
+                      c->coarse.U[c->coarse.cur], c->coarse.vin, c->coarse.vout, c->coarse.map, B::x(L), c->mg_halt);
     return;
   }
   MgLevel &C = c->mg[l + 1];
