@@ -588,7 +588,7 @@ double mg_coarse_check(icarat_ctx *c, int levels, int *n_coarse);
 // the last smoothing step also took z . r (and z . K p) and set the scalars.
 bool mg_vcycle(icarat_ctx *c, const double *r, int smooth, bool first_done = false,
                const CycleDot<double> *dot = nullptr);
-bool mg_vcycle_f32(icarat_ctx *c, const float *r, int smooth,
+bool mg_vcycle_f32(icarat_ctx *c, const float *r, int smooth, bool first_done = false,
                    const CycleDot<float> *dot = nullptr);
 // the context's V-cycle stop flag (icarat_ctx::mg_halt) for one scope
 struct HaltScope

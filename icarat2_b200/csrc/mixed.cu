@@ -187,10 +187,14 @@ __global__ void __launch_bounds__(ModalCfg<float>::threads, ModalCfg<float>::blo
   }
 }
 
-// x32 += alpha p, r32 -= alpha Ap; decide whether an FP64 refresh is due.
+// x32 += alpha p, r32 -= alpha Ap; decide whether an FP64 refresh is due.  With
+// x1 set also the first smoothing step of the V-cycle that follows, x1 =
+// inv_theta D^-1 r32, which as a pass of its own (k_cheb_first) read r32 again.
+// Memory bound, four values per thread and turn.
 __global__ void k_mx_update(int n, float *__restrict__ x32, float *__restrict__ r32,
                             const float *__restrict__ p, const float *__restrict__ Ap,
-                            double *__restrict__ partials, MxScalars *s)
+                            const float *__restrict__ invd, float inv_theta,
+                            float *__restrict__ x1, double *__restrict__ partials, MxScalars *s)
 {
   chain_wait();
   __shared__ double sh[32];
@@ -198,13 +202,39 @@ __global__ void k_mx_update(int n, float *__restrict__ x32, float *__restrict__ 
     return;
   const float alpha = (float)s->alpha;
   double rr = 0.0;
-  for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+  auto one = [&](int i)
   {
     x32[i] = fmaf(alpha, p[i], x32[i]);
     const float ri = fmaf(-alpha, Ap[i], r32[i]);
     r32[i] = ri;
     rr += (double)ri * (double)ri;
+    if(x1)
+      x1[i] = inv_theta * invd[i] * ri;
+  };
+  const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
+  for(int i = t0; i < n / 4; i += gridDim.x * blockDim.x)
+  {
+    float4 xv = reinterpret_cast<float4 *>(x32)[i], rv = reinterpret_cast<float4 *>(r32)[i];
+    const float4 pv = reinterpret_cast<const float4 *>(p)[i];
+    const float4 av = reinterpret_cast<const float4 *>(Ap)[i];
+    float4 dv = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if(x1)
+      dv = reinterpret_cast<const float4 *>(invd)[i];
+    xv = make_float4(fmaf(alpha, pv.x, xv.x), fmaf(alpha, pv.y, xv.y), fmaf(alpha, pv.z, xv.z),
+                     fmaf(alpha, pv.w, xv.w));
+    rv = make_float4(fmaf(-alpha, av.x, rv.x), fmaf(-alpha, av.y, rv.y),
+                     fmaf(-alpha, av.z, rv.z), fmaf(-alpha, av.w, rv.w));
+    reinterpret_cast<float4 *>(x32)[i] = xv;
+    reinterpret_cast<float4 *>(r32)[i] = rv;
+    if(x1)
+      reinterpret_cast<float4 *>(x1)[i] =
+          make_float4(inv_theta * dv.x * rv.x, inv_theta * dv.y * rv.y, inv_theta * dv.z * rv.z,
+                      inv_theta * dv.w * rv.w);
+    rr += (double)rv.x * (double)rv.x + (double)rv.y * (double)rv.y +
+          (double)rv.z * (double)rv.z + (double)rv.w * (double)rv.w;
   }
+  if(t0 < n % 4)
+    one(n - n % 4 + t0);
   double v[1] = {rr};
   block_sum<1>(v, sh);
   if(threadIdx.x == 0)
@@ -250,11 +280,13 @@ __global__ void k_mx_flush(int n, double *__restrict__ x, float *__restrict__ x3
   }
 }
 
-// Refresh, part 2: r = b - K x in FP64, r32 = (float) r, stop test on ||r||.
+// Refresh, part 2: r = b - K x in FP64, r32 = (float) r (and x1 again), stop test
+// on ||r||.
 __global__ void __launch_bounds__(ModalCfg<double>::threads, ModalCfg<double>::blocks)
     k_mx_residual(GridDev g, ModalPlan m, KhParam<double> kh, const double *__restrict__ E,
                   const uint8_t *__restrict__ fix, const double *__restrict__ b,
                   const double *__restrict__ x, float *__restrict__ r32,
+                  const float *__restrict__ invd, float inv_theta, float *__restrict__ x1,
                   double *__restrict__ partials, MxScalars *s)
 {
   chain_wait();
@@ -262,18 +294,33 @@ __global__ void __launch_bounds__(ModalCfg<double>::threads, ModalCfg<double>::b
   __shared__ double sh[32];
   if(s->done || !s->refresh)
     return;
+  struct Pre
+  {
+    ModalRhs<double> r;
+    float invd[3];
+  };
   double rr = 0.0;
   modal_march(g, m, kh, E, x, ms,
-              [&](int n) { return modal_rhs(g, fix, b, n); },
-              [&](int n, const double(&acc)[3], const double(&)[3], const ModalRhs<double> &pre)
+              [&](int n)
               {
-                const unsigned f = pre.fix;
+                Pre pre;
+                pre.r = modal_rhs(g, fix, b, n);
+#pragma unroll
+                for(int q = 0; q < 3; q++)
+                  pre.invd[q] = x1 ? invd[(long)q * g.numnp + n] : 0.0f;
+                return pre;
+              },
+              [&](int n, const double(&acc)[3], const double(&)[3], const Pre &pre)
+              {
+                const unsigned f = pre.r.fix;
 #pragma unroll
                 for(int q = 0; q < 3; q++)
                 {
                   const long id = (long)q * g.numnp + n;
-                  const double r = ((f >> q) & 1u) ? 0.0 : pre.b[q] - acc[q];
+                  const double r = ((f >> q) & 1u) ? 0.0 : pre.r.b[q] - acc[q];
                   r32[id] = (float)r;
+                  if(x1)
+                    x1[id] = inv_theta * pre.invd[q] * (float)r;
                   rr += r * r;
                 }
               });
@@ -364,8 +411,23 @@ __global__ void k_mx_pupdate(int n, const float *__restrict__ z, float *__restri
   if(s->done)
     return;
   const float beta = (float)s->beta;
-  for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+  const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
+  for(int i = t0; i < n / 4; i += gridDim.x * blockDim.x)
+  {
+    float4 zv = reinterpret_cast<const float4 *>(z)[i];
+    if(!first)
+    {
+      const float4 pv = reinterpret_cast<const float4 *>(p)[i];
+      zv = make_float4(fmaf(beta, pv.x, zv.x), fmaf(beta, pv.y, zv.y), fmaf(beta, pv.z, zv.z),
+                       fmaf(beta, pv.w, zv.w));
+    }
+    reinterpret_cast<float4 *>(p)[i] = zv;
+  }
+  if(t0 < n % 4)
+  {
+    const int i = n - n % 4 + t0;
     p[i] = first ? z[i] : fmaf(beta, p[i], z[i]);
+  }
 }
 
 static float *falloc(size_t n)
@@ -468,9 +530,9 @@ void apply_K_lowp(icarat_ctx *c, int op, const float *u, float *y)
 constexpr int kDefaultFineOp = ICARAT_OP_FP32;
 constexpr int kDefaultKrylovOp = ICARAT_OP_FP32;
 
-// z = M r32, zr, beta, p update
-// z = M r (the FP32 V-cycle), z . r, beta and p = z + beta p
-static void enqueue_precondition(icarat_ctx *c, int smooth, int first)
+// z = M r32 (the FP32 V-cycle), z . r, beta and p = z + beta p; first_done: the
+// Krylov step has taken the V-cycle's first smoothing step
+static void enqueue_precondition(icarat_ctx *c, int smooth, int first, bool first_done = false)
 {
   const int n = c->neq;
   // z stays in the finest level's x32 (read by z . r and the p update
@@ -480,7 +542,7 @@ static void enqueue_precondition(icarat_ctx *c, int smooth, int first)
   dot.partials = c->d_partials;
   dot.Ap = first ? nullptr : c->f_Ap;
   dot.first = first;
-  const bool done = mg_vcycle_f32(c, c->f_r, smooth, &dot);
+  const bool done = mg_vcycle_f32(c, c->f_r, smooth, first_done, &dot);
   const float *z = c->mg[0].x32;
   if(!done)
   {
@@ -494,16 +556,20 @@ static void enqueue_precondition(icarat_ctx *c, int smooth, int first)
 }
 
 // K p, the updates of x32 and r, and the FP64 refresh when one is due
-static void enqueue_krylov_step(icarat_ctx *c, int krylov_op, const double *b, double *x);
+static void enqueue_krylov_step(icarat_ctx *c, int krylov_op, const double *b, double *x,
+                                bool first_step = false);
 
 static void enqueue_iteration(icarat_ctx *c, int smooth, int krylov_op, const double *b,
                               double *x)
 {
-  enqueue_krylov_step(c, krylov_op, b, x);
-  enqueue_precondition(c, smooth, 0);
+  // the tensor-core operators' V-cycle keeps that step's d as well
+  const bool first_step = c->mx_fine_op == ICARAT_OP_FP32;
+  enqueue_krylov_step(c, krylov_op, b, x, first_step);
+  enqueue_precondition(c, smooth, 0, first_step);
 }
 
-static void enqueue_krylov_step(icarat_ctx *c, int krylov_op, const double *b, double *x)
+static void enqueue_krylov_step(icarat_ctx *c, int krylov_op, const double *b, double *x,
+                                bool first_step)
 {
   const MgLevel &L = c->mg[0];
   const int n = c->neq;
@@ -530,8 +596,11 @@ static void enqueue_krylov_step(icarat_ctx *c, int krylov_op, const double *b, d
     launch_ku_tc(c, TC_DOT, krylov_op == ICARAT_OP_TC_BF16X3 ? 3 : 1, a, c->stream);
   }
   note_launch(3);
+  const double lm = c->lam_max_dk;
+  const float inv_theta = (float)(1.0 / (0.5 * (lm + 0.1 * lm)));
+  float *x1 = first_step ? L.x32 : nullptr;
   launch_chained(k_mx_update, c->red_blocks, kRedThreads, 0, c->stream, n, c->f_x, c->f_r,
-                 c->f_p, c->f_Ap, c->d_partials, c->d_mx);
+                 c->f_p, c->f_Ap, (const float *)L.invd32, inv_theta, x1, c->d_partials, c->d_mx);
   launch_chained(k_mx_flush, c->red_blocks, kRedThreads, 0, c->stream, n, x, c->f_x, c->d_mx);
   int rblocks;
   size_t smem;
@@ -539,7 +608,8 @@ static void enqueue_krylov_step(icarat_ctx *c, int krylov_op, const double *b, d
       modal_launch<double>(L.g, (const void *)k_mx_residual,
                            c->sm_count, kMaxRedBlocks, rblocks, smem);
   launch_chained(k_mx_residual, rblocks, ModalCfg<double>::threads, smem, c->stream, L.g, rm,
-                 c->kh, c->d_E, L.fix, b, (const double *)x, c->f_r, c->d_partials, c->d_mx);
+                 c->kh, c->d_E, L.fix, b, (const double *)x, c->f_r,
+                 (const float *)L.invd32, inv_theta, x1, c->d_partials, c->d_mx);
 }
 
 static const MxScalars &read_scalars(icarat_ctx *c)

@@ -282,6 +282,7 @@ __global__ void __launch_bounds__(ModalCfg<T>::threads, ModalCfg<T>::blocks)
   {
     ModalRhs<T> r;
     T invd[3], d[3];
+    T Ap[DOT && sizeof(T) == 4 ? 3 : 1];
   };
   // z . b, and z . K p in FP32; summed per thread in shared memory (the FP64
   // march has no registers left for them)
@@ -301,6 +302,8 @@ __global__ void __launch_bounds__(ModalCfg<T>::threads, ModalCfg<T>::blocks)
                   const long id = (long)q * g.numnp + n;
                   pre.invd[q] = invd[id];
                   pre.d[q] = din ? din[id] : T(0);
+                  if constexpr(DOT && ND == 2)
+                    pre.Ap[q] = k.Ap ? k.Ap[id] : T(0);
                 }
                 return pre;
               },
@@ -323,9 +326,8 @@ __global__ void __launch_bounds__(ModalCfg<T>::threads, ModalCfg<T>::blocks)
                   if(DOT)
                   {
                     dot[0] += (double)z * (double)pre.r.b[q];
-                    if constexpr(ND == 2)
-                      if(k.Ap)
-                        dot[1] += (double)z * (double)k.Ap[id];
+                    if constexpr(DOT && ND == 2)
+                      dot[1] += (double)z * (double)pre.Ap[q];
                   }
                 }
                 if(DOT)
@@ -1186,7 +1188,8 @@ static void vcycle(icarat_ctx *c, int l, const T *b, int deg, bool first_done,
     const int n = c->coarse.n;
     if(n > 0)
       coarse_solve<T>(c->stream, c->coarse.tree, c->coarse.W[c->coarse.cur],
-                      c->coarse.U[c->coarse.cur], c->coarse.vin, c->coarse.vout, c->coarse.map, B::x(L), c->mg_halt);
+                      c->coarse.U[c->coarse.cur], c->coarse.vin, c->coarse.vout, c->coarse.map,
+                      B::x(L), c->mg_halt);
     return;
   }
   MgLevel &C = c->mg[l + 1];
@@ -1223,9 +1226,10 @@ bool mg_vcycle(icarat_ctx *c, const double *r, int deg, bool first_done,
   return dot == nullptr;
 }
 
-bool mg_vcycle_f32(icarat_ctx *c, const float *r, int deg, const CycleDot<float> *dot)
+bool mg_vcycle_f32(icarat_ctx *c, const float *r, int deg, bool first_done,
+                   const CycleDot<float> *dot)
 {
-  vcycle<float>(c, 0, r, deg, false, &dot);
+  vcycle<float>(c, 0, r, deg, first_done, &dot);
   ICK(cudaGetLastError());
   return dot == nullptr;
 }
