@@ -13,9 +13,9 @@
 // nodes of one height do not depend on one another.  At 17 x 9 x 9 nodes
 // (3,888 unknowns, D = 3) W holds 23 MB instead of the 60 MB of the plane
 // order's dense triangle, so W and W^T stay in L2 between V-cycles, and the
-// chain of 64-column steps is 20 instead of 61 long: the set-up takes 1.07 ms
+// chain of 64-column steps is 20 instead of 61 long: the set-up takes 0.92 ms
 // (3.58 before), the two products of a V-cycle 20 us (43).  At 9 x 5 x 5
-// (600 unknowns, D = 2, 7 steps instead of 10) the set-up takes 0.28 ms (0.60).
+// (600 unknowns, D = 2, 7 steps instead of 10) the set-up takes 0.26 ms (0.60).
 //
 // Factorization, heights from the leaves up, all nodes of a height together:
 // the matrix [A | I] is eliminated 64 columns at a time.  A node's panel
@@ -77,41 +77,46 @@ __device__ __forceinline__ double rsqrt_newton(double x)
 
 // Inverse of the 16 x 16 Cholesky factor of the block at S (lower part) into W
 // (zeros above its diagonal), by one warp: lanes 0-15 hold the rows of the
-// block (symmetric), lanes 16-31 the rows of the identity side.  Step j
+// block (symmetric), lanes 16-31 the rows of the identity side.  A column j
 // subtracts m_r = a_rj / a_jj times row j from the rows r > j of both sides;
-// the pivots' square roots scale the inverse at the end.  What lies left of
-// the pivot on the block's side is not used again and may hold anything.
+// the pivots' square roots scale the inverse at the end.  The chain of pivots
+// is what takes time, so two columns go together: the second pivot's
+// reciprocal is p11 / (p11 p22 - p12^2) and does not wait for the first's.
+// What lies left of the pivots on the block's side is not used again and may
+// hold anything.
 __device__ __forceinline__ void factor16(const double *S, double *W, int lane)
 {
+  constexpr unsigned all = 0xffffffffu;
   const int r = lane & 15;
   const bool block = lane < 16;
   double x[16], piv = 1.0;
 #pragma unroll
   for(int c = 0; c < 16; c++)
     x[c] = block ? S[max(r, c) * kLd + min(r, c)] : (r == c ? 1.0 : 0.0);
-  double p = __shfl_sync(0xffffffffu, x[0], 0);
-  double inv = recip_newton(p);
 #pragma unroll
-  for(int j = 0; j < 16; j++)
+  for(int j = 0; j < 16; j += 2)
   {
-    const double col = __shfl_sync(0xffffffffu, x[j], r);
-    const double m = r > j ? -col * inv : 0.0;
-    const double mb = block ? m : 0.0;
+    const double p11 = __shfl_sync(all, x[j], j), p12 = __shfl_sync(all, x[j + 1], j);
+    const double p22 = __shfl_sync(all, x[j + 1], j + 1);
+    const double c1 = __shfl_sync(all, x[j], r), c2 = __shfl_sync(all, x[j + 1], r);
+    const double i2 = p11 * recip_newton(fma(-p12, p12, p11 * p22));
+    const double i1 = recip_newton(p11), l21 = p12 * i1;
+    const double m1 = r > j ? -c1 * i1 : 0.0;
+    const double m2 = r > j + 1 ? -fma(-c1, l21, c2) * i2 : 0.0;
+    const double b1 = block ? m1 : 0.0, b2 = block ? m2 : 0.0;
     if(r == j)
-      piv = p;
-    if(j < 15) // the next pivot first: its reciprocal is the longest chain
-    {
-      x[j + 1] = fma(mb, __shfl_sync(0xffffffffu, x[j + 1], j), x[j + 1]);
-      p = __shfl_sync(0xffffffffu, x[j + 1], j + 1);
-      inv = recip_newton(p);
-    }
+      piv = p11;
+    if(r == j + 1)
+      piv = fma(-p12, l21, p22);
 #pragma unroll
-    for(int c = 0; c < 16; c++)
-      if(c != j + 1)
-      {
-        const double v = __shfl_sync(0xffffffffu, x[c], c > j ? j : 16 + j);
-        x[c] = fma(c > j ? mb : m, v, x[c]);
-      }
+    for(int t = 0; t < 16; t++)
+    {
+      const int c = (t + j + 2) & 15; // the next pivots' columns first
+      const bool right = c > j + 1;
+      const double v1 = __shfl_sync(all, x[c], right ? j : 16 + j);
+      const double v2 = fma(-l21, v1, __shfl_sync(all, x[c], right ? j + 1 : 17 + j));
+      x[c] = fma(right ? b2 : m2, v2, fma(right ? b1 : m1, v1, x[c]));
+    }
   }
   if(!block)
   {
@@ -122,19 +127,16 @@ __device__ __forceinline__ void factor16(const double *S, double *W, int lane)
   }
 }
 
-// Step `C / 16` of factor64: columns [C, C + 16).
+// Columns [C, C + 16) of factor64, whose diagonal block has been factored.
 __device__ __forceinline__ void factor64_step(int C, double *S, double *W)
 {
   const int NB = (kB - 16 - C) / 16; // 16-row blocks below
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   double *Wd = W + C * kLd + C;
-  if(threadIdx.x < 32)
-    factor16(S + C * kLd + C, Wd, threadIdx.x);
-  __syncthreads();
   // 48 vectors x of 16: the rows of S below (L_i = S_i W_d^T) and the columns of
   // W left of the block (E = W_d E); W_d x in place
   double out[3] = {0.0, 0.0, 0.0};
-#pragma unroll 4
+#pragma unroll
   for(int k = 0; k < 16; k++)
   {
     const double w = Wd[tx * kLd + k];
@@ -153,46 +155,74 @@ __device__ __forceinline__ void factor64_step(int C, double *S, double *W)
   __syncthreads();
   if(NB == 0)
     return;
-  // the rows below, 64 columns in all: S_ij -= L_i L_j^T (j <= i), E_i -= L_i E
-  double acc[3][4] = {};
-#pragma unroll 4
-  for(int k = 0; k < 16; k++)
+  double *L = S + (C + 16) * kLd + C; // rows below, 16 columns
+  if(threadIdx.x < 32)
   {
-    double b[4];
+    // the first warp: the next diagonal block and its factor
+    const int r = threadIdx.x & 15, c0 = 8 * (threadIdx.x >> 4);
+    double acc[8] = {};
+#pragma unroll 4
+    for(int k = 0; k < 16; k++)
+    {
+      const double a = L[r * kLd + k];
 #pragma unroll
-    for(int q = 0; q < 4; q++)
-      b[q] = q < NB ? S[(C + 16 + 16 * q + tx) * kLd + C + k]
-                    : W[(C + k) * kLd + 16 * (q - NB) + tx];
+      for(int c = 0; c < 8; c++)
+        acc[c] = fma(a, L[(c0 + c) * kLd + k], acc[c]);
+    }
+    double *D = L + 16;
 #pragma unroll
-    for(int i = 0; i < 3; i++)
-      if(i < NB)
+    for(int c = 0; c < 8; c++)
+      D[r * kLd + c0 + c] -= acc[c];
+    __syncwarp();
+    factor16(D, W + (C + 16) * kLd + C + 16, threadIdx.x);
+  }
+  else
+  {
+    // the others: the rest of the rows below, 64 columns in all, S_ij -= L_i L_j^T
+    // (16-column blocks j <= i) and E_i -= L_i E; 14 rows at a time
+    const int y = ty - 2;
+    double acc[4][4] = {};
+#pragma unroll 4
+    for(int k = 0; k < 16; k++)
+    {
+      double b[4];
+#pragma unroll
+      for(int q = 0; q < 4; q++)
+        b[q] = q < NB ? L[(16 * q + tx) * kLd + k] : W[(C + k) * kLd + 16 * (q - NB) + tx];
+#pragma unroll
+      for(int i = 0; i < 4; i++)
       {
-        const double a = S[(C + 16 + 16 * i + ty) * kLd + C + k];
+        const double a = L[min(y + 14 * i, 16 * NB - 1) * kLd + k];
 #pragma unroll
         for(int q = 0; q < 4; q++)
           acc[i][q] = fma(a, b[q], acc[i][q]);
       }
-  }
-#pragma unroll
-  for(int i = 0; i < 3; i++)
-#pragma unroll
-    for(int q = 0; q < 4; q++)
-    {
-      const int row = C + 16 + 16 * i + ty;
-      if(i < NB && q < NB && q <= i)
-        S[row * kLd + C + 16 + 16 * q + tx] -= acc[i][q];
-      else if(i < NB && q >= NB)
-        W[row * kLd + 16 * (q - NB) + tx] -= acc[i][q];
     }
+#pragma unroll
+    for(int i = 0; i < 4; i++)
+    {
+      const int row = y + 14 * i;
+      if(row < 16 * NB)
+#pragma unroll
+        for(int q = 0; q < 4; q++)
+          if(q >= NB)
+            W[(C + 16 + row) * kLd + 16 * (q - NB) + tx] -= acc[i][q];
+          else if(row >= 16 && q <= row / 16)
+            L[row * kLd + 16 + 16 * q + tx] -= acc[i][q];
+    }
+  }
   __syncthreads();
 }
 
 // W (64 x 64, zero on entry) = inverse Cholesky factor of the block S (lower
 // part; overwritten), 256 threads: [S | W] eliminated 16 columns at a time, as
 // the whole matrix is by 64.  16 columns are what one warp holds in registers;
-// the rest of a step is small products over all threads.
+// the rest of a step is small products over the other warps meanwhile.
 __device__ void factor64(double *S, double *W)
 {
+  if(threadIdx.x < 32)
+    factor16(S, W, threadIdx.x);
+  __syncthreads();
 #pragma unroll 1
   for(int c = 0; c < kB; c += 16)
     factor64_step(c, S, W);
@@ -242,14 +272,14 @@ __device__ __forceinline__ void tile_product(double (&acc)[4][4], const double *
   }
 }
 
-// f(row, column, value) for each element of a thread's share
-template <typename F> __device__ __forceinline__ void tile_each(const double (&acc)[4][4], F f)
+// f(i, q, row, column) for each element [i][q] of a thread's share
+template <typename F> __device__ __forceinline__ void tile_each(F f)
 {
 #pragma unroll
   for(int i = 0; i < 4; i++)
 #pragma unroll
     for(int q = 0; q < 4; q++)
-      f((int)(threadIdx.x >> 4) + 16 * i, (int)(threadIdx.x & 15) + 16 * q, acc[i][q]);
+      f(i, q, (int)(threadIdx.x >> 4) + 16 * i, (int)(threadIdx.x & 15) + 16 * q);
 }
 
 // the 64 x kw block T of row block k0 of node X's part of W, columns from
@@ -286,7 +316,8 @@ __global__ void k_coarse_add(const CoarseNode *__restrict__ nodes, int height,
 
 // One step's scaling: every block factors its node's diagonal block itself,
 // which saves a launch and a round trip through memory.  The pivots' serial
-// chain bounds it (about 24 us of latency; the product after it takes 3).
+// chain bounds it (31,000 cycles, 16 us; column by column 45,000; the product
+// after it takes 3.5 us).
 __global__ void __launch_bounds__(256)
     k_coarse_scale(const CoarseNode *__restrict__ nodes, const int *__restrict__ node_of,
                    const CoarseScaleTile *__restrict__ tiles, double *P, double *W, double *U)
@@ -321,22 +352,21 @@ __global__ void __launch_bounds__(256)
   if(tile.kind == kTilePanel)
   {
     tile_product<true>(acc, T, Wk);
-    tile_each(acc,
-              [&](int i, int j, double v)
-              {
-                if(i < rows && j < kw)
-                  panel[(long)i * X.m + j] = v;
-              });
+    tile_each([&](int i, int q, int row, int col) {
+      if(row < rows && col < kw)
+        panel[(long)row * X.m + col] = acc[i][q];
+    });
     return;
   }
   tile_product<false>(acc, Wk, T);
-  tile_each(acc, [&](int i, int j, double v) { S[i * kLd + j] = v; });
+  tile_each([&](int i, int q, int row, int col) { S[row * kLd + col] = acc[i][q]; });
   __syncthreads();
   store_inverse(X, nodes, node_of, k0, kw, X.lo + tile.first, cols, S, W, U);
 }
 
-// One step's updates.
-__global__ void __launch_bounds__(256)
+// One step's updates, bound by the FP64 units where tiles are many; two blocks to
+// an SM (three spill) hide the loads.
+__global__ void __launch_bounds__(256, 2)
     k_coarse_update(const CoarseUpdateTile *__restrict__ tiles, double *P, double *W)
 {
   chain_wait();
@@ -349,18 +379,22 @@ __global__ void __launch_bounds__(256)
   else
     stage_tile(B, P + g.b, g.ldb, g.N, g.K);
   __syncthreads();
-  double acc[4][4] = {};
+  // all of the tile is fetched before the first of it is stored, under the
+  // product
+  double *C = (g.to_w ? W : P) + g.c;
+  double acc[4][4] = {}, old[4][4];
+  tile_each([&](int i, int q, int row, int col) {
+    const bool in = row < g.M && col < g.N && (!g.lower || col <= row);
+    old[i][q] = in ? C[(long)row * g.ldc + col] : 0.0;
+  });
   if(g.from_w)
     tile_product<false>(acc, A, B);
   else
     tile_product<true>(acc, A, B);
-  double *C = (g.to_w ? W : P) + g.c;
-  tile_each(acc,
-            [&](int i, int j, double v)
-            {
-              if(i < g.M && j < g.N && (!g.lower || j <= i))
-                C[(long)i * g.ldc + j] -= v;
-            });
+  tile_each([&](int i, int q, int row, int col) {
+    if(row < g.M && col < g.N && (!g.lower || col <= row))
+      C[(long)row * g.ldc + col] = old[i][q] - acc[i][q];
+  });
 }
 
 // t = W v, blocks of 8 warps: a row each, or one long row together
