@@ -657,23 +657,17 @@ int icarat_ctx_create_sel_impl(const icarat_grid *grid, const icarat_material *m
     ICK(cudaMalloc(&c->d_fix, c->numnp));
     ICK(cudaMemcpy(c->d_fix, c->fix_h.data(), c->numnp, cudaMemcpyHostToDevice));
     {
-      std::vector<int> base(c->numnp, 0);
+      std::vector<int> base(c->numnp);
       bool consecutive = true;
       for(long n = 0; n < c->numnp; n++)
       {
-        int k = 0;
-        for(int q = 0; q < 3; q++)
-        {
-          const int eq = c->dof[3 * n + q];
-          const bool free = eq < c->numeq;
-          consecutive = consecutive && free == !((c->fix_h[n] >> q) & 1u);
-          if(!free)
-            continue;
-          if(k == 0)
-            base[n] = eq;
-          consecutive = consecutive && eq == base[n] + k;
-          k++;
-        }
+        const int *eq = c->dof.data() + 3 * n;
+        const int f0 = ~c->fix_h[n] & 1, f1 = (~c->fix_h[n] >> 1) & 1, f2 = (~c->fix_h[n] >> 2) & 1;
+        const int at = f0 ? eq[0] : f1 ? eq[1] : f2 ? eq[2] : 0;
+        const bool same = ((eq[0] < c->numeq) == f0) & ((eq[1] < c->numeq) == f1) &
+                          ((eq[2] < c->numeq) == f2);
+        consecutive &= same & (!f1 | (eq[1] == at + f0)) & (!f2 | (eq[2] == at + f0 + f1));
+        base[n] = at;
       }
       if(consecutive)
       {
