@@ -387,21 +387,22 @@ def fp64_peak_tflops(torch, dev):
 
 def traffic_from_profiles(grid):
     """dram bytes per launch of the stencil kernel from the committed ncu summary."""
-    path = os.path.join(ROOT, "profiles", "k_cg_spmv_%s.txt" % grid)
+    path = os.path.join(ROOT, "profiles", "kernel_counters.md")
     if not os.path.exists(path):
         return None
     for line in open(path):
-        if line.startswith("traffic_bytes_per_launch:"):
-            return float(line.split(":")[1])
+        cells = [c.strip(" `") for c in line.split("|")]
+        if len(cells) > 4 and cells[1].startswith("solve %s mg" % grid) and \
+                cells[2].startswith("k_cg_spmv"):
+            return float(cells[4]) * 1e6
     return None
 
 
 def mixed_section(a, G, torch, dev, flush, world, dist):
     """256x128x128 cantilever, densities U[0.1, 0.5] (seed 0), R = 3, MMA:
     design iterations per second of the mixed-precision loop (FP32 multigrid
-    PCG with the tcgen05 BF16 smoother, FP64 residual refresh) against the
-    plain FP64 multigrid-PCG loop (FP64 tensor-core operator on the finest
-    level) at the same residual, compliance and dc error of one solve
+    PCG, FP64 residual refresh) against the plain FP64 multigrid-PCG loop
+    at the same residual, compliance and dc error of one solve
     against an FP64 solve at rtol 1e-12, and K u GDOF/s of every operator
     on the same design."""
     from icarat2_b200.replicas import job_rate
@@ -528,11 +529,11 @@ def helmholtz_section(a, G, torch, dev, flush, world, dist):
     value, total = job_rate(ms, a.steps, world, dist, dev)
     ms_call = total / a.steps
     it = sum(its) / len(its)
-    # per node and CG iteration: K p (read p, write Ap: 16 B), the Jacobi
-    # update (read x p r Ap, write x r: 48 B; the diagonal comes from the node
-    # class), p = D^-1 r + beta p (read r p, write p: 24 B); per call:
-    # right-hand side, CG start and readout
-    bytes_call = numnp * (88.0 * it + 8 + 48 + 8) + 16.0 * nelx
+    # per node and CG iteration: p = D^-1 r + beta p and K p in one pass (read r
+    # p, write p Ap: 32 B), the Jacobi update (read x p r Ap, write x r: 48 B;
+    # the diagonal comes from the node class); per call: right-hand side with
+    # the CG start (write x r) and readout
+    bytes_call = numnp * (80.0 * it + 16 + 8) + 16.0 * nelx
     peaks = {}
     try:
         peaks = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))
@@ -590,8 +591,8 @@ def helmholtz_section(a, G, torch, dev, flush, world, dist):
            "e2e": {"value": e2e_v, "unit": "filter-calls/s", "h2d_bytes_per_step": 8 * nelx,
                    "d2h_bytes_per_step": 8 * nelx, "host_memory": "pinned",
                    "matches_device_call": ok},
-           "roofline": {"bound": "hbm", "kernel": "Jacobi-PCG iteration (k_helm_spmv, "
-                        "k_helm_update, k_helm_pupdate) + rhs/readout",
+           "roofline": {"bound": "hbm", "kernel": "Jacobi-PCG iteration (k_helm_step, "
+                        "k_helm_update) + rhs/readout",
                         "achieved": gbs, "peak": hbm, "unit": "GB/s", "frac": gbs / hbm,
                         "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)",
                         "bytes_per_call": bytes_call},
@@ -1118,8 +1119,8 @@ def gpu_arm(a):
                                        "CUDA events", "parallelism": "replicas" if world > 1
                                  else "single GPU"}),
             "e2e": e2e, "gpu_launches": int(launches),
-            "roofline": {"bound": "fp64", "kernel": "FP64 K u stencil (k_apply_K_f64 / "
-                         "k_cg_spmv)", "achieved": achieved, "peak": peak64,
+            "roofline": {"bound": "fp64", "kernel": "FP64 K u (k_apply_K_f64 / k_cg_spmv), in "
+                         "operations of the dense element products", "achieved": achieved, "peak": peak64,
                          "unit": "TFLOP/s", "frac": achieved / peak64,
                          "peak_source": "cuBLAS DGEMM 8192^3 measured in this run",
                          "traffic": traffic_from_profiles(a.grid),
