@@ -4,6 +4,7 @@
 // (MMA), with the radius Filter or the Helmholtz PDE filter of
 // opt_macro_oc.cpp:73-74 / opt_mma_Helmholtz.cpp:70-72 and an optional
 // Heaviside threshold.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -104,6 +105,14 @@ int loop_init(icarat_ctx *c, const icarat_loop_opts *o, const double *x0)
   L.object_f = 0.0;
   L.object_old = 0.0;
   loop_free_domains(c);
+  // nothing of an earlier run on this context is a start for this one: the
+  // cases' last solutions and the lagged coarsest factor go (the context's own
+  // solution at the first step, loop_pre).  The factor of a finished design
+  // with voids preconditions a uniform one so badly that the first solve
+  // stopped unconverged after 10,000 iterations (11 with its own factor,
+  // 56 x 24 x 28 after 6 steps with a threshold).
+  std::fill(L.cases_have.begin(), L.cases_have.end(), 0);
+  c->coarse.have = false;
   if(o->filter_kind == 1)
     helm_setup(c, o->filter_radius);
   else
@@ -142,7 +151,8 @@ double loop_pre(icarat_ctx *c)
   IREQUIRE(L.init, ICARAT_ERR_STATE, "icarat_loop_init first");
   const int n = c->nelx;
   const icarat_loop_opts &o = L.opts;
-  L.optstep++;
+  if(L.optstep++ == 0)
+    c->have_u = false; // a warm start is from the step before
   // filter -> threshold -> element design
   if(o.filter_kind == 1)
   {

@@ -113,7 +113,8 @@ typedef struct
   int krylov_op;  /* MIXED_IR: ICARAT_OP_* of K p in the Krylov loop (0 = default) */
   int warm_start; /* start from the solution held by the context (the previous
                      solve, e.g. of the previous design; the loop keeps one per
-                     load case) instead of 0; MIXED_IR, and JACOBI_PCG / MG_PCG
+                     load case, and its first step starts from 0) instead of 0;
+                     MIXED_IR, and JACOBI_PCG / MG_PCG
                      when the solve writes the context's own solution (icarat_solve,
                      the loop): r0 = b - K x0, same stop test ||r|| < rtol ||b|| */
   int fp64_tc;    /* JACOBI_PCG, MG_PCG: FP64 products K u element by element
@@ -128,7 +129,7 @@ typedef struct
                      is computed on a second stream, overlapped with the solve
                      (factor reuse across design iterations; every solve still
                      meets rtol on the current operator).  The first solve on a
-                     new hierarchy factors synchronously. */
+                     new hierarchy or of a new loop factors synchronously. */
   int coarse_op;  /* MG_PCG, MIXED_IR: ICARAT_COARSE_* operators of the coarse
                      multigrid levels (0 = rediscretised) */
 } icarat_solve_opts;
