@@ -100,8 +100,9 @@ __global__ void k_cast(long n, const Tin *__restrict__ in, Tout *__restrict__ ou
 }
 
 // ---------------------------------------------------------------- transfers
-// Blocks are 32 x 4 node columns of one plane (no index divisions; the parity
-// of a row is uniform in its warp).  NC components per thread: all three on
+// Blocks are 32 x 4 node columns of one plane (the parity of a row is uniform
+// in its warp), numbered along the one grid axis that no size of a grid
+// exceeds: planes or rows on the other two would end at 65,535.  NC components per thread: all three on
 // large levels, one on levels below kSplitNodes nodes, where the sums are
 // latency and more threads shorten them (33 x 17 x 17 nodes: restriction 10.7
 // -> 6.7 us; 65 x 33 x 33 is faster with three, 9.6 against 11.1).  Every load
@@ -109,6 +110,19 @@ __global__ void k_cast(long n, const Tin *__restrict__ in, Tout *__restrict__ ou
 // and left out of the sum.  Bound by memory on the finest level: 257 x 129 x
 // 129 nodes FP64, prolongation 62 -> 40 us (220 MB), restriction 32 -> 30.
 constexpr int kSplitNodes = 1 << 15;
+
+// the node (i, j, k) and first component of this thread; false outside
+template <int NC>
+__device__ __forceinline__ bool transfer_node(const GridDev &g, int &i, int &j, int &k, int &q0)
+{
+  const unsigned tx = (g.NX + 31) / 32, ty = (g.NY + 3) / 4;
+  const unsigned row = blockIdx.x / tx, plane = row / ty;
+  i = (blockIdx.x - row * tx) * 32 + threadIdx.x;
+  j = (row - plane * ty) * 4 + threadIdx.y;
+  k = NC == 3 ? plane : plane / 3;
+  q0 = NC == 3 ? 0 : plane % 3;
+  return i < g.NX && j < g.NY;
+}
 
 // coarse b = R r  (R = P^T, 27 fine nodes per coarse node, weights 1/2^d).
 // With xc set, also the coarse level's first Chebyshev step from zero
@@ -124,9 +138,8 @@ __global__ void __launch_bounds__(128)
   chain_wait();
   if(halted(halt))
     return;
-  const int I = blockIdx.x * 32 + threadIdx.x, J = blockIdx.y * 4 + threadIdx.y;
-  const int K = NC == 3 ? blockIdx.z : blockIdx.z / 3, q0 = NC == 3 ? 0 : blockIdx.z % 3;
-  if(I >= c.NX || J >= c.NY)
+  int I, J, K, q0;
+  if(!transfer_node<NC>(c, I, J, K, q0))
     return;
   T s[NC];
 #pragma unroll
@@ -180,9 +193,8 @@ __global__ void __launch_bounds__(128)
   chain_wait();
   if(halted(halt))
     return;
-  const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 4 + threadIdx.y;
-  const int k = NC == 3 ? blockIdx.z : blockIdx.z / 3, q0 = NC == 3 ? 0 : blockIdx.z % 3;
-  if(i >= f.NX || j >= f.NY)
+  int i, j, k, q0;
+  if(!transfer_node<NC>(f, i, j, k, q0))
     return;
   const int ox = i & 1, oy = j & 1, oz = k & 1;
   const int m0 = (i >> 1) + (j >> 1) * c.NX + (k >> 1) * c.NX * c.NY;
@@ -221,9 +233,9 @@ __global__ void __launch_bounds__(128)
   }
 }
 
-static dim3 transfer_grid(const GridDev &g, int nc)
+static unsigned transfer_grid(const GridDev &g, int nc)
 {
-  return dim3((g.NX + 31) / 32, (g.NY + 3) / 4, nc == 3 ? g.NZ : 3 * g.NZ);
+  return (unsigned)((g.NX + 31) / 32) * ((g.NY + 3) / 4) * g.NZ * (nc == 3 ? 1 : 3);
 }
 
 // ---------------------------------------------------------------- smoother
