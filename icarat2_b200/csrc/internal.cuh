@@ -383,8 +383,8 @@ struct icarat_ctx
   bool has_uD = false;
   // device
   int *d_free = nullptr;
-  // equation number of each node's first free component (null unless a node's
-  // equations are consecutive in component order, as countDOF numbers them)
+  // equation number of each node's first free component (its others follow in
+  // component order); part of d_free's buffer
   int *d_eqbase = nullptr;
   uint8_t *d_fix = nullptr;
   double *d_uD = nullptr;

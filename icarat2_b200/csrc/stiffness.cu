@@ -75,7 +75,7 @@ bool apply_K_equations(icarat_ctx *c, const double *u, double *y)
 {
   const GridDev g{c->nx, c->ny, c->nz, c->NX, c->NY, c->NZ, c->numnp, c->nelx};
   // blocks read u while others write y: they must not overlap
-  if(!c->d_eqbase || c->numeq == 0 || use_dmma(c, g) || (u < y + c->numeq && y < u + c->numeq))
+  if(c->numeq == 0 || use_dmma(c, g) || (u < y + c->numeq && y < u + c->numeq))
     return false;
   int blocks;
   size_t smem;
