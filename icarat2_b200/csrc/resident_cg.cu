@@ -30,7 +30,7 @@
 // iteration makes five (two per reduction, one for z); a march step takes 0.9.
 //
 // Waits are bounded: a block whose wait runs out reports an error status and
-// leaves, and so does every other.
+// leaves, and so does every other that still waits for it.
 #include "modal.cuh"
 #include "resident_cg.cuh"
 
@@ -439,17 +439,30 @@ __global__ void __launch_bounds__(kResThreads, 1)
       p[id] = sp[c * h.cells + in];
     }
   }
-  const bool lost = bad != 0;
-  if(t == 0 && lost)
+  // Block 0 reports the solve.  A block that lost a wait is not always seen by
+  // the others (they enter no further step after the launch's last), and may
+  // report before or after block 0: the verdict is settled by atomics, whose
+  // outcome is the error in either order.
+  if(t == 0 && blockIdx.x == 0)
   {
-    // every block's waits run out once one block has left
-    S.done = 1;
-    S.status = ICARAT_ERR_CUDA;
+    s->alpha = S.alpha;
+    s->beta = S.beta;
+    s->zr = S.zr;
+    s->zr_new = S.zr_new;
+    s->pAp = S.pAp;
+    s->rr = S.rr;
+    s->rnorm = S.rnorm;
+    s->iter = S.iter;
+    if(S.done)
+    {
+      atomicCAS(&s->status, ICARAT_OK, S.status);
+      atomicExch(&s->done, 1);
+    }
   }
-  if(t == 0 && (blockIdx.x == 0 || lost))
+  if(t == 0 && bad)
   {
-    S.counter = 0;
-    *s = S;
+    atomicExch(&s->status, ICARAT_ERR_CUDA);
+    atomicExch(&s->done, 1);
   }
 }
 
