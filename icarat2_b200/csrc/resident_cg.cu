@@ -29,6 +29,11 @@
 // 126 x 26 x 26 27.9 -> 11.7.  A trip through the L2 costs about 1 us and an
 // iteration makes five (two per reduction, one for z); a march step takes 0.9.
 //
+// Solves of several contexts share the GPU as far as their blocks fit side by
+// side: two threads with eight solves each take 41.6 ms at 33 x 17 x 17 nodes (one
+// after another 79.6; with three launches per iteration 82.3), and 358 ms at 126
+// x 26 x 26, where one solve fills the GPU (366; 544).
+//
 // Waits are bounded: a block whose wait runs out reports an error status and
 // leaves, and so does every other that still waits for it.
 #include "modal.cuh"
