@@ -32,6 +32,7 @@
 // writes and element-per-lane reads) to the element-per-lane order of the
 // node sums.
 #include <algorithm>
+#include <atomic>
 
 #include "stencil.cuh"
 
@@ -367,8 +368,8 @@ __global__ void __launch_bounds__(dm::kThreads, 2) k_ku_dmma(DmArgs a)
 // ---------------------------------------------------------------- host side
 template <int OP> static int dm_prepare()
 {
-  static int occ_of[kMaxDevices] = {};
-  int &occ = occ_of[device_slot()];
+  static std::atomic<int> occ_of[kMaxDevices];
+  std::atomic<int> &occ = occ_of[device_slot()];
   if(!occ)
   {
     ICK(cudaFuncSetAttribute(k_ku_dmma<OP>, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -37,6 +37,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <atomic>
 
 #include "internal.cuh"
 
@@ -433,13 +434,17 @@ int vol_tiles(const Vol &v)
   return ((v.X + kTX - 1) / kTX) * ((v.Y + kTY - 1) / kTY) * ((v.Z + kTZ - 1) / kTZ);
 }
 
-// the kernel's shared-memory limit, raised once per device
-template <typename K> void allow_smem(K kernel, size_t n, bool (&done)[kMaxDevices])
+// the kernel's shared-memory limit, raised once per device (by two threads at
+// once to the same value)
+typedef std::atomic<bool> OnceFlags[kMaxDevices];
+template <typename K> void allow_smem(K kernel, size_t n, OnceFlags &done)
 {
-  bool &d = done[device_slot()];
-  if(!d)
+  std::atomic<bool> &d = done[device_slot()];
+  if(!d.load())
+  {
     ICK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)n));
-  d = true;
+    d.store(true);
+  }
 }
 
 } // namespace
@@ -483,7 +488,7 @@ void conv3_wgrad(int X, int Y, int Z, const uint16_t *x, int cin, const uint16_t
 {
   const Vol v{X, Y, Z, (long)X * Y * Z};
   const int Cp = (cin + 15) / 16 * 16;
-  static bool done[kMaxDevices] = {};
+  static OnceFlags done;
   allow_smem(k_wgrad_mma, 2 * kWStage, done);
   const bf16 *g = reinterpret_cast<const bf16 *>(g3);
   note_launch(2);
@@ -513,14 +518,14 @@ void conv3_dgrad(int X, int Y, int Z, const uint16_t *g3, int cout, const uint16
   const Vol v{X, Y, Z, (long)X * Y * Z};
   const bf16 *g = reinterpret_cast<const bf16 *>(g3);
   const bf16 *wp = reinterpret_cast<const bf16 *>(wpk);
-  auto launch = [&](auto kernel, int nt, bool(&done)[kMaxDevices]) {
+  auto launch = [&](auto kernel, int nt, OnceFlags &done) {
     const size_t smem = 3 * kHalo * kRow + 27 * 8 * (size_t)nt * kRow;
     allow_smem(kernel, smem, done);
     note_launch();
     kernel<<<dim3(vol_tiles(v), cin / (8 * nt)), kDThreads, smem, st>>>(
         v, g, g + cout * v.V, g + 2 * cout * v.V, cout, wp, cin, dx);
   };
-  static bool done2[kMaxDevices] = {}, done4[kMaxDevices] = {};
+  static OnceFlags done2, done4;
   if(cin % 32 == 0)
     launch(k_dgrad_mma<4>, 4, done4);
   else

@@ -31,6 +31,8 @@
 // kernel records an error and leaves.
 #include <cuda_bf16.h>
 
+#include <atomic>
+
 #include "stencil.cuh"
 
 namespace icarat_b200
@@ -526,8 +528,8 @@ template <int TERMS> static size_t tc_smem_bytes() { return sizeof(tc::Smem<TERM
 
 template <int OP, int TERMS> static int tc_prepare()
 {
-  static int occ_of[kMaxDevices] = {};
-  int &occ = occ_of[device_slot()];
+  static std::atomic<int> occ_of[kMaxDevices];
+  std::atomic<int> &occ = occ_of[device_slot()];
   if(!occ)
   {
     ICK(cudaFuncSetAttribute(k_ku_tc<OP, TERMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
