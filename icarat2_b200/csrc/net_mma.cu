@@ -4,7 +4,9 @@
 // Both gradients multiply BF16 data (activations or weights) by the FP32
 // output gradient.  Its 24-bit significand is exactly three BF16 values
 // (high, middle, low: each the rounded rest of the one before), so three
-// BF16 products per term with FP32 sums replace an FP32 product.  The tensor
+// BF16 products per term with FP32 sums replace an FP32 product.  (Below
+// magnitudes of about 2^-109 the low part meets the smallest BF16 value,
+// 2^-133, and what is under that is lost.)  The tensor
 // core's own running sum is not used for long chains (it does not round to
 // nearest): a chain ends after at most 9 products and is added to FP32
 // registers.
@@ -458,13 +460,15 @@ void sum_parts(int blocks, int C, const double *part, float *out, cudaStream_t s
 
 int conv3_split_blocks(long V) { return (int)((V + 255) / 256); }
 
-// voxel splits of a layer's weight gradient: about two blocks per SM over its
-// channel tiles, at least two tiles each
+// Voxel splits of a layer's weight gradient: about kWgradBlocks blocks over its
+// channel tiles (two for each of the B200's 148 SMs), at least two tiles each.
+// A constant and not the device's SM count: it fixes the order of the sums.
+constexpr int kWgradBlocks = 2 * 148;
 int conv3_wgrad_splits(int X, int Y, int Z, int cin, int cout)
 {
   const Vol v{X, Y, Z, (long)X * Y * Z};
   const int ch = ((cin + 15) / 16) * (cout / 16), tiles = vol_tiles(v);
-  return std::max(1, std::min((2 * 148 + ch - 1) / ch, (tiles + 1) / 2));
+  return std::max(1, std::min((kWgradBlocks + ch - 1) / ch, (tiles + 1) / 2));
 }
 
 // parts of the masked gradient (three arrays of C V at g3, channel-last) and
