@@ -28,7 +28,8 @@
 //   update (k_coarse_update): A_ij -= L_ik L_jk^T in the panel and in the
 //     separators' own panels, E_i -= L_ik E_k for every later row i.
 // Each tile is one 64 x 64 x 64 product on the FP64 units: mma.sync m8n8k4 f64
-// takes 17 us for one on a whole SM here, scalar FMAs 2.1.  A separator receives from the
+// takes 17 us for one on a whole SM here, scalar FMAs 3.5 (7,000 cycles; 4,096
+// at the pipe's rate).  A separator receives from the
 // subtree on each of its sides: the right one adds into an accumulator of its
 // own (no two tiles of a launch share a target) that k_coarse_add joins.
 #include <algorithm>
@@ -316,8 +317,10 @@ __global__ void k_coarse_add(const CoarseNode *__restrict__ nodes, int height,
 
 // One step's scaling: every block factors its node's diagonal block itself,
 // which saves a launch and a round trip through memory.  The pivots' serial
-// chain bounds it (31,000 cycles, 16 us; column by column 45,000; the product
-// after it takes 3.5 us).
+// chain bounds it (31,000 cycles in the kernel, 16 us; column by column 45,000;
+// the product after it takes 3.5 us).  A launch of its own, with cold caches,
+// takes 33 to 36 us under a profiler; in the set-up's graph a step of scaling
+// and update takes 46 us.
 __global__ void __launch_bounds__(256)
     k_coarse_scale(const CoarseNode *__restrict__ nodes, const int *__restrict__ node_of,
                    const CoarseScaleTile *__restrict__ tiles, double *P, double *W, double *U)

@@ -24,7 +24,6 @@
 namespace icarat_b200
 {
 
-constexpr int kBallMax = 9;    // largest D2 compiled
 constexpr int kBallX = 32, kBallY = 8, kBallZ = 4;
 
 template <int D2> struct Ball

@@ -15,7 +15,7 @@
 // (lower face, interior, upper face per axis).  The table of 27 classes x 27
 // neighbour slots is assembled once on the host in the reference's order
 // (ascending element id) for the Jacobi diagonal; the solve runs
-// matrix-free with the same operator in sum-factorised form (k_helm_spmv).
+// matrix-free with the same operator in sum-factorised form (k_helm_step).
 // The CG iteration
 // keeps the device-resident scalar logic of the elasticity solve (one
 // stop-flag read per graph replay of `kHelmChunk` iterations).

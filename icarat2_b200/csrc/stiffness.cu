@@ -2,8 +2,9 @@
 //
 // Replaces LinearAnalysis::assemblingK and the sparse product inside the CG
 // (src/analysis/linear.hpp:117-166, src/analysis/solver/CG.cpp:76-99).
-// Work per node: 8 elements x 3 rows x 24 = 576 DFMA (1152 flop); compulsory
-// bytes per node: 24 read + 24 written (+ 8 per element modulus).
+// The products run in the parity blocks of the box element (modal.cuh): about 165
+// FP64 operations per element, against 576 FMAs for Ke0's dense products;
+// compulsory bytes per node: 24 read + 24 written (+ 8 per element modulus).
 #include "modal.cuh"
 #include "stencil.cuh"
 
@@ -174,10 +175,10 @@ static int node_blocks(const GridDev &g, int threads)
 }
 
 // Below kDmmaMinNodes the element tiles would leave most SMs idle.  The
-// column-march node stencil is the faster FP64 operator at every grid size
-// measured on a B200 (35 us against 62 us at 129 x 65 x 65 nodes, 273 us
-// against 331 us at 257 x 129 x 129), so the default (fp64_tc 0) is the
-// stencil and the FP64 tensor cores run only when asked for.
+// parity-block march is the faster FP64 operator at every grid size measured
+// on a B200 (24.6 us against 62 us at 129 x 65 x 65 nodes, 128 us against 331 us
+// at 257 x 129 x 129), so the default (fp64_tc 0) is the march and the FP64
+// tensor cores run only when asked for.
 constexpr int kDmmaMinNodes = 1 << 15;
 
 bool use_dmma(const icarat_ctx *c, const GridDev &g)
