@@ -453,10 +453,10 @@ template <int D2> static BallWeights<D2> ball_weights(const FilterState &F)
 // The compiled ball is the faster form from about 1e5 taps in all: below, the
 // launch is all the time there is and the tile's halo only adds to it (7 taps
 // on 7 k elements: 5.8 us by the list, 6.6 staged; 19 taps: 8.3 and 6.0).
-static bool use_ball(const icarat_ctx *c)
+static bool use_ball(const icarat_ctx *c, BallUse use)
 {
   return c->filt.ball > 0 && (double)c->filt.nofs * c->nelx >= 1.0e5 &&
-         ball_blocks(c->nx, c->ny, c->nz) < (1L << 31);
+         ball_pays(c->filt.ball, use, c->nx, c->ny, c->nz);
 }
 
 template <int NIN>
@@ -484,7 +484,7 @@ void filter_apply(icarat_ctx *c, const double *in, double *out, bool is_sens)
     IREQUIRE(F.radius >= 1.0e-10, ICARAT_ERR_FILTER,
              "coefficient aa is too small in the density filter");
     note_launch();
-    if(use_ball(c))
+    if(use_ball(c, kBallForward))
       ball_dispatch(F.ball, [&](auto D) {
         constexpr int d2 = decltype(D)::value;
         k_ball_fwd<d2><<<(unsigned)ball_blocks(c->nx, c->ny, c->nz), kBallX * kBallY,
@@ -500,7 +500,7 @@ void filter_apply(icarat_ctx *c, const double *in, double *out, bool is_sens)
     IREQUIRE(F.have_forward, ICARAT_ERR_STATE,
              "transposed filter needs a forward call first (filter.hpp:140-153)");
     note_launch();
-    if(use_ball(c))
+    if(use_ball(c, kBallTransposed))
       launch_ball_trans<1>(c, in, nullptr, out, nullptr);
     else
       k_filter_trans<<<eblocks(c), 256, 0, c->stream>>>(egrid(c), F.nofs, F.d_ofs, F.d_w, F.d_aa,
@@ -518,7 +518,7 @@ void filter_trans2(icarat_ctx *c, const double *in1, const double *in2, double *
   IREQUIRE(F.have_forward, ICARAT_ERR_STATE,
            "transposed filter needs a forward call first (filter.hpp:140-153)");
   note_launch();
-  if(use_ball(c))
+  if(use_ball(c, kBallTransposed))
     launch_ball_trans<2>(c, in1, in2, out1, out2);
   else
     k_filter_trans2<<<eblocks(c), 256, 0, c->stream>>>(egrid(c), F.nofs, F.d_ofs, F.d_w, F.d_aa,

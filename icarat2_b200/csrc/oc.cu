@@ -292,7 +292,7 @@ int oc_update_dev(icarat_ctx *c, double *x, const double *dfdx, double g,
   };
   note_launch();
   const long tiles = ball_blocks(c->nx, c->ny, c->nz);
-  if(c->filt.ball > 0 && tiles < (1L << 31))
+  if(c->filt.ball > 0 && ball_pays(c->filt.ball, kBallBisect, c->nx, c->ny, c->nz))
     ball_dispatch(c->filt.ball, [&](auto D) {
       constexpr int d2 = decltype(D)::value;
       const void *kernel = (const void *)k_oc_bisect_ball<d2>;
