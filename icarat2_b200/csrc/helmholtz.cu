@@ -154,7 +154,7 @@ __global__ void k_helm_start(HelmGrid g, HelmWeights w, HelmInvd iv, const doubl
 // through two in-plane sums per node, A = (mx my + c (sx my + mx sy)) p and
 // B = mx my p, and Ap(k) = sum_dz mz A(k+dz) + c sz B(k+dz).
 //
-// A block of 8 warps owns 32 x 8 node columns and marches through kz planes,
+// A block of 8 warps owns 32 x 16 node columns and marches through kz planes,
 // holding A and B of planes k-1, k, k+1 in registers.  r and the old p come
 // through rings of halo tiles filled by cp.async kHelmAhead planes ahead; one
 // plane ahead of the sums the block forms the new p in a tile of its own (and
@@ -166,11 +166,18 @@ __global__ void k_helm_start(HelmGrid g, HelmWeights w, HelmInvd iv, const doubl
 // the update of p another 24; this kernel takes 49.
 // Two rows per thread at two blocks per SM: one row 56 us, three blocks (80
 // registers) 48 there but slower on smaller grids, and a variant that spills
-// 80 bytes 95.
-constexpr int kHelmRows = 2, kHelmTx = 32, kHelmTy = kHelmRows * kHelmThreads / 32;
-constexpr int kHelmRing = 4, kHelmAhead = 2, kHelmBlocks = 2;
-constexpr int kHaloX = kHelmTx + 2, kHaloY = kHelmTy + 2, kHalo = kHaloX * kHaloY;
-constexpr int kStage = (kHalo + kHelmThreads - 1) / kHelmThreads;
+// 80 bytes 95.  Grids of up to 8 nodes along y take the one row: they fill half
+// of its tile's rows at most (601 x 2 x 601 nodes: 529 us a call before this
+// kernel, 622 with two rows, 497 with one).
+constexpr int kHelmTx = 32, kHelmRing = 4, kHelmAhead = 2, kHelmBlocks = 2;
+constexpr int kHaloX = kHelmTx + 2;
+template <int Rows> struct HelmTile
+{
+  static constexpr int ty = Rows * kHelmThreads / 32;
+  static constexpr int halo = kHaloX * (ty + 2);
+  static constexpr int stage = (halo + kHelmThreads - 1) / kHelmThreads; // cells per thread
+};
+inline int helm_rows(int NY) { return NY <= HelmTile<1>::ty ? 1 : 2; }
 
 // 1-D stencils per axis: neighbour weights mo, so (a neighbour outside the box
 // is staged as 0, so they hold for every node) and centre weights md, sd of a
@@ -181,15 +188,16 @@ struct HelmAxes
   double c;
 };
 
-// tiles of kHelmTx x kHelmTy columns and chunks of kz planes
+// tiles of kHelmTx x HelmTile::ty columns and chunks of kz planes
 struct HelmPlan
 {
   int tiles_x, tiles_y, kz, items;
 };
 
-struct HelmShared
+template <int Rows> struct HelmShared
 {
-  double r[kHelmRing][kHalo], p[kHelmRing][kHalo], q[2][kHalo];
+  double r[kHelmRing][HelmTile<Rows>::halo], p[kHelmRing][HelmTile<Rows>::halo],
+      q[2][HelmTile<Rows>::halo];
 };
 
 // 8-byte global -> shared copy, 0 where !valid
@@ -201,6 +209,7 @@ __device__ __forceinline__ void cp_async8(double *dst, const double *src, bool v
                : "memory");
 }
 
+template <int Rows>
 __global__ void __launch_bounds__(kHelmThreads, kHelmBlocks)
     k_helm_step(HelmGrid g, HelmPlan pl, const __grid_constant__ HelmAxes ax,
                 const __grid_constant__ HelmInvd iv, const double *__restrict__ r,
@@ -209,7 +218,9 @@ __global__ void __launch_bounds__(kHelmThreads, kHelmBlocks)
 {
   chain_wait();
   extern __shared__ __align__(16) unsigned char helm_raw[];
-  HelmShared &S = *reinterpret_cast<HelmShared *>(helm_raw);
+  constexpr int kTy = HelmTile<Rows>::ty, kHalo = HelmTile<Rows>::halo;
+  constexpr int kStage = HelmTile<Rows>::stage;
+  HelmShared<Rows> &S = *reinterpret_cast<HelmShared<Rows> *>(helm_raw);
   __shared__ double sh[32], s_iv[kHelmClasses];
   if(s->done)
     return;
@@ -219,11 +230,11 @@ __global__ void __launch_bounds__(kHelmThreads, kHelmBlocks)
   const int NZ = g.nz + 1;
   const int plane = g.NX * g.NY;
   const double c = ax.c;
-  const int lx = threadIdx.x & 31, ly = (threadIdx.x >> 5) * kHelmRows;
+  const int lx = threadIdx.x & 31, ly = (threadIdx.x >> 5) * Rows;
   double dot = 0.0;
   for(int t = blockIdx.x; t < pl.items; t += gridDim.x)
   {
-    const int i0 = t % pl.tiles_x * kHelmTx, j0 = t / pl.tiles_x % pl.tiles_y * kHelmTy;
+    const int i0 = t % pl.tiles_x * kHelmTx, j0 = t / pl.tiles_x % pl.tiles_y * kTy;
     const int k0 = t / (pl.tiles_x * pl.tiles_y) * pl.kz;
     const int k1 = min(k0 + pl.kz, NZ);
     const int i = i0 + lx, j = j0 + ly;
@@ -240,7 +251,7 @@ __global__ void __launch_bounds__(kHelmThreads, kHelmBlocks)
       const bool in = e < kHalo && x >= 0 && x < g.NX && y >= 0 && y < g.NY;
       off[q] = in ? x + y * g.NX : -1;
       cls[q] = in ? node_class(x, g.NX) + 3 * node_class(y, g.NY) : 0;
-      own[q] = in && hx > 0 && hx <= kHelmTx && hy > 0 && hy <= kHelmTy;
+      own[q] = in && hx > 0 && hx <= kHelmTx && hy > 0 && hy <= kTy;
     }
     auto stage = [&](int k) { // raw plane k into its ring slot
       if(k <= k1)
@@ -285,9 +296,9 @@ __global__ void __launch_bounds__(kHelmThreads, kHelmBlocks)
     // centre weights of this thread's nodes
     const double ex = node_class(min(i, g.NX - 1), g.NX) == 1 ? 2.0 : 1.0;
     const double mx = ex * ax.md[0], sx = ex * ax.sd[0];
-    double my[kHelmRows], sy[kHelmRows];
+    double my[Rows], sy[Rows];
 #pragma unroll
-    for(int q = 0; q < kHelmRows; q++)
+    for(int q = 0; q < Rows; q++)
     {
       const double ey = node_class(min(j + q, g.NY - 1), g.NY) == 1 ? 2.0 : 1.0;
       my[q] = ey * ax.md[1];
@@ -302,7 +313,7 @@ __global__ void __launch_bounds__(kHelmThreads, kHelmBlocks)
     combine(k0 - 1);
     // per row: L = this plane's share of either neighbour plane's K p, done =
     // the output plane's sum but for the plane above, its p
-    double L[kHelmRows] = {}, done[kHelmRows] = {}, pc[kHelmRows] = {};
+    double L[Rows] = {}, done[Rows] = {}, pc[Rows] = {};
     for(int m = k0 - 1; m <= k1; m++)
     {
       // raw plane m + 1 has landed and the new p of plane m is complete
@@ -311,20 +322,20 @@ __global__ void __launch_bounds__(kHelmThreads, kHelmBlocks)
       stage(m + 1 + kHelmAhead);
       combine(m + 1);
       const double *buf = S.q[(m - k0) & 1] + ly * kHaloX + lx;
-      double rm[kHelmRows + 2], rs[kHelmRows + 2], pn0[kHelmRows];
+      double rm[Rows + 2], rs[Rows + 2], pn0[Rows];
 #pragma unroll
-      for(int q = 0; q < kHelmRows + 2; q++)
+      for(int q = 0; q < Rows + 2; q++)
       {
         const double v0 = buf[q * kHaloX + 1], t = buf[q * kHaloX] + buf[q * kHaloX + 2];
         rm[q] = fma(ax.mo[0], t, mx * v0);
         rs[q] = fma(ax.so[0], t, sx * v0);
-        if(q >= 1 && q <= kHelmRows)
+        if(q >= 1 && q <= Rows)
           pn0[q - 1] = v0;
       }
       const double ez = node_class(min(max(m, 0), NZ - 1), NZ) == 1 ? 2.0 : 1.0;
       const double mz = ez * ax.md[2], sz = ez * ax.sd[2] * ax.c, so = ax.so[2] * ax.c;
 #pragma unroll
-      for(int q = 0; q < kHelmRows; q++)
+      for(int q = 0; q < Rows; q++)
       {
         const double tm = rm[q] + rm[q + 2], ts = rs[q] + rs[q + 2];
         const double B = fma(ax.mo[1], tm, my[q] * rm[q + 1]);
@@ -582,8 +593,8 @@ void helm_setup(icarat_ctx *c, double R)
   H.d_oc = dalloc(3 * (size_t)c->nelx);
   ICK(cudaMalloc(&H.d_cg, sizeof(CgScalars)));
   ICK(cudaMemsetAsync(H.d_cg, 0, sizeof(CgScalars), c->stream));
-  ICK(cudaFuncSetAttribute(k_helm_step, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)sizeof(HelmShared)));
+  ICK(cudaFuncSetAttribute(k_helm_step<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)sizeof(HelmShared<2>)));
   H.ready = true;
 }
 
@@ -600,7 +611,8 @@ static int helm_red_blocks(const icarat_ctx *c)
 // halo are formed again per chunk and kHelmBlocks blocks fit an SM.
 static HelmPlan helm_plan(const icarat_ctx *c)
 {
-  HelmPlan p{(c->NX + kHelmTx - 1) / kHelmTx, (c->NY + kHelmTy - 1) / kHelmTy, c->NZ, 0};
+  const int ty = helm_rows(c->NY) == 1 ? HelmTile<1>::ty : HelmTile<2>::ty;
+  HelmPlan p{(c->NX + kHelmTx - 1) / kHelmTx, (c->NY + ty - 1) / ty, c->NZ, 0};
   const long tiles = (long)p.tiles_x * p.tiles_y, slots = (long)kHelmBlocks * c->sm_count;
   double best = 0.0;
   for(int kz = 1; kz <= c->NZ; kz++)
@@ -634,8 +646,12 @@ static void helm_iteration(icarat_ctx *c, int k)
   const int blocks = pl.items < kMaxRedBlocks ? pl.items : kMaxRedBlocks;
   double *from = H.d_p[k & 1], *to = H.d_p[1 - (k & 1)];
   note_launch(2);
-  launch_chained(k_helm_step, blocks, kHelmThreads, sizeof(HelmShared), c->stream, hgrid(c), pl,
-                 helm_axes(c), iv, H.d_r, from, to, H.d_Ap, H.d_partials, H.d_cg);
+  if(helm_rows(c->NY) == 1)
+    launch_chained(k_helm_step<1>, blocks, kHelmThreads, sizeof(HelmShared<1>), c->stream,
+                   hgrid(c), pl, helm_axes(c), iv, H.d_r, from, to, H.d_Ap, H.d_partials, H.d_cg);
+  else
+    launch_chained(k_helm_step<2>, blocks, kHelmThreads, sizeof(HelmShared<2>), c->stream,
+                   hgrid(c), pl, helm_axes(c), iv, H.d_r, from, to, H.d_Ap, H.d_partials, H.d_cg);
   launch_chained(k_helm_update, helm_red_blocks(c), kRedThreads, 0, c->stream, hgrid(c), iv,
                  H.d_val, H.d_r, to, H.d_Ap, H.d_partials, H.d_cg);
   ICK(cudaGetLastError());
